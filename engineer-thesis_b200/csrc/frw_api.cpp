@@ -696,6 +696,17 @@ frw_status frw_layout_create(const float *rects, int64_t n, const double *bounds
         dl.slack = (float)ldexp(4.0, ex - 1 - 23);
         M = 4.0 * std::max(M, std::max(bw, bh)) + 16.0;
         dl.delta = ldexp(M, -40);
+        // the replay's lattice: a query's (d* - 1) * qscale is below
+        // 2^halvings * max(W, H) / dist0 = 20 * 2^halvings (d* is at most the
+        // bounds distance), rounded three times; outside [1, 26] halvings the
+        // lattice does not fit 32 bits or has no step, and a guard of 1 sends
+        // every query to the loop
+        dl.qscale = 0.0;
+        dl.qguard = 1.0;
+        if (halvings >= 1 && halvings <= 26) {
+            dl.qscale = ldexp(1.0, halvings) / dist;
+            dl.qguard = 2.0 * dl.delta * dl.qscale + ldexp(20.0, halvings - 50);
+        }
     }
     dl.n = (int32_t)n;
     dl.nodes = L->T.nodes;

@@ -39,6 +39,7 @@ struct DevLayout {
     const int4 *nref;     // [nodes]
     double bx0, by0, bx1, by1;  // layer bounds (reference getLayerSize)
     double dist0;               // 0.05 * max(W, H): drawBiggestSquareAtPoint's first step
+    double qscale, qguard;      // 2^halvings / dist0 and the lattice distance that settles a replay (query.cuh)
     double delta;               // tie window of the clearance replay (see query.cuh)
     float slack;                // FP32 pre-filter margin: 4 ulp_f32(max |bound|)
     int32_t n, nodes;
