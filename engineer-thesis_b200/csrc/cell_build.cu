@@ -10,20 +10,20 @@
 // are every rect the query at p can find nearest, tied within 2 delta, or
 // containing p (max with 0).  The margin (M * 2^-30, M the layout's
 // coordinate scale) covers the rounding of the cell index of p and of the
-// cell's coordinates, both of order M * 2^-50.  Built from the tree: one
-// clearance query at each cell centre and one box enumeration per cell (the
-// count pass), a scan, then the fill pass, which copies the rects the count
-// pass staged (the first kStage of each cell) and enumerates again only the
-// longer cells, from the radius the count pass kept.  Large grids first
-// build coarse cells (4 x 4 cells each) that way and then answer each cell's
-// clearance and enumeration from its coarse cell's list instead of the tree.
-// Cells with more than max_per_cell rects keep count -1 and their points use
-// the tree.
+// cell's coordinates, both of order M * 2^-50.  One pass over the cells finds
+// the clearance at each cell centre, enumerates the rects of its grown box and
+// writes its record (up to kCellSlots rects in place; a longer list goes to
+// the shared list buffer at an offset from a global cursor, one atomic per
+// block).  Large grids first build coarse cells (4 x 4 cells each) from the
+// tree -- count, scan, fill -- and answer each cell's clearance and enumeration
+// from its coarse cell's list.  Cells with more than max_per_cell rects are
+// left to the tree.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <initializer_list>
+#include <vector>
 
 #include "query.cuh"
 
@@ -33,8 +33,7 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-// rect indices staged per cell by the count pass (a cell of the configs'
-// density lists about 2 rects)
+// rect indices staged per coarse cell by the count pass
 constexpr int kStage = 4;
 
 // Visits the tree's rects touching the closed box B, in tree order, until
@@ -101,108 +100,196 @@ __device__ __forceinline__ void grown_box(const Grid &G, int64_t c, double r, do
     B[3] = (y0 + G.side) + r;
 }
 
-// The radius r_C of cell c (plus `extra`) from the clearance at the cell
-// centre: the tree's, or, when L carries coarse cell lists, the coarse
-// list's (the same value: the list holds every rect the query can need).
-__device__ __forceinline__ double cell_radius(const DevLayout &L, const Grid &G, int64_t c, double extra) {
+// Coarse cells of a build: cell (first, count) into rects and ids, count -1
+// when the cell overflowed.
+struct CoarseLists {
+    int2 *cells = nullptr;
+    float4 *rects = nullptr;
+    int32_t *ids = nullptr;
+    int nx = 0, ny = 0;
+};
+
+// The radius r_C of a cell from the clearance best at its centre.
+__device__ __forceinline__ double radius_of(const DevLayout &L, const Grid &G, double best) {
+    return fmax(best, 0.0) + 0.5 * G.side + 2.0 * L.delta + G.margin;
+}
+
+// A point's distance to the bounds.
+__device__ __forceinline__ double bounds_distance(const DevLayout &L, double x, double y) {
+    return dmin(dmin(x - L.bx0, L.bx1 - x), dmin(y - L.by0, L.by1 - y));
+}
+
+// The centre of cell c.
+__device__ __forceinline__ double2 centre_of(const Grid &G, int64_t c) {
     const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
-    const double x0 = G.gx0 + ix * G.side, y0 = G.gy0 + iy * G.side;
-    Cands C;
-    int hit;
-    double best;
-    clearance(L, x0 + 0.5 * G.side, y0 + 0.5 * G.side, C, hit, best);
-    return fmax(best, 0.0) + 0.5 * G.side + 2.0 * L.delta + G.margin + extra;
+    return make_double2(G.gx0 + ix * G.side + 0.5 * G.side, G.gy0 + iy * G.side + 0.5 * G.side);
 }
 
-// Where cell c's rects come from: the entries of the coarse cell (of
-// factor x factor cells) that covers it, when L carries coarse lists and that
-// coarse cell did not overflow; else (count -1) the tree.
-__device__ __forceinline__ int2 coarse_range(const DevLayout &L, const Grid &G, int factor, int64_t c) {
-    if (!L.cells) return make_int2(0, -1);
-    const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
-    return __ldg(L.cells + (int64_t)(iy / factor) * L.gnx + ix / factor);
-}
-
-// Visits the rects touching B, from the coarse entries ce (positions into
-// L.crects) or from the tree (Morton positions) when ce.y < 0.  A fine
-// cell's grown box lies inside its coarse cell's grown box (the coarse radius
-// carries an extra margin over the Lipschitz bound r_fine <= r_coarse), so
-// the coarse list holds every rect touching it.
-template <typename F>
-__device__ __forceinline__ bool touching_from(const DevLayout &L, int2 ce, const double B[4], F &&visit) {
-    if (ce.y < 0) return touching(L, B, visit);
-    for (int k = ce.x; k < ce.x + ce.y; k++) {
-        const float4 r = __ldg(L.crects + k);
-        if ((double)r.z >= B[0] && B[2] >= (double)r.x && (double)r.w >= B[1] && B[3] >= (double)r.y)
-            if (!visit(k, r)) return true;
-    }
-    return true;
-}
-
-// Per cell: its list length, or -1 (in cells[c].y) when it exceeds cap or
-// the enumeration was incomplete; cnt[c] = entries to reserve; rad[c] its
-// radius and stage[kStage c ..] the source positions of its first kStage
-// rects, for the fill pass.
-__global__ void k_cell_count(DevLayout L, Grid G, int factor, double extra, int cap, int64_t *__restrict__ cnt,
-                             int2 *__restrict__ cells, float *__restrict__ crad, double *__restrict__ rad,
-                             int32_t *__restrict__ stage, unsigned long long *overflow, int64_t nthreads) {
+// Coarse cells, from the tree (L without cells).  Per cell: its list length,
+// or -1 (in cells[c].y) when it exceeds cap or the enumeration was incomplete;
+// cnt[c] = entries to reserve; rad[c] its radius (one margin above the
+// Lipschitz bound r_cell <= r_coarse) and stage[kStage c ..] the tree positions
+// of its first kStage rects, for the fill pass.
+__global__ void k_cell_count(DevLayout L, Grid G, int cap, int64_t *__restrict__ cnt, int2 *__restrict__ cells,
+                             double *__restrict__ rad, int32_t *__restrict__ stage, int64_t nthreads) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nthreads) return;
     const int64_t c = tiled_cell(G, t);
     if (c < 0) return;
-    const double r = cell_radius(L, G, c, extra);
+    const double2 p = centre_of(G, c);
+    Cands C;
+    int hit;
+    double best;
+    clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
+    const double r = radius_of(L, G, best) + G.margin;
     double B[4];
     grown_box(G, c, r, B);
     rad[c] = r;
-    // a point of the cell lies within margin/2 of it whatever the rounding of
-    // its cell index, so every rect within r - margin of the point is listed
-    crad[c] = __double2float_rd(r - G.margin);
     int n = 0;
     int32_t *sg = stage + kStage * c;
-    const bool complete = touching_from(L, coarse_range(L, G, factor, c), B, [&](int k, float4) {
+    const bool complete = touching(L, B, [&](int k, float4) {
         if (n < kStage) sg[n] = k;
         return ++n <= cap;
     });
     const bool ok = complete && n <= cap;
     cnt[c] = ok ? n : 0;
     cells[c] = make_int2(0, ok ? n : -1);
-    if (!ok) atomicAdd(overflow, 1ull);
 }
 
-// Writes the lists of the cells that did not overflow: the staged rects, or
-// for longer lists the enumeration of the same grown box from the same source
-// again (its order is deterministic, so it meets the same rects as the
-// count).
-__global__ void k_cell_fill(DevLayout L, Grid G, int factor, const int64_t *__restrict__ start,
-                            const double *__restrict__ rad, const int32_t *__restrict__ stage,
-                            int2 *__restrict__ cells, float4 *__restrict__ crects, int32_t *__restrict__ cids,
-                            int64_t ncells) {
+// Writes the coarse lists that did not overflow: the staged rects, or for
+// longer lists the enumeration of the same grown box again (its order is
+// deterministic, so it meets the same rects as the count).
+__global__ void k_cell_fill(DevLayout L, Grid G, const int64_t *__restrict__ start, const double *__restrict__ rad,
+                            const int32_t *__restrict__ stage, int2 *__restrict__ cells, float4 *__restrict__ crects,
+                            int32_t *__restrict__ cids, int64_t ncells) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncells) return;
     const int m = cells[c].y;
     if (m < 0) return;
     const int64_t s = start[c];
-    const int2 ce = coarse_range(L, G, factor, c);
-    const float4 *src = ce.y < 0 ? L.rects : L.crects;
-    const int32_t *sid = ce.y < 0 ? L.ids : L.cids;
     if (m <= kStage) {
         for (int i = 0; i < m; i++) {
             const int k = stage[kStage * c + i];
-            crects[s + i] = __ldg(src + k);
-            cids[s + i] = __ldg(sid + k);
+            crects[s + i] = __ldg(L.rects + k);
+            cids[s + i] = __ldg(L.ids + k);
         }
     } else {
         double B[4];
         grown_box(G, c, rad[c], B);
         int n = 0;
-        touching_from(L, ce, B, [&](int k, float4 r) {
+        touching(L, B, [&](int k, float4 r) {
             if (n >= m) return false;
             crects[s + n] = r;
-            cids[s + n] = __ldg(sid + k);
+            cids[s + n] = __ldg(L.ids + k);
             return ++n < m;
         });
     }
     cells[c] = make_int2((int)s, m);
+}
+
+constexpr int kRecordThreads = 256;
+
+// The records of the cells, radii included.  kCoarse: rects come from the
+// coarse cell (of `factor` x `factor` cells) covering the cell -- its list
+// holds every rect the clearance at the centre and the grown box can need --
+// unless it overflowed; else from the tree.  tot[0]: list entries reserved,
+// tot[1]: entries of all cells (records included), tot[2]: cells left to the
+// tree.  Lists past `room` entries are counted, not written (the caller runs
+// the pass again with room for tot[0]).
+// Bound by its writes (84 bytes a cell: 16e6 cells at 10^6 rects take 0.2 ms
+// at the copy rate) and the FP64 gaps of the coarse lists (about 6 rects,
+// twice); it replaces a count pass, a scan and a fill pass with 84 bytes of
+// counts, radii and staged positions per cell between them.
+template <bool kCoarse>
+__global__ void __launch_bounds__(kRecordThreads)
+    k_cell_records(DevLayout L, CoarseLists K, Grid G, int factor, int cap, float4 *__restrict__ cells,
+                   int4 *__restrict__ cellids, float *__restrict__ crad, float4 *__restrict__ crects,
+                   int32_t *__restrict__ cids, int64_t room, unsigned long long *tot, int64_t nthreads) {
+    __shared__ unsigned s_warp[kRecordThreads / 32];
+    __shared__ unsigned long long s_base;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t c = t < nthreads ? tiled_cell(G, t) : -1;
+    int2 ce = make_int2(0, -1);
+    double B[4] = {0, 0, 0, 0};
+    int n = 0;
+    bool tree = false;
+    // visits the rects touching B in a fixed order
+    auto each = [&](auto &&visit) {
+        if (!kCoarse || ce.y < 0) return touching(L, B, [&](int k, float4 r) { return visit(L.ids + k, r); });
+        for (int k = ce.x; k < ce.x + ce.y; k++) {
+            const float4 r = __ldg(K.rects + k);
+            if (touches_box(r, B) && !visit(K.ids + k, r)) break;
+        }
+        return true;
+    };
+    if (c >= 0) {
+        const double2 p = centre_of(G, c);
+        double best = -1.0;
+        if (kCoarse) {
+            const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
+            ce = __ldg(K.cells + (int64_t)(iy / factor) * K.nx + ix / factor);
+        }
+        if (kCoarse && ce.y >= 0) {
+            best = bounds_distance(L, p.x, p.y);
+            for (int k = ce.x; k < ce.x + ce.y; k++) best = dmin(best, rect_gap(__ldg(K.rects + k), p.x, p.y));
+        } else {
+            Cands C;
+            int hit;
+            clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
+        }
+        const double r = radius_of(L, G, best);
+        grown_box(G, c, r, B);
+        // a point of the cell lies within margin/2 of it whatever the rounding of
+        // its cell index, so every rect within r - margin of the point is listed
+        crad[c] = __double2float_rd(r - G.margin);
+        float4 *rec = cells + kCellSlots * c;
+        int32_t *rid = reinterpret_cast<int32_t *>(cellids + c);
+        const bool complete = each([&](const int32_t *id, float4 q) {
+            if (n < kCellSlots) {
+                rec[n] = q;
+                rid[n] = __ldg(id);
+            }
+            return ++n <= cap;
+        });
+        tree = !complete || n > cap;
+        for (int k = n; k < kCellSlots; k++) {
+            rec[k] = make_float4(kFarRect, kFarRect, kFarRect, kFarRect);
+            rid[k] = -1;
+        }
+    }
+    // offsets of the longer lists: a warp scan, the warps' totals, one atomic
+    const unsigned want = !tree && n > kCellSlots ? (unsigned)n : 0u;
+    unsigned x = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[w] = x;
+    const unsigned kept = __reduce_add_sync(0xFFFFFFFFu, tree ? 0u : (unsigned)n);
+    const unsigned trees = __popc(__ballot_sync(0xFFFFFFFFu, tree));
+    if (lane == 0 && kept) atomicAdd(tot + 1, (unsigned long long)kept);
+    if (lane == 0 && trees) atomicAdd(tot + 2, (unsigned long long)trees);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned s = 0;
+        for (int k = 0; k < kRecordThreads / 32; k++) s += s_warp[k];
+        s_base = s ? atomicAdd(tot, (unsigned long long)s) : 0ull;
+    }
+    __syncthreads();
+    if (!want && !tree) return;
+    unsigned long long at = s_base + (x - want);
+    for (int k = 0; k < w; k++) at += s_warp[k];
+    float4 *rec = cells + kCellSlots * c;
+    rec[kCellSlots - 1] = make_float4(kListRect, __int_as_float(tree ? 0 : (int)at), __int_as_float(tree ? kTreeCell : n), 0.f);
+    if (tree || at + want > (unsigned long long)room) return;
+    int m = 0;
+    each([&](const int32_t *id, float4 q) {
+        crects[at + m] = q;
+        cids[at + m] = __ldg(id);
+        return ++m < n;
+    });
 }
 
 // Exclusive scan of int64 values: tile sums, a one-block scan of the tile
@@ -280,13 +367,14 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const int64_t *__res
 }  // namespace
 
 void free_cells(CellBuffers *c, cudaStream_t st) {
-    for (void *p : {(void *)c->cells, (void *)c->crects, (void *)c->cids, (void *)c->crad})
+    for (void *p : {(void *)c->cells, (void *)c->cellids, (void *)c->crects, (void *)c->cids, (void *)c->crad})
         if (p) cudaFreeAsync(p, st);
     *c = CellBuffers();
 }
 
 void attach_cells(DevLayout &L, const CellBuffers &c) {
     L.cells = c.cells;
+    L.cellids = c.cellids;
     L.crects = c.crects;
     L.cids = c.cids;
     L.crad = c.crad;
@@ -300,19 +388,76 @@ void attach_cells(DevLayout &L, const CellBuffers &c) {
 
 namespace {
 
-// Coarse cells, of kCoarse x kCoarse cells each, serve the fine build on
-// grids of at least kTwoLevelMin cells: their lists (from the tree, up to
-// kCoarseCap rects) answer the fine cells' clearance and enumeration, so the
-// tree is traversed once per coarse cell instead of once per cell.
+// Coarse cells, of kCoarse x kCoarse cells each, serve the build of grids of
+// at least kTwoLevelMin cells: their lists (from the tree, up to kCoarseCap
+// rects) answer the cells' clearance and enumeration, so the tree is
+// traversed once per coarse cell instead of once per cell.
 constexpr int kCoarse = 4;
 constexpr int64_t kTwoLevelMin = 1 << 16;
 constexpr int kCoarseCap = 64;
 
-// Count -> scan -> fill of the cells of grid G over L (with coarse lists of
-// factor `factor` attached, or the tree alone); the cell buffers in C.
-frw_status build_grid(const DevLayout &L, const Grid &G, int factor, double extra, int cap, cudaStream_t st,
-                      CellBuffers &C) {
-    const int64_t ncells = (int64_t)G.nx * G.ny;
+// Device buffers of a build, released in stream order at scope exit unless
+// taken.
+struct BuildBufs {
+    std::vector<void *> p;
+    cudaStream_t st;
+    explicit BuildBufs(cudaStream_t s) : st(s) {}
+    template <typename T>
+    frw_status get(T **x, size_t bytes, const char *what) {
+        const cudaError_t e = cudaMallocAsync((void **)x, std::max<size_t>(bytes, 16), st);
+        if (e != cudaSuccess) return cuda_fail(e, what);
+        p.push_back(*x);
+        return FRW_OK;
+    }
+    void drop(void *q) {
+        p.erase(std::find(p.begin(), p.end(), q));
+        cudaFreeAsync(q, st);
+    }
+    void take(void *q) { p.erase(std::find(p.begin(), p.end(), q)); }
+    ~BuildBufs() {
+        for (void *q : p) cudaFreeAsync(q, st);
+    }
+};
+
+// Count -> scan -> fill of coarse cells over the tree of L.
+frw_status build_coarse(const DevLayout &L, const Grid &G, cudaStream_t st, BuildBufs &B, CoarseLists *K) {
+    const int64_t ncells = (int64_t)G.nx * G.ny, tiles = scan_i64_tiles(ncells), nt = tiled_threads(G.nx, G.ny);
+    int64_t *cnt, *start, *sums, *grand;
+    double *rad;
+    int32_t *stage;
+    frw_status rc;
+    if ((rc = B.get(&K->cells, (size_t)ncells * sizeof(int2), "malloc coarse cells"))) return rc;
+    if ((rc = B.get(&cnt, (size_t)ncells * 8, "malloc cell counts"))) return rc;
+    if ((rc = B.get(&start, (size_t)ncells * 8, "malloc cell starts"))) return rc;
+    if ((rc = B.get(&rad, (size_t)ncells * 8, "malloc cell radii (build)"))) return rc;
+    if ((rc = B.get(&stage, (size_t)ncells * kStage * 4, "malloc staged rects"))) return rc;
+    if ((rc = B.get(&sums, (size_t)tiles * 8, "malloc tile sums"))) return rc;
+    if ((rc = B.get(&grand, 8, "malloc total"))) return rc;
+    k_cell_count<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(L, G, kCoarseCap, cnt, K->cells, rad, stage, nt);
+    launch_scan_i64(cnt, ncells, start, sums, grand, st);
+    FRW_CK(cudaGetLastError());
+    int64_t total = 0;
+    if ((rc = read_back(&total, grand, 8, st, "build_cells: coarse list total"))) return rc;
+    if (total > INT32_MAX) {
+        set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
+        return FRW_E_ARG;
+    }
+    if ((rc = B.get(&K->rects, (size_t)total * 16, "malloc coarse rects"))) return rc;
+    if ((rc = B.get(&K->ids, (size_t)total * 4, "malloc coarse ids"))) return rc;
+    if (total > 0)
+        k_cell_fill<<<(unsigned)((ncells + 127) / 128), 128, 0, st>>>(L, G, start, rad, stage, K->cells, K->rects,
+                                                                      K->ids, ncells);
+    FRW_CK(cudaGetLastError());
+    K->nx = G.nx;
+    K->ny = G.ny;
+    return FRW_OK;
+}
+
+// The records of grid G over L (from coarse cells when K has any), the
+// buffers in C.
+frw_status build_records(const DevLayout &L, const CoarseLists &K, const Grid &G, int cap, cudaStream_t st,
+                         BuildBufs &B, CellBuffers &C) {
+    const int64_t ncells = (int64_t)G.nx * G.ny, nt = tiled_threads(G.nx, G.ny);
     C.ncells = ncells;
     C.nx = G.nx;
     C.ny = G.ny;
@@ -320,56 +465,53 @@ frw_status build_grid(const DevLayout &L, const Grid &G, int factor, double extr
     C.gy0 = G.gy0;
     C.side = G.side;
     C.ginv = 1.0 / G.side;
-    int64_t *cnt = nullptr, *start = nullptr, *sums = nullptr, *grand = nullptr;
-    double *rad = nullptr;
-    int32_t *stage = nullptr;
-    unsigned long long *ovf = nullptr;
-    const int64_t tiles = (ncells + kScanTile - 1) / kScanTile;
-    frw_status rc = FRW_OK;
-    auto ck = [&](cudaError_t e, const char *what) {
-        if (e != cudaSuccess && rc == FRW_OK) rc = cuda_fail(e, what);
-        return rc == FRW_OK;
-    };
-    do {
-        if (!ck(cudaMallocAsync(&C.cells, (size_t)ncells * sizeof(int2), st), "malloc cells")) break;
-        if (!ck(cudaMallocAsync(&C.crad, (size_t)ncells * sizeof(float), st), "malloc cell radii")) break;
-        if (!ck(cudaMallocAsync(&cnt, (size_t)ncells * 8, st), "malloc cell counts")) break;
-        if (!ck(cudaMallocAsync(&start, (size_t)ncells * 8, st), "malloc cell starts")) break;
-        if (!ck(cudaMallocAsync(&rad, (size_t)ncells * 8, st), "malloc cell radii (build)")) break;
-        if (!ck(cudaMallocAsync(&stage, (size_t)ncells * kStage * 4, st), "malloc staged rects")) break;
-        if (!ck(cudaMallocAsync(&sums, (size_t)tiles * 8, st), "malloc tile sums")) break;
-        // the list total and the overflow count side by side: one read-back
-        if (!ck(cudaMallocAsync(&grand, 16, st), "malloc total")) break;
-        ovf = reinterpret_cast<unsigned long long *>(grand + 1);
-        if (!ck(cudaMemsetAsync(ovf, 0, 8, st), "memset")) break;
-        const unsigned blocks = (unsigned)((ncells + 127) / 128);
-        const int64_t nt = tiled_threads(G.nx, G.ny);
-        k_cell_count<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(L, G, factor, extra, cap, cnt, C.cells, C.crad,
-                                                                  rad, stage, ovf, nt);
-        k_tile_sums<<<(unsigned)tiles, kScanThreads, 0, st>>>(cnt, ncells, sums);
-        k_scan_sums<<<1, kScanThreads, 0, st>>>(sums, tiles, grand);
-        k_tile_scan<<<(unsigned)tiles, kScanThreads, 0, st>>>(cnt, ncells, sums, start);
-        if (!ck(cudaGetLastError(), "cell count")) break;
-        unsigned long long h[2] = {0, 0};  // list total, overflowed cells
-        if ((rc = read_back(h, grand, 16, st, "build_cells: list total"))) break;
-        const int64_t total = (int64_t)h[0];
-        if (total > INT32_MAX) {
+    frw_status rc;
+    unsigned long long *tot;
+    if ((rc = B.get(&C.cells, (size_t)ncells * kCellSlots * sizeof(float4), "malloc cells"))) return rc;
+    if ((rc = B.get(&C.cellids, (size_t)ncells * sizeof(int4), "malloc cell ids"))) return rc;
+    if ((rc = B.get(&C.crad, (size_t)ncells * sizeof(float), "malloc cell radii"))) return rc;
+    if ((rc = B.get(&tot, 24, "malloc totals"))) return rc;
+    // one entry of list room per cell holds the lists of the benchmark's
+    // densities (0.3 at 16 cells per rect); denser ones take a second pass
+    int64_t room = std::max<int64_t>(ncells, 4096);
+    unsigned long long h[3] = {0, 0, 0};
+    float4 *rects = nullptr;
+    int32_t *ids = nullptr;
+    for (int pass = 0; pass < 2; pass++) {
+        if ((rc = B.get(&rects, (size_t)room * 16, "malloc cell rects"))) return rc;
+        if ((rc = B.get(&ids, (size_t)room * 4, "malloc cell ids"))) return rc;
+        FRW_CK(cudaMemsetAsync(tot, 0, 24, st));
+        const unsigned blocks = (unsigned)((nt + kRecordThreads - 1) / kRecordThreads);
+        if (K.cells)
+            k_cell_records<true><<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, cap, C.cells, C.cellids, C.crad,
+                                                                    rects, ids, room, tot, nt);
+        else
+            k_cell_records<false><<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, cap, C.cells, C.cellids,
+                                                                     C.crad, rects, ids, room, tot, nt);
+        FRW_CK(cudaGetLastError());
+        if ((rc = read_back(h, tot, 24, st, "build_cells: list total"))) return rc;
+        if (h[0] >= (unsigned long long)kMaxListEntries) {
             set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
-            rc = FRW_E_ARG;
-            break;
+            return FRW_E_ARG;
         }
-        C.entries = total;
-        C.overflow = (int64_t)h[1];
-        if (!ck(cudaMallocAsync(&C.crects, (size_t)std::max<int64_t>(total, 1) * 16, st), "malloc cell rects")) break;
-        if (!ck(cudaMallocAsync(&C.cids, (size_t)std::max<int64_t>(total, 1) * 4, st), "malloc cell ids")) break;
-        if (total > 0)
-            k_cell_fill<<<blocks, 128, 0, st>>>(L, G, factor, start, rad, stage, C.cells, C.crects, C.cids, ncells);
-        if (!ck(cudaGetLastError(), "cell fill")) break;
-    } while (0);
-    for (void *p : {(void *)cnt, (void *)start, (void *)sums, (void *)grand, (void *)rad, (void *)stage})
-        if (p) cudaFreeAsync(p, st);
-    C.bytes = ncells * (int64_t)(sizeof(int2) + sizeof(float)) + C.entries * 20;
-    return rc;
+        if ((int64_t)h[0] <= room) break;
+        B.drop(rects);
+        B.drop(ids);
+        room = (int64_t)h[0];
+    }
+    // the lists in buffers of their size
+    const int64_t total = (int64_t)h[0];
+    if ((rc = B.get(&C.crects, (size_t)total * 16, "malloc cell rects"))) return rc;
+    if ((rc = B.get(&C.cids, (size_t)total * 4, "malloc cell ids"))) return rc;
+    if (total) {
+        FRW_CK(cudaMemcpyAsync(C.crects, rects, (size_t)total * 16, cudaMemcpyDeviceToDevice, st));
+        FRW_CK(cudaMemcpyAsync(C.cids, ids, (size_t)total * 4, cudaMemcpyDeviceToDevice, st));
+    }
+    C.entries = (int64_t)h[1];
+    C.overflow = (int64_t)h[2];
+    C.bytes = ncells * (int64_t)(kCellSlots * sizeof(float4) + sizeof(int4) + sizeof(float)) + total * 20;
+    for (void *q : {(void *)C.cells, (void *)C.cellids, (void *)C.crad, (void *)C.crects, (void *)C.cids}) B.take(q);
+    return FRW_OK;
 }
 
 }  // namespace
@@ -403,42 +545,31 @@ frw_status build_cells(const DevLayout &Lin, double cells_per_rect, int cap, cud
     const double margin = std::ldexp(M, -30);
     const Grid G{L.bx0, L.by0, side, margin, (int)nx, (int)ny};
 
-    cudaEvent_t e0, e1;
-    FRW_CK(cudaEventCreate(&e0));
-    FRW_CK(cudaEventCreate(&e1));
-    CellBuffers C, K;  // the cells; coarse cells serving their build
-    frw_status rc = FRW_OK;
-    do {
-        if (cudaEventRecord(e0, st) != cudaSuccess) {
-            rc = cuda_fail(cudaGetLastError(), "event");
-            break;
-        }
+    Events ev(2);
+    if (!ev.ok(2)) return cuda_fail(cudaErrorUnknown, "build_cells: cudaEventCreate");
+    FRW_CK(cudaEventRecord(ev[0], st));
+    CellBuffers C;
+    {
+        BuildBufs B(st);
+        CoarseLists K;
+        frw_status rc = FRW_OK;
         if (ncells >= kTwoLevelMin) {
-            // coarse radius one margin above the Lipschitz bound r_cell <= r_coarse
             const Grid Gk{L.bx0, L.by0, side * kCoarse, margin, (int)((nx + kCoarse - 1) / kCoarse),
                           (int)((ny + kCoarse - 1) / kCoarse)};
-            if ((rc = build_grid(L, Gk, 1, margin, kCoarseCap, st, K))) break;
-            DevLayout Lk = L;
-            attach_cells(Lk, K);
-            rc = build_grid(Lk, G, kCoarse, 0.0, cap, st, C);
-        } else {
-            rc = build_grid(L, G, 1, 0.0, cap, st, C);
+            rc = build_coarse(L, Gk, st, B, &K);
         }
-        if (rc) break;
-        if (cudaEventRecord(e1, st) != cudaSuccess) {
-            rc = cuda_fail(cudaGetLastError(), "event");
-            break;
-        }
-        if ((rc = wait_event(e1, "build_cells"))) break;
-        cudaEventElapsedTime(&C.build_ms, e0, e1);
-    } while (0);
-    free_cells(&K, st);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (rc != FRW_OK) {
+        if (!rc) rc = build_records(L, K, G, cap, st, B, C);
+        if (rc) return rc;
+    }
+    frw_status rc = FRW_OK;
+    const cudaError_t e = cudaEventRecord(ev[1], st);
+    if (e != cudaSuccess) rc = cuda_fail(e, "event");
+    if (!rc) rc = wait_event(ev[1], "build_cells");
+    if (rc) {
         free_cells(&C, st);
         return rc;
     }
+    cudaEventElapsedTime(&C.build_ms, ev[0], ev[1]);
     *out = C;
     return FRW_OK;
 }

@@ -95,26 +95,30 @@ static __device__ int nearest_other_tree(const DevLayout &L, double px, double p
 // (ties included); otherwise the tree.  Writes the rect, false when none.
 static __device__ __forceinline__ bool nearest_other(const DevLayout &L, double px, double py, int exclude, float4 &o) {
     if (L.cells && px >= L.bx0 && py >= L.by0 && px <= L.bx1 && py <= L.by1) {
-        int ix = (int)__dmul_rn(__dsub_rn(px, L.gx0), L.ginv);
-        int iy = (int)__dmul_rn(__dsub_rn(py, L.gy0), L.ginv);
-        ix = ix < 0 ? 0 : (ix >= L.gnx ? L.gnx - 1 : ix);
-        iy = iy < 0 ? 0 : (iy >= L.gny ? L.gny - 1 : iy);
-        const int64_t cell = (int64_t)iy * L.gnx + ix;
-        const int2 ce = __ldg(L.cells + cell);
-        if (ce.y >= 0) {
+        const int64_t cell = cell_of(L, px, py);
+        const float4 *r = L.cells + kCellSlots * cell;
+        const int32_t *ids = reinterpret_cast<const int32_t *>(L.cellids + cell);
+        const float4 last = __ldg(r + kCellSlots - 1);
+        int n = kCellSlots;
+        if (last.x > kFarRect) {  // a longer list, or (n < 0) the tree
+            n = __float_as_int(last.z);
+            r = L.crects + __float_as_int(last.y);
+            ids = L.cids + __float_as_int(last.y);
+        }
+        if (n >= 0) {
             double best = 1e300;
             int best_id = 0x7FFFFFFF;
             float4 bo = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = ce.x; k < ce.x + ce.y; k++) {
-                const int id = __ldg(L.cids + k);
-                if (id == exclude) continue;
-                const float4 r = __ldg(L.crects + k);
+            for (int k = 0; k < n; k++) {
+                const int id = __ldg(ids + k);
+                if (id == exclude || id < 0) continue;
+                const float4 q = __ldg(r + k);
                 const double g =
-                    fmax(fmax((double)r.x - px, px - (double)r.z), fmax((double)r.y - py, py - (double)r.w));
+                    fmax(fmax((double)q.x - px, px - (double)q.z), fmax((double)q.y - py, py - (double)q.w));
                 if (g < best || (g == best && id < best_id)) {
                     best = g;
                     best_id = id;
-                    bo = r;
+                    bo = q;
                 }
             }
             if (best <= (double)__ldg(L.crad + cell)) {

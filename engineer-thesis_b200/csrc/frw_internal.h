@@ -32,6 +32,18 @@ FRW_HD int leaf_ref(int first, int count) { return -2 - ((first << kLeafBits) | 
 FRW_HD int leaf_first(int ref) { return (-2 - ref) >> kLeafBits; }
 FRW_HD int leaf_count(int ref) { return (-2 - ref) & kLeafCountMax; }
 
+// A cell's record: its rects, unused slots holding a rect too far to matter
+// (kFarRect in every coordinate); or, when it lists more than kCellSlots
+// rects, its first kCellSlots - 1 and a last slot of kListRect and the bits of
+// (first, count, -): all its rects are entries first .. first + count - 1 of
+// the lists, count < 0 when the tree answers the cell's points.  Read as a
+// rect that slot is as far as an unused one (first < kMaxListEntries keeps its
+// bits below kListRect), so the gaps of a record need no test.
+constexpr int kCellSlots = 4;
+constexpr float kFarRect = 3.0e38f, kListRect = 3.3e38f;
+constexpr int64_t kMaxListEntries = 0x7F000000;
+constexpr int32_t kTreeCell = INT32_MIN;
+
 struct DevLayout {
     const float4 *rects;  // [n] Morton order
     const int32_t *ids;   // [n] Morton position -> layer index
@@ -45,10 +57,11 @@ struct DevLayout {
     int32_t n, nodes;
     int32_t halvings;  // bisection steps of the replay with dist above MIN_DIST: dist0 halved that often
     // cell lists (optional, cells == nullptr: tree only): a gnx x gny grid of
-    // side 1/ginv from (gx0, gy0); cell (start, count) into crects / cids,
-    // count < 0 when the cell overflowed and its points use the tree
-    const int2 *cells;
-    const float4 *crects;
+    // side 1/ginv from (gx0, gy0), one 64-byte record (kCellSlots rects) per
+    // cell, see cell_build.cu
+    const float4 *cells;    // [kCellSlots * cells]
+    const int4 *cellids;    // [cells] layer indices of the record's rects
+    const float4 *crects;   // lists of the cells with more than kCellSlots rects, all their rects
     const int32_t *cids;
     const float *crad;  // per cell: every rect within this L-inf distance of any point of the cell is listed
     double gx0, gy0, ginv;
@@ -214,7 +227,8 @@ void free_tree(TreeBuffers *t, cudaStream_t stream);
 // rect whose L-inf distance to a cell can be within 2 delta of the clearance
 // of a point of the cell, per cell, at most max_per_cell of them.
 struct CellBuffers {
-    int2 *cells = nullptr;
+    float4 *cells = nullptr;
+    int4 *cellids = nullptr;
     float4 *crects = nullptr;
     int32_t *cids = nullptr;
     float *crad = nullptr;

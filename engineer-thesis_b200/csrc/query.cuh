@@ -31,19 +31,30 @@ constexpr int kNoHit = 0x7FFFFFFF;
 constexpr double kMinDist = (double).095f;  // drawBiggestSquareAtPoint MIN_DIST
 
 // The rects the replay tests for boxes within delta of the clearance: a
-// point answered by a cell list keeps its cell's whole list (first >= 0:
-// the cell-list entries first .. first + n - 1), a superset of the near
-// ties; a point answered by the tree keeps the near-tie list idx[0 .. n) of
-// tree rects (first == -1).  Testing more rects than the ties is as exact:
-// every listed rect is a real rect of the layout.  More ties than kCandMax
-// (rects whose near sides line up tie exactly) set first = -2: the replay's
-// boxes near the clearance are then tested against the whole tree.
+// point answered by a cell list keeps its cell (first >= 0), whose whole list
+// is a superset of the near ties; a point answered by the tree keeps the
+// near-tie list idx[0 .. n) of tree rects (first == -1).  Testing more rects
+// than the ties is as exact: every listed rect is a real rect of the layout.
+// More ties than kCandMax (rects whose near sides line up tie exactly) set
+// first = -2: the replay's boxes near the clearance are then tested against
+// the whole tree.
 struct Cands {
     int idx[kCandMax];  // tree: positions of the near-tied rects among the tree's rects
     float g[kCandMax];  // their gaps, rounded down (keeping extra entries is harmless)
     int n;
     int first;
 };
+
+// Minimum and maximum without fmin / fmax's NaN rules (the operands are
+// differences of finite coordinates): a comparison and a select each.
+__device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }
+
+// gap(R, p): <= 0 exactly when p lies in the closed rect (each difference is
+// <= 0 exactly when p is on that side).
+__device__ __forceinline__ double rect_gap(const float4 r, double px, double py) {
+    return dmax(dmax((double)r.x - px, px - (double)r.z), dmax((double)r.y - py, py - (double)r.w));
+}
 
 // L-infinity distance from a point (in FP32) to a box, 0 inside.
 __device__ __forceinline__ float lb_box_f(const float4 b, float px, float py) {
@@ -174,28 +185,37 @@ static __device__ __noinline__ uint32_t tree_clearance_call(const float4 *nbox, 
     return tree_clearance<kTies>(nbox, nref, rects, ids, px, py, r2, slack, C, hit, best);
 }
 
+// The cell of a point inside the bounds (the far edge's cells by clamping).
+__device__ __forceinline__ int64_t cell_of(const DevLayout &L, double px, double py) {
+    const unsigned ix = min((unsigned)(int)__dmul_rn(__dsub_rn(px, L.gx0), L.ginv), (unsigned)(L.gnx - 1));
+    const unsigned iy = min((unsigned)(int)__dmul_rn(__dsub_rn(py, L.gy0), L.ginv), (unsigned)(L.gny - 1));
+    return (int64_t)iy * L.gnx + ix;
+}
+
 // The clearance of p and its near-tie list.  With cell lists the list of
 // p's cell holds every rect that can come within 2*delta of the clearance of
 // any point of the cell (the cell's radius is bounded by the clearance of
 // its centre plus half a side, with a margin far above the rounding of the
 // cell index), so scanning it gives the same d*, the same containing rect and
-// a superset of the same ties as the whole tree; a list holds about two
-// rects, so every one gets the exact FP64 gap without an FP32 screen, and
-// the list itself stands for the ties.  Otherwise (no cell lists, or an
-// overflowed cell): one depth-first, nearest-child-first traversal.  Node
-// boxes and rect gaps are screened in FP32 (errors below L.slack); only
-// rects that can matter -- inside the current tie window or containing p --
-// get the exact FP64 gap.  Returns status bits.
+// a superset of the same ties as the whole tree.  A cell lists about two
+// rects, so its record keeps them in place: one aligned 64-byte read instead
+// of a record and then its list (1e7 random points on 10^6 rects: 254 -> 150
+// bytes of DRAM reads each, 0.545 -> 0.468 ms), every slot taking the exact
+// FP64 gap without a loop or a test.  Otherwise (no cell lists, or an overflowed cell): one
+// depth-first, nearest-child-first traversal.  Node boxes and rect gaps are
+// screened in FP32 (errors below L.slack); only rects that can matter --
+// inside the current tie window or containing p -- get the exact FP64 gap.
+// Returns status bits.
+// bd: p's distance to the bounds (negative outside).
 // kInside: the caller has checked that p lies inside the bounds.
 // kOutOfLineTree: the tree traversal is a call (smaller code at the caller).
 // kTies: see scan_rect.
 template <bool kInside = false, bool kOutOfLineTree = false, bool kTies = true>
 __device__ __forceinline__ uint32_t clearance(const DevLayout &L, double px, double py, Cands &C,
-                                              int &hit, double &best, double bd = -1.0) {
+                                              int &hit, double &best, double bd) {
     uint32_t st = 0;
     const double r2 = 2.0 * L.delta;
-    // bd: the bounds distance, when the caller has it (kInside)
-    best = kInside ? bd : fmin(fmin(px - L.bx0, L.bx1 - px), fmin(py - L.by0, L.by1 - py));
+    best = bd;
     hit = kNoHit;
     C.n = 0;
     C.first = -1;
@@ -206,24 +226,27 @@ __device__ __forceinline__ uint32_t clearance(const DevLayout &L, double px, dou
         return 0;
     }
     if (L.cells) {
-        int ix = (int)__dmul_rn(__dsub_rn(px, L.gx0), L.ginv);
-        int iy = (int)__dmul_rn(__dsub_rn(py, L.gy0), L.ginv);
-        ix = ix < 0 ? 0 : (ix >= L.gnx ? L.gnx - 1 : ix);
-        iy = iy < 0 ? 0 : (iy >= L.gny ? L.gny - 1 : iy);
-        const int2 ce = __ldg(L.cells + (int64_t)iy * L.gnx + ix);
-        if (ce.y >= 0) {
-            C.first = ce.x;
-            C.n = ce.y;
-#pragma unroll 2
-            for (int k = ce.x; k < ce.x + ce.y; k++) {
-                const float4 r = __ldg(L.crects + k);
-                const double x0 = r.x, y0 = r.y, x1 = r.z, y1 = r.w;
-                const double g = fmax(fmax(x0 - px, px - x1), fmax(y0 - py, py - y1));
-                if (g <= 0.0) {  // each difference is <= 0 exactly when p is on that side
-                    const int id = __ldg(L.cids + k);
-                    hit = id < hit ? id : hit;
-                }
-                best = fmin(best, g);
+        const int64_t cell = cell_of(L, px, py);
+        const float4 *e = L.cells + kCellSlots * cell;
+        const float4 r0 = __ldg(e), r1 = __ldg(e + 1), r2 = __ldg(e + 2), r3 = __ldg(e + 3);
+        const int n = r3.x > kFarRect ? __float_as_int(r3.z) : 0;  // a longer list, or the tree
+        if (n >= 0) {
+            const double g0 = rect_gap(r0, px, py), g1 = rect_gap(r1, px, py), g2 = rect_gap(r2, px, py),
+                         g3 = rect_gap(r3, px, py);
+            best = dmin(best, dmin(dmin(g0, g1), dmin(g2, g3)));
+            C.first = (int)cell;
+            if (!(best > 0.0)) {  // p may lie in listed rects: the lowest layer index
+                const int4 id = __ldg(L.cellids + cell);
+                if (g0 <= 0.0) hit = min(hit, id.x);
+                if (g1 <= 0.0) hit = min(hit, id.y);
+                if (g2 <= 0.0) hit = min(hit, id.z);
+                if (g3 <= 0.0) hit = min(hit, id.w);
+            }
+            for (int k = kCellSlots - 1; k < n; k++) {  // the rest of a longer list
+                const int i = __float_as_int(r3.y) + k;
+                const double g = rect_gap(__ldg(L.crects + i), px, py);
+                if (g <= 0.0) hit = min(hit, __ldg(L.cids + i));
+                best = dmin(best, g);
             }
             return st;
         }
@@ -240,13 +263,24 @@ __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, c
 // boxes of the replay, see the file comment).  Only boxes within delta of the
 // clearance get here (rarely), so the listed rects are read back on demand
 // rather than held in registers through the whole replay.
+__device__ __forceinline__ bool touches_box(const float4 r, const double o[4]) {
+    return (double)r.z >= o[0] && o[2] >= (double)r.x && (double)r.w >= o[1] && o[3] >= (double)r.y;
+}
 __device__ __forceinline__ bool collides_listed(const DevLayout &L, const Cands &C, const double o[4]) {
     if (!(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1)) return true;
-    for (int q = 0; q < C.n; q++) {
-        const float4 r = __ldg(C.first >= 0 ? L.crects + C.first + q : L.rects + C.idx[q]);
-        if ((double)r.z >= o[0] && o[2] >= (double)r.x && (double)r.w >= o[1] && o[3] >= (double)r.y)
-            return true;
+    const float4 *r = L.rects;
+    int n = C.n;
+    if (C.first >= 0) {  // the cell's record, or its list when it has one (slots too far touch nothing)
+        r = L.cells + (int64_t)kCellSlots * C.first;
+        n = kCellSlots;
+        const float4 last = __ldg(r + kCellSlots - 1);
+        if (last.x > kFarRect) {
+            r = L.crects + __float_as_int(last.y);
+            n = __float_as_int(last.z);
+        }
     }
+    for (int q = 0; q < n; q++)
+        if (touches_box(__ldg(r + (C.first >= 0 ? q : C.idx[q])), o)) return true;
     return false;
 }
 
@@ -375,15 +409,23 @@ __device__ __forceinline__ void box_at(double px, double py, double h, double o[
 // above.  The reference first returns p +- 1 or p +- 2 when that box collides;
 // d* settles both unless it lies within delta of 1 or 2 (then the other of
 // the two is settled: it differs from d* by about 1), so one box is tested.
+// Points with d* = 1 or 2 exactly are common -- walks start one unit from
+// their target, and points truncated to int lie whole units from rects -- and
+// collide: with |p| >= 4 on both axes a difference x0 - p near h <= 2 is
+// exact (both are multiples of p's last place, 2^-50 or more), so the nearest
+// rect's gap <= h holds without rounding, p + h >= x0, and rounding p + h
+// keeps that.  Its test against the listed rects ran in nearly every round of
+// a warp (1e7 capacitance walks on 10^4 rects 2.22 -> 2.06 ms without it).  Not so where
+// the bounds, which a box may touch, are as near (bd: their distance).
 template <bool kTree = false>
 __device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cands &C, double px,
-                                                  double py, double dstar, double o[4]) {
+                                                  double py, double dstar, double bd, double o[4]) {
     uint32_t st = 0;
     const bool one = dstar < 1.5;
     const double h = one ? 1.0 : 2.0;
     box_at(px, py, h, o);
     const double e = __dsub_rn(dstar, h);
-    bool c = e < -L.delta;
+    bool c = e < -L.delta || (e <= 0.0 && bd > 3.0 && fabs(px) >= 4.0 && fabs(py) >= 4.0);
     if (!c && e <= L.delta) {  // rare: within delta of the clearance
         if (kTree)
             c = !(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1) ||
@@ -460,12 +502,12 @@ struct ReplayOut {
     uint32_t st;
 };
 static __device__ __noinline__ ReplayOut replay_tree_call(const DevLayout L, double px, double py,
-                                                          double dstar) {
+                                                          double dstar, double bd) {
     Cands C;
     C.n = 0;
     C.first = -2;
     ReplayOut r;
-    r.st = replay_square<true>(L, C, px, py, dstar, r.sq);
+    r.st = replay_square<true>(L, C, px, py, dstar, bd, r.sq);
     return r;
 }
 
@@ -477,13 +519,14 @@ __device__ __forceinline__ uint32_t query_point(const DevLayout &L, double px, d
                                                 int &hit, double bd = -1.0) {
     Cands C;
     double best;
+    if (!kInside) bd = fmin(fmin(px - L.bx0, L.bx1 - px), fmin(py - L.by0, L.by1 - py));
     uint32_t st = clearance<kInside, kOutOfLineTree, kTies>(L, px, py, C, hit, best, bd);
     if (kTies && C.first == -2) {
-        const ReplayOut r = replay_tree_call(L, px, py, best);
+        const ReplayOut r = replay_tree_call(L, px, py, best, bd);
         sq[0] = r.sq[0]; sq[1] = r.sq[1]; sq[2] = r.sq[2]; sq[3] = r.sq[3];
         st |= r.st;
     } else {
-        st |= replay_square(L, C, px, py, best, sq);
+        st |= replay_square(L, C, px, py, best, bd, sq);
     }
     return st;
 }
@@ -538,53 +581,42 @@ __device__ __forceinline__ double div200(double x) {
 }
 
 // RectHost::getPointFromNindex (CPU/rectHost.cpp:107-161; GPU twin
-// Cuda/d_Rect.cu:34-101): branch structure and operand order kept because
-// they decide ties; the perimeter is truncated to int unless `exact`.
+// Cuda/d_Rect.cu:34-101): its comparisons and operand order kept because they
+// decide ties; the perimeter is truncated to int unless `exact`.  The
+// reference branches seven ways (four sides and the corners between them),
+// and the lanes of a warp take them all, so the sides are computed without
+// branches -- the last two are the same operations on other operands -- and
+// the point selected (319 -> 290 warp instructions per walk on 10^6 rects
+// together with the cells' records).
 __device__ __forceinline__ void point_from_index(const double s[4], int index, bool exact, double &ox,
                                                  double &oy) {
-    const double per2 = __dadd_rn(__dmul_rn(2.0, __dsub_rn(s[2], s[0])), __dmul_rn(2.0, __dsub_rn(s[3], s[1])));
-    const double perim = exact ? per2 : (double)__double2int_rz(per2);
-    const double v = exact ? __ddiv_rn(perim, (double)FRW_NSAMPLE) : div200(perim);
     const double h = __dsub_rn(s[3], s[1]);
     const double w = __dsub_rn(s[2], s[0]);
+    const double w2 = __dmul_rn(2.0, w);
+    const double per2 = __dadd_rn(w2, __dmul_rn(2.0, h));
+    const double v = exact ? __ddiv_rn(per2, (double)FRW_NSAMPLE) : div200((double)__double2int_rz(per2));
     const double iv = __dmul_rn((double)index, v), jv = __dmul_rn((double)(index - 1), v);
     const double hv = __dmul_rn(v, 0.5);
-    const double wh = __dadd_rn(w, h), w2h = __dadd_rn(__dmul_rn(2.0, w), h);
-    if (iv < w) {
-        ox = (double)__double2int_rz(__dadd_rn(__dadd_rn(jv, hv), s[0]));
-        oy = s[1];
-    } else if (jv < w && iv > w) {
-        ox = s[2];
-        oy = s[1];
-    } else if (iv < wh) {
-        ox = s[2];
-        if (jv > w) oy = __dadd_rn(__dsub_rn(__dadd_rn(s[1], jv), w), hv);
-        else {
-            const double t = __dsub_rn(iv, w);
-            oy = __dadd_rn(__dsub_rn(__dadd_rn(s[1], iv), w), __dmul_rn(t, 0.5));
-        }
-    } else if (jv < wh && iv > wh) {
-        ox = s[2];
-        oy = s[3];
-    } else if (iv < w2h) {
-        oy = s[3];
-        if (jv > wh) ox = __dsub_rn(s[2], __dadd_rn(__dsub_rn(__dsub_rn(jv, w), h), hv));
-        else {
-            const double t = __dsub_rn(__dsub_rn(iv, w), h);
-            ox = __dsub_rn(s[2], __dadd_rn(t, __dmul_rn(t, 0.5)));
-        }
-    } else if (jv < w2h && iv > w2h) {
-        ox = s[0];
-        oy = s[3];
-    } else {
-        ox = s[0];
-        const double w2 = __dmul_rn(2.0, w);
-        if (jv > w2h) oy = __dsub_rn(s[3], __dadd_rn(__dsub_rn(__dsub_rn(jv, w2), h), hv));
-        else {
-            const double t = __dsub_rn(__dsub_rn(iv, w2), h);
-            oy = __dsub_rn(s[3], __dadd_rn(t, __dmul_rn(t, 0.5)));
-        }
-    }
+    const double wh = __dadd_rn(w, h), w2h = __dadd_rn(w2, h);
+    // where the index lies, in the reference's order of tests: top, its corner
+    // with the right side, right, corner, bottom, corner, left
+    const int at = iv < w ? 0
+                 : jv < w && iv > w ? 1
+                 : iv < wh ? 2
+                 : jv < wh && iv > wh ? 3
+                 : iv < w2h ? 4
+                 : jv < w2h && iv > w2h ? 5 : 6;
+    // top: truncated to int
+    const double top = (double)__double2int_rz(__dadd_rn(__dadd_rn(jv, hv), s[0]));
+    // right
+    const bool m2 = jv > w;
+    const double right = __dadd_rn(__dsub_rn(__dadd_rn(s[1], m2 ? jv : iv), w), m2 ? hv : __dmul_rn(__dsub_rn(iv, w), 0.5));
+    // bottom (from the right end, after w and h) or left (from the bottom end, after 2w and h)
+    const bool bottom = at == 4, m3 = jv > (bottom ? wh : w2h);
+    const double t = __dsub_rn(__dsub_rn(m3 ? jv : iv, bottom ? w : w2), h);
+    const double back = __dsub_rn(bottom ? s[2] : s[3], __dadd_rn(t, m3 ? hv : __dmul_rn(t, 0.5)));
+    ox = at == 0 ? top : at < 4 ? s[2] : bottom ? back : s[0];
+    oy = at < 2 ? s[1] : at == 2 ? right : at < 6 ? s[3] : back;
 }
 
 // Uniform point on the Gaussian perimeter, clockwise from the top-left

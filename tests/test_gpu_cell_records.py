@@ -1,0 +1,64 @@
+"""Cell records at the edges of their format: cells that list up to four rects
+keep them in place, longer lists go to the shared buffer (also when it has to
+grow), capped cells to the tree.  Queries equal the oracle's."""
+import numpy as np
+import pytest
+
+import frw
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def row_of(k, side=2.0, gap=4.0):
+    """k rects of one size around a centre, all about as near to it."""
+    a = np.arange(k) * 2 * np.pi / k
+    c = np.stack([200 + np.round(60 * np.cos(a)), 200 + np.round(60 * np.sin(a))], 1)
+    return np.concatenate([c, c + side], 1)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 9, 31, 32, 33])
+def test_record_of_k_rects(k):
+    r = row_of(k)
+    b = np.array([0.0, 0.0, 400.0, 400.0])
+    rng = np.random.default_rng(k)
+    p = np.concatenate([rng.uniform(0, 400, (4000, 2)), r[rng.integers(0, k, 500), :2], rng.uniform(190, 210, (500, 2))])
+    ref, hit_ref = O.Grid(r, b).query_batch(p)
+    with frw.Layout.from_rects(r, b) as L:
+        for cells_per_rect in (16.0, 0.2, 400.0):
+            L.set_cells(cells_per_rect)
+            sq, hit = L.query(p)
+            assert np.array_equal(sq, ref) and np.array_equal(hit, hit_ref)
+
+
+def test_overlapping_rects_report_the_lowest_index():
+    """Nested rects share their cells: the lowest layer index wins in a record
+    and in a longer list."""
+    for k in (3, 4, 5, 20):
+        i = np.arange(k)[::-1, None] * 1.0  # the smallest rect has the highest index
+        r = np.concatenate([100 - i, 100 - i, 110 + i, 110 + i], 1)
+        b = np.array([0.0, 0.0, 220.0, 220.0])
+        p = np.random.default_rng(3).uniform(70, 140, (3000, 2))
+        ref, hit_ref = O.Grid(r, b).query_batch(p)
+        with frw.Layout.from_rects(r, b) as L:
+            sq, hit = L.query(p)
+            assert np.array_equal(sq, ref) and np.array_equal(hit, hit_ref)
+
+
+def test_lists_past_the_first_buffer():
+    """A dense block in wide bounds: nearly every cell sees dozens of rects, more
+    list entries than cells, so the lists take a second pass."""
+    gx, gy = np.meshgrid(np.arange(24) * 3.0, np.arange(24) * 3.0)
+    r = np.stack([gx.ravel(), gy.ravel(), gx.ravel() + 1, gy.ravel() + 1], 1) + 5000.0
+    b = np.array([0.0, 0.0, 10000.0, 10000.0])
+    rng = np.random.default_rng(9)
+    p = np.concatenate([rng.uniform(0, 10000, (3000, 2)), rng.uniform(4990, 5090, (3000, 2))])
+    ref, hit_ref = O.Grid(r, b).query_batch(p)
+    with frw.Layout.from_rects(r, b) as L:
+        for cells_per_rect, cap in ((0.5, 600), (16.0, 600), (200.0, 600), (200.0, 32)):
+            L.set_cells(cells_per_rect, cap)
+            c = L.cells
+            if cap == 600:
+                assert c.overflow_cells == 0 and c.entries > c.cells
+            sq, hit = L.query(p)
+            assert np.array_equal(sq, ref) and np.array_equal(hit, hit_ref)
