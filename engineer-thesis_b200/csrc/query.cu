@@ -4,23 +4,37 @@
 namespace frw {
 namespace {
 
+// A square in one 256-bit store (32-byte aligned), past the caches that the
+// cells want.
+__device__ __forceinline__ void store_square(double4 *p, const double s[4]) {
+    asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(s[0]), "d"(s[1]), "d"(s[2]), "d"(s[3])
+                 : "memory");
+}
+
 // One point per thread: drawBiggestSquareAtPoint + checkCollisons(point),
 // batched (the reference issues them one walk hop at a time,
 // Cuda/randomwalk.cu:102-103).  kTies: L.tree_points is set, so points with
 // many exact ties can reach the whole-tree replay (compiled out otherwise).
+// Random points: bound by the reads of their records, in L2 for 10^4 rects (a
+// warp's 32 records are 64 separate 32-byte reads; 16-byte reads doubled the
+// L1 lookups, 1e7 points 0.304 -> 0.228 ms; 12 blocks per SM against 10:
+// 0.240, 16 spill: 0.242) and in HBM for 10^6 (150 bytes read and 40 written
+// per point, 0.545 -> 0.453 ms).  Records fetched ahead of their points --
+// through shared memory by asynchronous copies, or the coordinates alone in a
+// persistent grid -- were slower (1.05 and 0.59 ms).
 template <bool kTies>
-__global__ void __launch_bounds__(128) k_query(DevLayout L, const double2 *__restrict__ pts, int64_t n,
-                                               double4 *__restrict__ sq, int64_t *__restrict__ hit,
-                                               uint32_t *status) {
+__global__ void __launch_bounds__(128, kTies ? 8 : 12)
+    k_query(DevLayout L, const double2 *__restrict__ pts, int64_t n, double4 *__restrict__ sq,
+            int64_t *__restrict__ hit, uint32_t *status) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t st = 0;
     if (i < n) {
-        const double2 p = pts[i];
+        const double2 p = __ldcs(pts + i);
         double s[4];
         int h;
         st = query_point<false, false, kTies>(L, p.x, p.y, s, h);
-        sq[i] = make_double4(s[0], s[1], s[2], s[3]);
-        hit[i] = h == kNoHit ? -1 : (int64_t)h;
+        store_square(sq + i, s);
+        __stcs((long long *)hit + i, h == kNoHit ? -1ll : (long long)h);
     }
     if (st) atomicOr(status, st);
 }

@@ -192,6 +192,40 @@ __device__ __forceinline__ int64_t cell_of(const DevLayout &L, double px, double
     return (int64_t)iy * L.gnx + ix;
 }
 
+// Two neighbouring rects of a record in one 256-bit read (32-byte aligned).
+__device__ __forceinline__ void load_pair(const float4 *p, float4 &a, float4 &b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// The clearance of p from its cell's record r0 .. r3 (best: the bounds
+// distance so far, hit: kNoHit).  False when the tree answers the cell.
+__device__ __forceinline__ bool record_clearance(const DevLayout &L, int64_t cell, const float4 r0, const float4 r1,
+                                                 const float4 r2, const float4 r3, double px, double py, Cands &C,
+                                                 int &hit, double &best) {
+    const int n = r3.x > kFarRect ? __float_as_int(r3.z) : 0;  // a longer list, or the tree
+    if (n < 0) return false;
+    const double g0 = rect_gap(r0, px, py), g1 = rect_gap(r1, px, py), g2 = rect_gap(r2, px, py),
+                 g3 = rect_gap(r3, px, py);
+    best = dmin(best, dmin(dmin(g0, g1), dmin(g2, g3)));
+    C.first = (int)cell;
+    if (!(best > 0.0)) {  // p may lie in listed rects: the lowest layer index
+        const int4 id = __ldg(L.cellids + cell);
+        if (g0 <= 0.0) hit = min(hit, id.x);
+        if (g1 <= 0.0) hit = min(hit, id.y);
+        if (g2 <= 0.0) hit = min(hit, id.z);
+        if (g3 <= 0.0) hit = min(hit, id.w);
+    }
+    for (int k = kCellSlots - 1; k < n; k++) {  // the rest of a longer list
+        const int i = __float_as_int(r3.y) + k;
+        const double g = rect_gap(__ldg(L.crects + i), px, py);
+        if (g <= 0.0) hit = min(hit, __ldg(L.cids + i));
+        best = dmin(best, g);
+    }
+    return true;
+}
+
 // The clearance of p and its near-tie list.  With cell lists the list of
 // p's cell holds every rect that can come within 2*delta of the clearance of
 // any point of the cell (the cell's radius is bounded by the clearance of
@@ -227,29 +261,10 @@ __device__ __forceinline__ uint32_t clearance(const DevLayout &L, double px, dou
     }
     if (L.cells) {
         const int64_t cell = cell_of(L, px, py);
-        const float4 *e = L.cells + kCellSlots * cell;
-        const float4 r0 = __ldg(e), r1 = __ldg(e + 1), r2 = __ldg(e + 2), r3 = __ldg(e + 3);
-        const int n = r3.x > kFarRect ? __float_as_int(r3.z) : 0;  // a longer list, or the tree
-        if (n >= 0) {
-            const double g0 = rect_gap(r0, px, py), g1 = rect_gap(r1, px, py), g2 = rect_gap(r2, px, py),
-                         g3 = rect_gap(r3, px, py);
-            best = dmin(best, dmin(dmin(g0, g1), dmin(g2, g3)));
-            C.first = (int)cell;
-            if (!(best > 0.0)) {  // p may lie in listed rects: the lowest layer index
-                const int4 id = __ldg(L.cellids + cell);
-                if (g0 <= 0.0) hit = min(hit, id.x);
-                if (g1 <= 0.0) hit = min(hit, id.y);
-                if (g2 <= 0.0) hit = min(hit, id.z);
-                if (g3 <= 0.0) hit = min(hit, id.w);
-            }
-            for (int k = kCellSlots - 1; k < n; k++) {  // the rest of a longer list
-                const int i = __float_as_int(r3.y) + k;
-                const double g = rect_gap(__ldg(L.crects + i), px, py);
-                if (g <= 0.0) hit = min(hit, __ldg(L.cids + i));
-                best = dmin(best, g);
-            }
-            return st;
-        }
+        float4 r0, r1, r2, r3;
+        load_pair(L.cells + kCellSlots * cell, r0, r1);
+        load_pair(L.cells + kCellSlots * cell + 2, r2, r3);
+        if (record_clearance(L, cell, r0, r1, r2, r3, px, py, C, hit, best)) return st;
     }
     if (kOutOfLineTree)
         return tree_clearance_call<kTies>(L.nbox, L.nref, L.rects, L.ids, px, py, r2, L.slack, C, hit, best);
