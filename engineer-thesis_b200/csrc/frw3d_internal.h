@@ -45,6 +45,7 @@ struct Dev3Layout {
     double g0x, g0y, g0z;  // grid origin (every level)
     double ginv;           // 1 / cell side
     double hq;             // half a cell side + rounding margin
+    float fslack;          // absolute part of the FP32 screen's error (nearest3)
     int nx, ny, nz;
     int nup;               // coarser levels
     const Level3 *up;      // [nup] device array
