@@ -236,21 +236,10 @@ frw_status prepare_walk(const frw3_layout *L, int64_t target, uint64_t first, ui
     return FRW_OK;
 }
 
-int walk_blocks(int dev, int bps_opt) {
+int sm_count(int dev) {
     const double *t2;
     int sms = 148;
-    if (device_tables(dev, &t2, &sms) != FRW_OK) sms = 148;
-    static std::mutex mu;
-    static std::map<int, int> bps_cache;
-    int bps;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = bps_cache.find(dev);
-        if (it == bps_cache.end()) it = bps_cache.emplace(dev, walk3_max_blocks_per_sm()).first;
-        bps = it->second;
-    }
-    if (bps_opt > 0) bps = std::min(bps, bps_opt);
-    return sms * bps;
+    return device_tables(dev, &t2, &sms) == FRW_OK ? sms : 148;
 }
 
 }  // namespace
@@ -515,7 +504,7 @@ frw_status frw3_walk(const frw3_layout *L, int64_t target, uint64_t walks, uint6
     if (!ev.ok(2)) return cuda_fail(cudaErrorUnknown, "event create");
     FRW_CK(cudaEventRecord(ev[0], st));
     if (walks > 0) {
-        rc = launch_walk3(P, walk_blocks(L->device, o->blocks_per_sm), st);
+        rc = launch_walk3(P, sm_count(L->device), o->blocks_per_sm, st);
         if (rc) return rc;
     }
     FRW_CK(cudaEventRecord(ev[1], st));
@@ -585,7 +574,7 @@ frw_status frw3_walk_device(const frw3_layout *L, int64_t target, uint64_t walks
     P.sum_w2 = sum_w2;
     P.stats = (unsigned long long *)stats;
     P.L.status = status;  // lookup failures go to the caller's word
-    return launch_walk3(P, walk_blocks(L->device, o.blocks_per_sm), st);
+    return launch_walk3(P, sm_count(L->device), o.blocks_per_sm, st);
 }
 
 frw_status frw3_walk_batch(const frw3_layout *L, const int64_t *targets, int32_t ntargets, uint64_t walks_per_target,
@@ -654,7 +643,7 @@ frw_status frw3_walk_batch(const frw3_layout *L, const int64_t *targets, int32_t
     if (!ev.ok(2)) return cuda_fail(cudaErrorUnknown, "event create");
     FRW_CK(cudaEventRecord(ev[0], st));
     if (total > 0) {
-        rc = launch_walk3_batch(P, walk_blocks(L->device, o.blocks_per_sm), st);
+        rc = launch_walk3_batch(P, sm_count(L->device), o.blocks_per_sm, st);
         if (rc) return rc;
     }
     FRW_CK(cudaEventRecord(ev[1], st));
@@ -745,7 +734,7 @@ frw_status frw3_walk_trace(const frw3_layout *L, int64_t target, uint64_t first_
         set_error("frw3_walk_trace: no output array");
         return FRW_E_ARG;
     }
-    rc = launch_walk3(P, walk_blocks(L->device, o->blocks_per_sm), st);
+    rc = launch_walk3(P, sm_count(L->device), o->blocks_per_sm, st);
     if (rc) return rc;
     rc = wait_stream(st, "frw3_walk_trace");
     if (rc) return rc;

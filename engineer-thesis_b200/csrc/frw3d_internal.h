@@ -114,6 +114,7 @@ struct Walk3Params {
     uint64_t seed;
     uint32_t stream;
     uint64_t first, walks;
+    uint32_t chunk;  // walks a warp claims at a time (set by the launch)
     unsigned long long *counter;  // walks claimed (cleared by the caller)
     // rows (capacitance mode): per box, plus stats[4] = escaped, aborted, hops, walks
     unsigned long long *hits;
@@ -147,9 +148,8 @@ void free_grid3(Grid3Buffers *g, cudaStream_t stream);
 void attach_grid3(Dev3Layout &L, const Grid3Buffers &g, const double bounds[6]);
 frw_status launch_query3(const Dev3Layout &L, const double *d_pts, int64_t n, double *d_clear,
                          int64_t *d_nearest, cudaStream_t stream);
-frw_status launch_walk3(const Walk3Params &P, int blocks, cudaStream_t stream);
-frw_status launch_walk3_batch(const Walk3Params &P, int blocks, cudaStream_t stream);
-int walk3_max_blocks_per_sm();
-int walk3_threads();
+// blocks_per_sm: resident blocks of 256 threads, 0 for the library's choice.
+frw_status launch_walk3(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t stream);
+frw_status launch_walk3_batch(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t stream);
 
 }  // namespace frw

@@ -107,7 +107,7 @@ struct WalkParams {
     double permittivity;
     uint64_t seed;
     const uint64_t *seed_dev;  // when set, the seed is read here (captured graphs replay with new seeds)
-    uint32_t chunk;            // walks a warp claims per global atomic (0: 128)
+    uint32_t chunk;            // walks a warp claims per global atomic (0: chosen by the launch)
     uint64_t total_walks;
     unsigned long long *counter;  // global walk counter (refill)
     // per-conductor accumulators (dense rows, acc_base + layer index)

@@ -34,10 +34,16 @@
 namespace frw {
 namespace {
 
+// Two launch shapes of 32 warps per SM at 64 registers: four blocks of 256,
+// or one of 1024 that also holds the CDF thresholds in shared memory (60 KB at
+// n = 50, read at a random place in every hop: from L1 they competed with the
+// cells' lists, 78 -> 92% hits without them; 1e7 walks on 10^4 boxes 4.10 ->
+// 3.47 ms, four rows of 10^5 boxes 1.10 -> 0.99 ms).
 constexpr int kW3Threads = 256;
 constexpr int kW3MinBlocks = 4;
+constexpr int kW3BigThreads = 1024;
+constexpr size_t kW3ThrBytes = 96 << 10;  // thresholds that fit beside the guide (n <= 64)
 constexpr unsigned kFull = 0xFFFFFFFFu;
-constexpr uint64_t kW3Chunk = 128;  // walks a warp claims at a time
 constexpr int64_t kMaxCells3 = int64_t(1) << 26;
 constexpr int kMaxAxisCells3 = 1 << 14;
 
@@ -516,10 +522,14 @@ __device__ __forceinline__ void flush_job(const Walk3Params &P, int job, unsigne
     ts = ts2 = 0.0;
 }
 
-template <bool kMulti>
-__global__ void __launch_bounds__(kW3Threads, kW3MinBlocks) k_walk3(const Walk3Params P) {
+template <bool kMulti, bool kBig>
+__global__ void __launch_bounds__(kBig ? kW3BigThreads : kW3Threads, kBig ? 1 : kW3MinBlocks)
+    k_walk3(const Walk3Params P) {
     __shared__ uint16_t s_guide[1 << kGuide3Bits];
     __shared__ double s_offs[FRW3_NSAMPLE_MAX];
+    extern __shared__ uint32_t s_thr[];  // kBig: the nb thresholds
+    if (kBig)
+        for (int k = threadIdx.x; k < P.nb; k += blockDim.x) s_thr[k] = P.thr[k];
     for (int k = threadIdx.x; k < (1 << kGuide3Bits); k += blockDim.x) s_guide[k] = P.guide[k];
     for (int k = threadIdx.x; k < P.n; k += blockDim.x) s_offs[k] = P.offs[k];
     __syncthreads();
@@ -544,14 +554,14 @@ __global__ void __launch_bounds__(kW3Threads, kW3MinBlocks) k_walk3(const Walk3P
         while (idle && !exhausted) {
             if (next >= cend) {
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(P.counter, (unsigned long long)kW3Chunk);
+                if (lane == 0) base = atomicAdd(P.counter, (unsigned long long)P.chunk);
                 base = __shfl_sync(kFull, base, 0);
                 if (base >= P.walks) {
                     exhausted = true;
                     break;
                 }
                 next = (uint64_t)base;
-                cend = next + kW3Chunk < P.walks ? next + kW3Chunk : P.walks;
+                cend = next + P.chunk < P.walks ? next + P.chunk : P.walks;
             }
             const uint64_t avail = cend - next;
             const unsigned rank = __popc(idle & lt);
@@ -591,7 +601,7 @@ __global__ void __launch_bounds__(kW3Threads, kW3MinBlocks) k_walk3(const Walk3P
             if (pass == 2) W.rnd = block3(P, P.first + W.idx, t >> 2);
             const uint32_t x = word_of(W.rnd, t);
             int b = s_guide[x >> (32 - kGuide3Bits)];
-            while (b + 1 < P.nb && __ldg(P.thr + b + 1) <= x) b++;
+            while (b + 1 < P.nb && (kBig ? s_thr[b + 1] : __ldg(P.thr + b + 1)) <= x) b++;
             land(P, s_offs, W, b, d);
             if (W.hops == 1) {
                 W.b1 = b;
@@ -931,24 +941,39 @@ frw_status launch_query3(const Dev3Layout &L, const double *d_pts, int64_t n, do
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k3_query");
 }
 
-frw_status launch_walk3(const Walk3Params &P, int blocks, cudaStream_t st) {
-    k_walk3<false><<<blocks, kW3Threads, 0, st>>>(P);
+namespace {
+// One block of 1024 per SM from one walk per lane on (300,000 walks: 0.306 ms
+// against 0.331 in blocks of 256; 100,000: 0.246 and 0.247, and small runs
+// spread over more SMs in small blocks), unless the caller asks for a number of
+// blocks or the table is too long.  A warp claims 32 walks at a time in runs of
+// a few walks per lane -- claims of 128 put four walks one after another on a
+// lane: 30,000 walks 0.37 -> 0.22 ms -- and 128 in long ones.
+template <bool kMulti>
+frw_status launch_walk3_as(Walk3Params P, int sms, int bps, cudaStream_t st) {
+    const size_t thr = (size_t)P.nb * sizeof(uint32_t);
+    const uint64_t warps = (uint64_t)sms * (kW3BigThreads / 32);
+    const bool big = bps == 0 && thr <= kW3ThrBytes && P.walks >= warps * 32;
+    P.chunk = P.walks < warps * 128 ? 32 : 128;
+    if (big) {
+        cudaError_t e = cudaFuncSetAttribute(k_walk3<kMulti, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)thr);
+        if (e != cudaSuccess) return cuda_fail(e, "k_walk3: shared memory");
+        k_walk3<kMulti, true><<<sms, kW3BigThreads, thr, st>>>(P);
+    } else {
+        const uint64_t need = std::max<uint64_t>((P.walks + kW3Threads - 1) / kW3Threads, 1);
+        const int full = sms * (bps > 0 ? std::min(bps, kW3MinBlocks) : kW3MinBlocks);
+        k_walk3<kMulti, false><<<(unsigned)std::min<uint64_t>(need, full), kW3Threads, 0, st>>>(P);
+    }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k_walk3");
 }
+}  // namespace
 
-frw_status launch_walk3_batch(const Walk3Params &P, int blocks, cudaStream_t st) {
-    k_walk3<true><<<blocks, kW3Threads, 0, st>>>(P);
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k_walk3 batch");
+frw_status launch_walk3(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t st) {
+    return launch_walk3_as<false>(P, sms, blocks_per_sm, st);
 }
 
-int walk3_max_blocks_per_sm() {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_walk3<false>, kW3Threads, 0) != cudaSuccess) return 1;
-    return std::max(b, 1);
+frw_status launch_walk3_batch(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t st) {
+    return launch_walk3_as<true>(P, sms, blocks_per_sm, st);
 }
-
-int walk3_threads() { return kW3Threads; }
 
 }  // namespace frw
