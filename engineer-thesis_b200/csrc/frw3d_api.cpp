@@ -83,74 +83,6 @@ frw_status device_cube_tables(int dev, int n, const Cube3Tables **out) {
 
 bool fp32_exact3(double v) { return std::isfinite(v) && (double)(float)v == v && fabs(v) < 16777216.0; }
 
-// Interiors pairwise disjoint (touching faces allowed): boxes are binned
-// into a hash grid of cells about one box across (count -> prefix -> fill),
-// and the boxes sharing a cell are compared pairwise.
-frw_status check_disjoint(const float *b, int64_t n) {
-    double emax = 0, lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int64_t i = 0; i < n; i++)
-        for (int c = 0; c < 3; c++) {
-            emax = std::max(emax, (double)b[6 * i + 3 + c] - b[6 * i + c]);
-            lo[c] = std::min(lo[c], (double)b[6 * i + c]);
-            hi[c] = std::max(hi[c], (double)b[6 * i + 3 + c]);
-        }
-    double vol = 1.0;
-    for (int c = 0; c < 3; c++) vol *= std::max(hi[c] - lo[c], 1e-30);
-    double cs = std::max(emax, std::cbrt(vol / (double)n));
-    int64_t nc[3], total;
-    for (;;) {
-        total = 1;
-        for (int c = 0; c < 3; c++) {
-            nc[c] = std::max<int64_t>(1, (int64_t)floor((hi[c] - lo[c]) / cs) + 1);
-            total *= nc[c];
-        }
-        if (total <= 8 * n + 64) break;
-        cs *= 1.25;
-    }
-    auto range = [&](const float *p, int64_t c0[3], int64_t c1[3]) {
-        for (int c = 0; c < 3; c++) {
-            c0[c] = std::min(nc[c] - 1, (int64_t)floor((p[c] - lo[c]) / cs));
-            c1[c] = std::min(nc[c] - 1, (int64_t)floor((p[3 + c] - lo[c]) / cs));
-        }
-    };
-    std::vector<int64_t> start((size_t)total + 1, 0);
-    std::vector<int32_t> items;
-    for (int pass = 0; pass < 2; pass++) {
-        for (int64_t i = 0; i < n; i++) {
-            int64_t c0[3], c1[3];
-            range(b + 6 * i, c0, c1);
-            for (int64_t z = c0[2]; z <= c1[2]; z++)
-                for (int64_t y = c0[1]; y <= c1[1]; y++)
-                    for (int64_t x = c0[0]; x <= c1[0]; x++) {
-                        const int64_t cell = (z * nc[1] + y) * nc[0] + x;
-                        if (pass == 0) start[(size_t)cell + 1]++;
-                        else items[(size_t)start[(size_t)cell]++] = (int32_t)i;
-                    }
-        }
-        if (pass == 0) {
-            for (int64_t c = 0; c < total; c++) start[(size_t)c + 1] += start[(size_t)c];
-            items.resize((size_t)start[(size_t)total]);
-        } else {
-            for (int64_t c = total; c > 0; c--) start[(size_t)c] = start[(size_t)c - 1];
-            start[0] = 0;
-        }
-    }
-    for (int64_t cell = 0; cell < total; cell++)
-        for (int64_t u = start[(size_t)cell]; u < start[(size_t)cell + 1]; u++)
-            for (int64_t v = u + 1; v < start[(size_t)cell + 1]; v++) {
-                const int32_t i = items[(size_t)u], j = items[(size_t)v];
-                const float *p = b + 6 * (int64_t)i, *q = b + 6 * (int64_t)j;
-                bool ov = true;
-                for (int c = 0; c < 3 && ov; c++) ov = p[c] < q[3 + c] && q[c] < p[3 + c];
-                if (ov) {
-                    set_error("boxes " + std::to_string(std::min(i, j)) + " and " + std::to_string(std::max(i, j)) +
-                              " overlap");
-                    return FRW_E_ARG;
-                }
-            }
-    return FRW_OK;
-}
-
 frw_status check_opts3(const frw3_opts *o) {
     if (!o || o->struct_size != sizeof(frw3_opts)) {
         set_error("frw3_opts.struct_size mismatch (call frw3_opts_default)");
@@ -292,30 +224,42 @@ frw_status frw3_layout_create(const float *boxes, int64_t n, const double *bound
     int sms;
     frw_status rc = device_tables(device, &t2, &sms);
     if (rc) return rc;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY}, emin = INFINITY;
-    for (int64_t i = 0; i < n; i++) {
-        const float *q = boxes + 6 * i;
-        for (int c = 0; c < 3; c++) {
-            if (!fp32_exact3(q[c]) || !fp32_exact3(q[3 + c])) {
-                set_error("box " + std::to_string(i) + ": coordinate not finite or |c| >= 2^24");
-                return FRW_E_ARG;
-            }
-            if (!(q[c] < q[3 + c])) {
-                set_error("box " + std::to_string(i) + ": empty or inverted (need x0 < x1, y0 < y1, z0 < z1)");
-                return FRW_E_ARG;
-            }
-            lo[c] = std::min(lo[c], (double)q[c]);
-            hi[c] = std::max(hi[c], (double)q[3 + c]);
-            emin = std::min(emin, (double)q[3 + c] - (double)q[c]);
-        }
-    }
-    rc = check_disjoint(boxes, n);
-    if (rc) return rc;
     auto L = std::make_unique<frw3_layout>();
     L->device = device;
     L->n = n;
-    L->boxes.assign(boxes, boxes + 6 * n);
-    L->min_edge = emin;
+    Dev3Guard g(device);
+    cudaStream_t st = nullptr;
+    const size_t bytes = (size_t)n * 6 * sizeof(float);
+    Scratch3 upload(st), checks(st);  // released in stream order on errors
+    FRW_CK(cudaMallocAsync(&upload.p, bytes, st));
+    FRW_CK(cudaMallocAsync(&checks.p, sizeof(BoxCheck), st));
+    float *d_boxes = (float *)upload.p;
+    BoxCheck *d_chk = (BoxCheck *)checks.p, chk;
+    cudaError_t e = cudaMemcpyAsync(d_boxes, boxes, bytes, cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return cuda_fail(e, "upload boxes");
+    if ((rc = check_boxes3(d_boxes, n, sms, st, d_chk))) return rc;
+    L->boxes.assign(boxes, boxes + 6 * n);  // while the device checks them
+    if ((rc = read_back(&chk, d_chk, sizeof(chk), st, "frw3_layout_create: checks"))) return rc;
+    if (chk.bad != ~0ull) {
+        set_error("box " + std::to_string(chk.bad >> 2) +
+                  ((chk.bad & 3) == 1 ? ": coordinate not finite or |c| >= 2^24"
+                                      : ": empty or inverted (need x0 < x1, y0 < y1, z0 < z1)"));
+        return FRW_E_ARG;
+    }
+    double lo[3], hi[3], emax;
+    for (int c = 0; c < 3; c++) {
+        lo[c] = (double)key_value(chk.lo[c]);
+        hi[c] = (double)key_value(chk.hi[c]);
+    }
+    memcpy(&L->min_edge, &chk.emin, 8);
+    memcpy(&emax, &chk.emax, 8);
+    if ((rc = check_disjoint3(d_boxes, n, lo, hi, emax, st, d_chk))) return rc;
+    if ((rc = read_back(&chk, d_chk, sizeof(chk), st, "frw3_layout_create: overlaps"))) return rc;
+    if (chk.pair != ~0ull) {
+        set_error("boxes " + std::to_string(chk.pair >> 32) + " and " + std::to_string(chk.pair & 0xFFFFFFFFu) +
+                  " overlap");
+        return FRW_E_ARG;
+    }
     if (bounds) {
         for (int c = 0; c < 3; c++) {
             if (!(bounds[c] < bounds[3 + c]) || !std::isfinite(bounds[c]) || !std::isfinite(bounds[3 + c]) ||
@@ -333,20 +277,9 @@ frw_status frw3_layout_create(const float *boxes, int64_t n, const double *bound
             L->bounds[3 + c] = hi[c] + add;
         }
     }
-    Dev3Guard g(device);
-    cudaStream_t st = nullptr;
-    const size_t bytes = (size_t)n * 6 * sizeof(float);
-    FRW_CK(cudaMallocAsync(&L->d_boxes, bytes, st));
-    cudaError_t e = cudaMemcpyAsync(L->d_boxes, boxes, bytes, cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(L->d_boxes, st);
-        return cuda_fail(e, "upload boxes");
-    }
-    rc = build_grid3(L->d_boxes, n, L->bounds, cells_per_box > 0 ? cells_per_box : 8.0, st, &L->grid);
-    if (rc) {
-        cudaFreeAsync(L->d_boxes, st);  // stream-ordered: after any build work still queued
-        return rc;
-    }
+    if ((rc = build_grid3(d_boxes, n, L->bounds, cells_per_box > 0 ? cells_per_box : 8.0, st, &L->grid))) return rc;
+    L->d_boxes = d_boxes;
+    upload.p = nullptr;  // the layout's now
     attach_grid3(L->dl, L->grid, L->bounds);
     *out = L.release();
     return FRW_OK;

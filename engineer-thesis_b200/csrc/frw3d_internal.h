@@ -142,6 +142,18 @@ void cube_deriv_point(double *dg, double a, double eta, double dzeta);
 bool cube_walk_tables(int n, uint32_t *thr, uint16_t *guide, double *w, double *offs);
 
 // walk3d.cu
+// Device checks of a layout's boxes (float[6] each): bad = min of (index << 2 |
+// reason), all ones when every box is finite, below 2^24 and not empty; lo / hi:
+// f_key of the extent; emin / emax: bits of the shortest and longest edge; pair
+// = an overlapping pair i << 32 | j, i < j, all ones when disjoint.
+struct BoxCheck {
+    unsigned long long bad, emin, emax, pair;
+    unsigned lo[3], hi[3];
+};
+// Neither waits: the caller reads *d_out back.
+frw_status check_boxes3(const float *d_boxes, int64_t n, int sms, cudaStream_t stream, BoxCheck *d_out);
+frw_status check_disjoint3(const float *d_boxes, int64_t n, const double lo[3], const double hi[3], double emax,
+                           cudaStream_t stream, BoxCheck *d_out);
 frw_status build_grid3(const float *d_boxes, int64_t n, const double bounds[6], double cells_per_box,
                        cudaStream_t stream, Grid3Buffers *out);
 void free_grid3(Grid3Buffers *g, cudaStream_t stream);

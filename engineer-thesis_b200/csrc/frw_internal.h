@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 
@@ -205,6 +206,20 @@ struct TreeBuffers {
     int32_t nodes = 0, depth = 0;
     int64_t bytes = 0;
 };
+// Order-preserving unsigned key of a float (+0 for -0): unsigned order of the
+// keys is the order of the values.
+#if defined(__CUDACC__)
+__device__ __forceinline__ unsigned f_key(float f) {
+    const unsigned u = __float_as_uint(f + 0.0f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+#endif
+inline float key_value(unsigned k) {
+    const unsigned u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
+    float f;
+    memcpy(&f, &u, 4);
+    return f;
+}
 // Device check of a layout's rects (finite, |c| < 2^24, x0 <= x1 and
 // y0 <= y1, inside `given` when not null) and the extent of the rects:
 // bad = index of the first offending rect (-1: none) and why its reason

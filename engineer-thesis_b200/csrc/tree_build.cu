@@ -392,13 +392,6 @@ __global__ void __launch_bounds__(1024) k_build_small(const uint32_t *__restrict
     }
 }
 
-// Order-preserving unsigned key of a float (+0 for -0): unsigned order of
-// the keys is the order of the values.
-__device__ __forceinline__ unsigned f_key(float f) {
-    const unsigned u = __float_as_uint(f + 0.0f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-
 // Checks every rect (finite, |c| < 2^24, not inverted, inside the given
 // bounds when there are any) and reduces the extent of the valid ones:
 // out->bad = min over bad rects of (index << 2 | reason), out->key = keys of
@@ -461,13 +454,6 @@ __global__ void __launch_bounds__(256) k_check_rects(const float4 *__restrict__ 
         atomicMax(&out->key[3], k3);
         if (bad != ~0ull) atomicMin(&out->bad, bad);
     }
-}
-
-float key_value(unsigned k) {
-    const unsigned u = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
-    float f;
-    memcpy(&f, &u, 4);
-    return f;
 }
 
 }  // namespace

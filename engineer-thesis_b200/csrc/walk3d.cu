@@ -120,6 +120,82 @@ __global__ void k3_bin_fill(const float *__restrict__ boxes, int64_t n, Grid3 G,
                 items[atomicAdd(cursor + ((int64_t)z * G.n[1] + y) * G.n[0] + x, 1ull)] = (int32_t)i;
 }
 
+// Layout checks.  out->bad: min over bad boxes of (index << 2 | reason: 1
+// coordinate, 2 empty or inverted), the first reason met axis by axis; extents
+// as order-preserving keys, the shortest and longest edge as the bits of
+// positive doubles.
+__global__ void __launch_bounds__(256) k3_check_boxes(const float *__restrict__ boxes, int64_t n,
+                                                      BoxCheck *__restrict__ out) {
+    unsigned lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0u, 0u, 0u};
+    unsigned long long bad = ~0ull, emin = ~0ull, emax = 0ull;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float *b = boxes + 6 * i;
+        int why = 0;
+        for (int c = 0; c < 3 && !why; c++) {
+            const float x0 = __ldg(b + c), x1 = __ldg(b + 3 + c);
+            if (!(isfinite(x0) && fabsf(x0) < 16777216.0f && isfinite(x1) && fabsf(x1) < 16777216.0f)) why = 1;
+            else if (!(x0 < x1)) why = 2;
+            if (why) break;
+            lo[c] = min(lo[c], f_key(x0));
+            hi[c] = max(hi[c], f_key(x1));
+            const unsigned long long e = (unsigned long long)__double_as_longlong((double)x1 - (double)x0);
+            emin = min(emin, e);
+            emax = max(emax, e);
+        }
+        if (why) bad = min(bad, ((unsigned long long)i << 2) | (unsigned)why);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        for (int c = 0; c < 3; c++) {
+            lo[c] = min(lo[c], __shfl_xor_sync(kFull, lo[c], o));
+            hi[c] = max(hi[c], __shfl_xor_sync(kFull, hi[c], o));
+        }
+        bad = min(bad, __shfl_xor_sync(kFull, bad, o));
+        emin = min(emin, __shfl_xor_sync(kFull, emin, o));
+        emax = max(emax, __shfl_xor_sync(kFull, emax, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        for (int c = 0; c < 3; c++) {
+            atomicMin(&out->lo[c], lo[c]);
+            atomicMax(&out->hi[c], hi[c]);
+        }
+        atomicMin(&out->emin, emin);
+        atomicMax(&out->emax, emax);
+        if (bad != ~0ull) atomicMin(&out->bad, bad);
+    }
+}
+
+// Boxes of one bin compared pairwise, a thread per bin entry against the later
+// ones of its bin up to the first that overlaps it (interiors meet): *pair =
+// min over the pairs found of (lower index << 32 | higher).  Two overlapping
+// boxes share a bin.
+__global__ void __launch_bounds__(256) k3_overlaps(const float *__restrict__ boxes, const int64_t *__restrict__ bstart,
+                                                   int64_t nbins, const int32_t *__restrict__ items,
+                                                   unsigned long long *__restrict__ pair) {
+    const int64_t total = bstart[nbins];
+    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (int64_t)gridDim.x * blockDim.x) {
+        int64_t a = 0, b = nbins;  // the bin of entry u: bstart[a] <= u < bstart[a + 1]
+        while (b - a > 1) {
+            const int64_t m = (a + b) >> 1;
+            if (bstart[m] <= u) a = m;
+            else b = m;
+        }
+        const int64_t e = bstart[a + 1];
+        const int i = items[u];
+        float4 lo, hi;
+        load_box(boxes, i, lo, hi);
+        for (int64_t v = u + 1; v < e; v++) {
+            const int j = items[v];
+            float4 l2, h2;
+            load_box(boxes, j, l2, h2);
+            if (lo.x < h2.x && l2.x < hi.x && lo.y < h2.y && l2.y < hi.y && lo.z < h2.z && l2.z < hi.z) {
+                atomicMin(pair, ((unsigned long long)(unsigned)min(i, j) << 32) | (unsigned)max(i, j));
+                break;
+            }
+        }
+    }
+}
+
 // List entries (pairs of float4) ordered by (d_c in hi.w, box index in lo.w).
 __device__ __forceinline__ bool entry_less(const float4 *e, int64_t a, int64_t b) {
     const float ka = e[2 * a + 1].w, kb = e[2 * b + 1].w;
@@ -899,6 +975,58 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
 }
 
 }  // namespace
+
+frw_status check_boxes3(const float *d_boxes, int64_t n, int sms, cudaStream_t st, BoxCheck *d_out) {
+    // indices, minima: all ones; maxima: zero
+    FRW_CK(cudaMemsetAsync(d_out, 0xFF, sizeof(BoxCheck), st));
+    FRW_CK(cudaMemsetAsync(&d_out->emax, 0, 8, st));
+    FRW_CK(cudaMemsetAsync(d_out->hi, 0, sizeof(d_out->hi), st));
+    const int64_t blocks = std::min<int64_t>((n + 255) / 256, (int64_t)std::max(sms, 1) * 8);
+    k3_check_boxes<<<(unsigned)blocks, 256, 0, st>>>(d_boxes, n, d_out);
+    FRW_CK(cudaGetLastError());
+    return FRW_OK;
+}
+
+// Bins about one box across over the boxes' own extent (a box meets at most
+// two per axis), however wide the bounds are.
+frw_status check_disjoint3(const float *d_boxes, int64_t n, const double lo[3], const double hi[3], double emax,
+                           cudaStream_t st, BoxCheck *d_out) {
+    double vol = 1.0;
+    for (int c = 0; c < 3; c++) vol *= std::max(hi[c] - lo[c], 1e-30);
+    double cs = std::max(emax, std::cbrt(vol / (double)n));
+    int64_t nc[3], total;
+    for (;;) {
+        total = 1;
+        for (int c = 0; c < 3; c++) {
+            nc[c] = std::max<int64_t>(1, (int64_t)std::floor((hi[c] - lo[c]) / cs) + 1);
+            total *= nc[c];
+        }
+        if (total <= 8 * n + 64) break;
+        cs *= 1.25;
+    }
+    Grid3 G{};
+    for (int c = 0; c < 3; c++) {
+        G.o[c] = lo[c];
+        G.n[c] = (int)nc[c];
+    }
+    G.inv = 1.0 / cs;
+    const size_t cb = (size_t)(total + 1) * 8;
+    const int64_t tiles = scan_i64_tiles(total + 1), most = 27 * n;  // entries: two bins per axis, three by rounding
+    char *p = nullptr;
+    FRW_CK(cudaMallocAsync(&p, 2 * cb + (size_t)tiles * 8 + 8 + (size_t)most * 4, st));
+    int64_t *cnt = (int64_t *)p, *start = cnt + total + 1, *sums = start + total + 1, *grand = sums + tiles;
+    int32_t *items = (int32_t *)(grand + 1);
+    cudaError_t e = cudaMemsetAsync(cnt, 0, cb, st);
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    k3_bin_count<<<nb, 256, 0, st>>>(d_boxes, n, G, (unsigned long long *)cnt);
+    launch_scan_i64(cnt, total + 1, start, sums, grand, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, start, cb, cudaMemcpyDeviceToDevice, st);
+    k3_bin_fill<<<nb, 256, 0, st>>>(d_boxes, n, G, (unsigned long long *)cnt, items);
+    k3_overlaps<<<(unsigned)((3 * n + 255) / 256), 256, 0, st>>>(d_boxes, start, total, items, &d_out->pair);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    cudaFreeAsync(p, st);
+    return e == cudaSuccess ? FRW_OK : cuda_fail(e, "3-D layout check");
+}
 
 frw_status build_grid3(const float *d_boxes, int64_t n, const double bounds[6], double cells_per_box,
                        cudaStream_t st, Grid3Buffers *out) {
