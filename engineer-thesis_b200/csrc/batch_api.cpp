@@ -241,7 +241,7 @@ frw_status frw_batch_create(const frw_layout *const *layouts, const int64_t *tar
     B->tuning.struct_size = sizeof(frw_tuning);
     B->tuning.blocks_per_sm = o.blocks_per_sm;
     B->tuning.refill_min = o.refill_min > 0 ? o.refill_min : 1;
-    B->tuning.chunk = 128;
+    B->tuning.chunk = B->total <= (uint64_t)grid_for(B, B->tuning, B->total) * 256 ? 32 : 128;  // as launch_walk chooses
     rc = build_graph(B);
     if (rc) {
         free_batch(B);

@@ -168,6 +168,85 @@ frw_status prepare_walk(const frw3_layout *L, int64_t target, uint64_t first, ui
     return FRW_OK;
 }
 
+// Device scratch of walks from T targets: the rows of T x n boxes and a header
+// of words (counter, row count, grid status, pad, stats[4 T]), cleared in one
+// memset; the nonzero rows as entries behind the header; `extra` bytes.
+struct WalkScratch3 {
+    Scratch3 mem{nullptr};
+    cudaStream_t st = nullptr;
+    size_t nrow = 0, words = 0;
+    int64_t room = 0;
+    unsigned long long *hits = nullptr, *hdr = nullptr;
+    char *extra = nullptr;
+    void fill(Walk3Params &P) const {
+        P.counter = hdr;
+        P.stats = hdr + 4;
+        P.hits = hits;
+        P.sum_w = (double *)(hits + nrow);
+        P.sum_w2 = P.sum_w + nrow;
+    }
+    // The walks' stats (4 per target) and nonzero rows; the layout's status
+    // word (set only if a lookup ever found no list on the whole chain of grid
+    // levels, which the build rules out) is checked.
+    frw_status read(const uint32_t *status, const char *what, std::vector<unsigned long long> *stats,
+                    std::vector<RowEntry> *rows) const {
+        const double *sw = (const double *)(hits + nrow);
+        frw_status rc = launch_compact_entries(hits, sw, sw + nrow, (int64_t)nrow, (RowEntry *)(hdr + words), hdr + 1,
+                                               status, (uint32_t *)(hdr + 2), st);
+        if (rc) return rc;
+        std::vector<unsigned long long> h(words);
+        if ((rc = read_rows(hdr, words * 8, 8, room, st, what, h.data(), rows))) return rc;
+        if (h[2]) {
+            set_error("3-D grid: a lookup found no candidate list on any level");
+            return FRW_E_KERNEL;
+        }
+        stats->assign(h.begin() + 4, h.end());
+        return FRW_OK;
+    }
+};
+
+frw_status walk_scratch3(int64_t T, int64_t n, uint64_t walks, size_t extra, cudaStream_t st, WalkScratch3 *W) {
+    W->st = W->mem.st = st;
+    W->nrow = (size_t)(T * n);
+    W->words = 4 + 4 * (size_t)T;
+    W->room = (int64_t)std::min<uint64_t>(W->nrow, std::max<uint64_t>(walks, 1));
+    const size_t clear = (3 * W->nrow + W->words) * 8, rows = (size_t)W->room * sizeof(RowEntry);
+    FRW_CK(cudaMallocAsync(&W->mem.p, clear + rows + extra, st));
+    FRW_CK(cudaMemsetAsync(W->mem.p, 0, clear, st));
+    W->hits = (unsigned long long *)W->mem.p;
+    W->hdr = W->hits + 3 * W->nrow;
+    W->extra = (char *)W->mem.p + clear + rows;
+    return FRW_OK;
+}
+
+// A result from its target's sorted entries (rows from row0 on).
+void fill_result3(uint64_t walks, const unsigned long long *stats, const double *G, double shell, float ms,
+                  int64_t target, const RowEntry *e, const RowEntry *end, int64_t row0, frw3_result *res) {
+    res->walks = walks;
+    res->escaped = stats[0];
+    res->aborted = stats[1];
+    res->hops_total = stats[2];
+    memcpy(res->gauss, G, sizeof(res->gauss));
+    res->shell = shell;
+    res->kernel_ms = ms;
+    uint64_t on_target = 0;
+    const double N = (double)walks;
+    res->n_entries = end - e;
+    for (int64_t k = 0; e < end; e++, k++) {
+        if (e->row - row0 == target) on_target = e->n;
+        if (k >= res->capacity) continue;
+        const double m = e->s / N;
+        const double var = std::max(e->s2 / N - m * m, 0.0);
+        if (res->conductor) res->conductor[k] = e->row - row0;
+        if (res->hits) res->hits[k] = e->n;
+        if (res->cap) res->cap[k] = m;
+        if (res->cap_se) res->cap_se[k] = walks > 1 ? sqrt(var / (N - 1)) : 0.0;
+        if (res->sum_w) res->sum_w[k] = e->s;
+        if (res->sum_w2) res->sum_w2[k] = e->s2;
+    }
+    res->fraction_other = walks ? (double)(walks - on_target) / N : 0.0;
+}
+
 int sm_count(int dev) {
     const double *t2;
     int sms = 148;
@@ -422,17 +501,9 @@ frw_status frw3_walk(const frw3_layout *L, int64_t target, uint64_t walks, uint6
     Dev3Guard g(L->device);
     cudaStream_t st = (cudaStream_t)stream;
     const int64_t n = L->n;
-    // scratch: counter | stats[4] | hits[n] | sum_w[n] | sum_w2[n]
-    const size_t bytes = (size_t)(5 + 3 * n) * 8;
-    Scratch3 s(st);
-    FRW_CK(cudaMallocAsync(&s.p, bytes, st));
-    FRW_CK(cudaMemsetAsync(s.p, 0, bytes, st));
-    unsigned long long *u = (unsigned long long *)s.p;
-    P.counter = u;
-    P.stats = u + 1;
-    P.hits = u + 5;
-    P.sum_w = (double *)(u + 5 + n);
-    P.sum_w2 = (double *)(u + 5 + 2 * n);
+    WalkScratch3 W;
+    if ((rc = walk_scratch3(1, n, walks, 0, st, &W))) return rc;
+    W.fill(P);
     Events ev(2);
     if (!ev.ok(2)) return cuda_fail(cudaErrorUnknown, "event create");
     FRW_CK(cudaEventRecord(ev[0], st));
@@ -441,43 +512,16 @@ frw_status frw3_walk(const frw3_layout *L, int64_t target, uint64_t walks, uint6
         if (rc) return rc;
     }
     FRW_CK(cudaEventRecord(ev[1], st));
-    std::vector<unsigned long long> h(5 + 3 * (size_t)n);
-    rc = read_back(h.data(), s.p, bytes, st, "frw3_walk");
-    if (rc) return rc;
+    std::vector<unsigned long long> stats;
+    std::vector<RowEntry> rows;
+    if ((rc = W.read(L->grid.status, "frw3_walk", &stats, &rows))) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, ev[0], ev[1]);
-    const unsigned long long *stats = h.data() + 1, *hits = h.data() + 5;
-    const double *sw = (const double *)(h.data() + 5 + n), *sw2 = (const double *)(h.data() + 5 + 2 * n);
     if (stats[3] != walks) {
         set_error("3-D walk kernel finished " + std::to_string(stats[3]) + " of " + std::to_string(walks) + " walks");
         return FRW_E_KERNEL;
     }
-    rc = check_grid_status(L, st);
-    if (rc) return rc;
-    res->walks = walks;
-    res->escaped = stats[0];
-    res->aborted = stats[1];
-    res->hops_total = stats[2];
-    memcpy(res->gauss, P.G, sizeof(res->gauss));
-    res->shell = shell;
-    res->kernel_ms = ms;
-    res->fraction_other = walks ? (double)(walks - hits[target]) / (double)walks : 0.0;
-    int64_t k = 0;
-    for (int64_t i = 0; i < n; i++) {
-        if (!hits[i]) continue;
-        if (k < res->capacity) {
-            const double N = (double)walks, m = sw[i] / N;
-            const double var = std::max(sw2[i] / N - m * m, 0.0);
-            if (res->conductor) res->conductor[k] = i;
-            if (res->hits) res->hits[k] = hits[i];
-            if (res->cap) res->cap[k] = m;
-            if (res->cap_se) res->cap_se[k] = walks > 1 ? sqrt(var / (N - 1)) : 0.0;
-            if (res->sum_w) res->sum_w[k] = sw[i];
-            if (res->sum_w2) res->sum_w2[k] = sw2[i];
-        }
-        k++;
-    }
-    res->n_entries = k;
+    fill_result3(walks, stats.data(), P.G, shell, ms, target, rows.data(), rows.data() + rows.size(), 0, res);
     return FRW_OK;
 }
 
@@ -553,22 +597,12 @@ frw_status frw3_walk_batch(const frw3_layout *L, const int64_t *targets, int32_t
     Dev3Guard g(L->device);
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t total = (uint64_t)ntargets * walks_per_target;
-    // scratch: counter | stats[4 T] | hits[T n] | sum_w[T n] | sum_w2[T n] | jobs
-    const size_t nrow = (size_t)ntargets * (size_t)n;
-    const size_t words = 1 + 4 * (size_t)ntargets + 3 * nrow;
-    const size_t bytes = words * 8 + jobs.size() * sizeof(Job3);
-    Scratch3 s(st);
-    FRW_CK(cudaMallocAsync(&s.p, bytes, st));
-    FRW_CK(cudaMemsetAsync(s.p, 0, words * 8, st));
-    unsigned long long *u = (unsigned long long *)s.p;
-    Job3 *d_jobs = (Job3 *)(u + words);
-    FRW_CK(cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(Job3), cudaMemcpyHostToDevice, st));
-    P.counter = u;
-    P.stats = u + 1;
-    P.hits = u + 1 + 4 * ntargets;
-    P.sum_w = (double *)(P.hits + nrow);
-    P.sum_w2 = P.sum_w + nrow;
-    P.jobs = d_jobs;
+    WalkScratch3 W;
+    const size_t job_bytes = jobs.size() * sizeof(Job3);
+    if ((rc = walk_scratch3(ntargets, n, total, job_bytes, st, &W))) return rc;
+    W.fill(P);
+    FRW_CK(cudaMemcpyAsync(W.extra, jobs.data(), job_bytes, cudaMemcpyHostToDevice, st));
+    P.jobs = (const Job3 *)W.extra;
     P.walks_per_job = walks_per_target;
     P.nboxes = n;
     P.walks = total;
@@ -580,51 +614,22 @@ frw_status frw3_walk_batch(const frw3_layout *L, const int64_t *targets, int32_t
         if (rc) return rc;
     }
     FRW_CK(cudaEventRecord(ev[1], st));
-    std::vector<unsigned long long> h(words);
-    rc = read_back(h.data(), s.p, words * 8, st, "frw3_walk_batch");
-    if (rc) return rc;
-    rc = check_grid_status(L, st);
-    if (rc) return rc;
+    std::vector<unsigned long long> stats;
+    std::vector<RowEntry> rows;
+    if ((rc = W.read(L->grid.status, "frw3_walk_batch", &stats, &rows))) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, ev[0], ev[1]);
-    const unsigned long long *hits_all = h.data() + 1 + 4 * ntargets;
-    const double *sw_all = (const double *)(hits_all + nrow), *sw2_all = sw_all + nrow;
+    const RowEntry *e = rows.data(), *end = e + rows.size();
     for (int32_t t = 0; t < ntargets; t++) {
-        const unsigned long long *stt = h.data() + 1 + 4 * t;
+        const unsigned long long *stt = stats.data() + 4 * (size_t)t;
         if (stt[3] != walks_per_target) {
             set_error("3-D batch: target " + std::to_string(t) + " finished " + std::to_string(stt[3]) + " of " +
                       std::to_string(walks_per_target) + " walks");
             return FRW_E_KERNEL;
         }
-        frw3_result *res = results + t;
-        const unsigned long long *hits = hits_all + (size_t)t * n;
-        const double *sw = sw_all + (size_t)t * n, *sw2 = sw2_all + (size_t)t * n;
-        const int64_t tk = targets[t];
-        res->walks = walks_per_target;
-        res->escaped = stt[0];
-        res->aborted = stt[1];
-        res->hops_total = stt[2];
-        memcpy(res->gauss, jobs[t].G, sizeof(res->gauss));
-        res->shell = shell;
-        res->kernel_ms = ms;
-        res->fraction_other =
-            walks_per_target ? (double)(walks_per_target - hits[tk]) / (double)walks_per_target : 0.0;
-        int64_t k = 0;
-        for (int64_t i = 0; i < n; i++) {
-            if (!hits[i]) continue;
-            if (k < res->capacity) {
-                const double N = (double)walks_per_target, m = sw[i] / N;
-                const double var = std::max(sw2[i] / N - m * m, 0.0);
-                if (res->conductor) res->conductor[k] = i;
-                if (res->hits) res->hits[k] = hits[i];
-                if (res->cap) res->cap[k] = m;
-                if (res->cap_se) res->cap_se[k] = walks_per_target > 1 ? sqrt(var / (N - 1)) : 0.0;
-                if (res->sum_w) res->sum_w[k] = sw[i];
-                if (res->sum_w2) res->sum_w2[k] = sw2[i];
-            }
-            k++;
-        }
-        res->n_entries = k;
+        const RowEntry *first = e;
+        while (e < end && e->row < (int64_t)(t + 1) * n) e++;
+        fill_result3(walks_per_target, stt, jobs[t].G, shell, ms, targets[t], first, e, (int64_t)t * n, results + t);
     }
     return FRW_OK;
 }

@@ -278,9 +278,7 @@ struct WalkRun {
     uint64_t escaped = 0, aborted = 0, hops = 0, done = 0;
     double gauss[4] = {0, 0, 0, 0};
     float kernel_ms = 0.f;
-    std::vector<int64_t> row;
-    std::vector<unsigned long long> n;
-    std::vector<double> s, s2;
+    std::vector<RowEntry> rows;  // sorted by row
 };
 
 // One job on one layout; records optional; host results optional.
@@ -295,34 +293,30 @@ frw_status run_walks(const frw_layout *lay, int64_t target, uint64_t first_walk,
         set_error("target conductor index out of range");
         return FRW_E_ARG;
     }
-    // one scratch block: a header cleared with the per-conductor rows in one
-    // memset, read back in one copy; compacted rows after it
+    // one scratch block: per-conductor rows and a header, cleared in one
+    // memset, then the nonzero rows as entries, read back with the header
     struct Hdr {
         double4 gauss;
         unsigned long long stats[4], counter, cnt;
-        uint32_t status, pad;
-        double4 tgt;
+        uint32_t status, pad[3];
     };
-    static_assert(sizeof(Hdr) % 16 == 0, "header keeps 16-byte alignment");
+    static_assert(sizeof(Hdr) % 32 == 0, "header keeps the entries' alignment");
     const int64_t rows = lay->n;  // the kernel flushes every conductor it reaches
-    const size_t R = (size_t)std::max<int64_t>(rows, 1);
+    const size_t R = ((size_t)std::max<int64_t>(rows, 1) + 3) & ~(size_t)3;
+    const int64_t room = out ? (int64_t)std::min<uint64_t>((uint64_t)std::max<int64_t>(rows, 1), std::max<uint64_t>(walks, 1)) : 0;
     Scratch S(st);
     char *blk;
-    FRW_CK(S.get(&blk, sizeof(Hdr) + R * 8 * (out ? 7 : 3)));
-    Hdr *h = reinterpret_cast<Hdr *>(blk);
-    unsigned long long *d_acc_n = reinterpret_cast<unsigned long long *>(blk + sizeof(Hdr));
+    FRW_CK(S.get(&blk, R * 24 + sizeof(Hdr) + (size_t)room * sizeof(RowEntry)));
+    unsigned long long *d_acc_n = reinterpret_cast<unsigned long long *>(blk);
     double *d_acc_s = reinterpret_cast<double *>(d_acc_n + R);
     double *d_acc_s2 = d_acc_s + R;
-    double4 *d_tgt = &h->tgt, *d_gauss = &h->gauss;
+    Hdr *h = reinterpret_cast<Hdr *>(d_acc_s2 + R);
+    double4 *d_gauss = &h->gauss;
     uint32_t *d_status = &h->status;
     unsigned long long *d_counter = &h->counter, *d_stats = h->stats;
-    const double *r = lay->rects.get() + 4 * target;
-    const double tg[4] = {r[0], r[1], r[2], r[3]};
-    FRW_CK(cudaMemsetAsync(blk, 0, offsetof(Hdr, tgt), st));
-    if (rows) FRW_CK(cudaMemsetAsync(d_acc_n, 0, R * 24, st));
-    FRW_CK(cudaMemcpyAsync(d_tgt, tg, sizeof(tg), cudaMemcpyHostToDevice, st));
-    rc = launch_gauss(lay->dl, (const double *)d_tgt, 1, o.gauss_mode, o.gauss_param, (double *)d_gauss,
-                      d_status, st);
+    FRW_CK(cudaMemsetAsync(blk, 0, R * 24 + sizeof(Hdr), st));
+    rc = launch_gauss_of(lay->dl, lay->rects.get() + 4 * target, o.gauss_mode, o.gauss_param, (double *)d_gauss,
+                         d_status, st);
     if (rc) return rc;
 
     WalkParams P{};
@@ -385,31 +379,15 @@ frw_status run_walks(const frw_layout *lay, int64_t target, uint64_t first_walk,
         return check_status(d_status, st);
     }
     FRW_CK(cudaEventRecord(e1, st));
-    // compact nonzero rows (after the accumulators in the same block)
-    int64_t *d_row = reinterpret_cast<int64_t *>(d_acc_s2 + R);
-    unsigned long long *d_cn = reinterpret_cast<unsigned long long *>(d_row + R);
-    double *d_cs = reinterpret_cast<double *>(d_cn + R);
-    double *d_cs2 = d_cs + R;
-    rc = launch_compact(d_acc_n, d_acc_s, d_acc_s2, rows, d_row, d_cn, d_cs, d_cs2, &h->cnt, st);
+    rc = launch_compact_entries(d_acc_n, d_acc_s, d_acc_s2, rows, reinterpret_cast<RowEntry *>(h + 1), &h->cnt, nullptr,
+                                nullptr, st);
     if (rc) return rc;
     Hdr hh;
-    rc = read_back(&hh, h, offsetof(Hdr, tgt), st, "walk results");
+    rc = read_rows(h, sizeof(Hdr), offsetof(Hdr, cnt), room, st, "walk results", &hh, &out->rows);
     if (rc) return rc;
     rc = status_error(hh.status);
     if (rc) return rc;
-    const unsigned long long h_cnt = hh.cnt;
     memcpy(out->gauss, &hh.gauss, sizeof(out->gauss));
-    out->row.resize(h_cnt);
-    out->n.resize(h_cnt);
-    out->s.resize(h_cnt);
-    out->s2.resize(h_cnt);
-    if (h_cnt) {
-        FRW_CK(cudaMemcpyAsync(out->row.data(), d_row, h_cnt * 8, cudaMemcpyDeviceToHost, st));
-        FRW_CK(cudaMemcpyAsync(out->n.data(), d_cn, h_cnt * 8, cudaMemcpyDeviceToHost, st));
-        FRW_CK(cudaMemcpyAsync(out->s.data(), d_cs, h_cnt * 8, cudaMemcpyDeviceToHost, st));
-        FRW_CK(cudaMemcpyAsync(out->s2.data(), d_cs2, h_cnt * 8, cudaMemcpyDeviceToHost, st));
-        FRW_CK(cudaStreamSynchronize(st));
-    }
     out->escaped = hh.stats[0];
     out->aborted = hh.stats[1];
     out->hops = hh.stats[2];
@@ -489,6 +467,34 @@ frw_status read_back(void *host, const void *dev, size_t bytes, cudaStream_t st,
     cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // only this copy is left on the stream
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, what);
+}
+
+frw_status read_rows(const void *dev, size_t hdr_bytes, size_t count_at, int64_t room, cudaStream_t st,
+                     const char *what, void *hdr, std::vector<RowEntry> *rows) {
+    // the header and as many entries as read_back stages in one piece
+    constexpr size_t kStage = 4096;
+    const size_t few = hdr_bytes < kStage ? (kStage - hdr_bytes) / sizeof(RowEntry) : 0;
+    const size_t head = (size_t)std::min<int64_t>((int64_t)few, room);
+    std::vector<char> buf(hdr_bytes + head * sizeof(RowEntry));
+    frw_status rc = read_back(buf.data(), dev, buf.size(), st, what);
+    if (rc) return rc;
+    memcpy(hdr, buf.data(), hdr_bytes);
+    unsigned long long cnt;
+    memcpy(&cnt, buf.data() + count_at, 8);
+    if (cnt > (unsigned long long)room) {
+        set_error(std::string(what) + ": more rows than room for them");
+        return FRW_E_KERNEL;
+    }
+    rows->resize(cnt);
+    const size_t got = std::min<size_t>(head, cnt);
+    if (got) memcpy(rows->data(), buf.data() + hdr_bytes, got * sizeof(RowEntry));
+    if (cnt > got) {
+        const char *rest = static_cast<const char *>(dev) + hdr_bytes + got * sizeof(RowEntry);
+        FRW_CK(cudaMemcpyAsync(rows->data() + got, rest, (cnt - got) * sizeof(RowEntry), cudaMemcpyDeviceToHost, st));
+        FRW_CK(cudaStreamSynchronize(st));
+    }
+    std::sort(rows->begin(), rows->end(), [](const RowEntry &a, const RowEntry &b) { return a.row < b.row; });
+    return FRW_OK;
 }
 
 // The FP64 host copy of a layout's rects (layer order), converted by host
@@ -991,24 +997,21 @@ frw_status frw_walk(const frw_layout *L, int64_t target, uint64_t walks, uint64_
     res->hops_total = R.hops;
     memcpy(res->gauss, R.gauss, sizeof(res->gauss));
     res->kernel_ms = R.kernel_ms;
-    std::vector<size_t> ord(R.row.size());
-    for (size_t i = 0; i < ord.size(); i++) ord[i] = i;
-    std::sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return R.row[a] < R.row[b]; });
     uint64_t on_target = 0;
-    res->n_entries = (int64_t)ord.size();
+    res->n_entries = (int64_t)R.rows.size();
     const double N = (double)walks;
-    for (size_t k = 0; k < ord.size(); k++) {
-        const size_t i = ord[k];
-        if (R.row[i] == target) on_target = R.n[i];
+    for (size_t k = 0; k < R.rows.size(); k++) {
+        const RowEntry &e = R.rows[k];
+        if (e.row == target) on_target = e.n;
         if ((int64_t)k >= res->capacity) continue;
-        const double mean = R.s[i] / N;
-        const double var = walks > 1 ? std::max(R.s2[i] / N - mean * mean, 0.0) * N / (N - 1.0) : 0.0;
-        if (res->conductor) res->conductor[k] = R.row[i];
-        if (res->hits) res->hits[k] = R.n[i];
+        const double mean = e.s / N;
+        const double var = walks > 1 ? std::max(e.s2 / N - mean * mean, 0.0) * N / (N - 1.0) : 0.0;
+        if (res->conductor) res->conductor[k] = e.row;
+        if (res->hits) res->hits[k] = e.n;
         if (res->cap) res->cap[k] = mean;
         if (res->cap_se) res->cap_se[k] = sqrt(var / N);
-        if (res->sum_w) res->sum_w[k] = R.s[i];
-        if (res->sum_w2) res->sum_w2[k] = R.s2[i];
+        if (res->sum_w) res->sum_w[k] = e.s;
+        if (res->sum_w2) res->sum_w2[k] = e.s2;
     }
     res->fraction_other = walks ? (double)(walks - on_target) / N : 0.0;
     return FRW_OK;
@@ -1048,15 +1051,11 @@ frw_status frw::walk_device_rows(const frw_layout *L, int64_t target, uint64_t w
     if (rc) return rc;
     Scratch S(st);
     char *blk;
-    FRW_CK(S.get(&blk, 64 + 32));  // counter, then the target rect (32 B) and its Gaussian surface
+    FRW_CK(S.get(&blk, 64));  // counter, then the Gaussian surface
     unsigned long long *d_counter = reinterpret_cast<unsigned long long *>(blk);
-    double4 *d_tgt = reinterpret_cast<double4 *>(blk + 32);
-    double4 *d_gauss = reinterpret_cast<double4 *>(blk + 64);
-    const double *r = L->rects.get() + 4 * target;
-    const double tg[4] = {r[0], r[1], r[2], r[3]};
+    double4 *d_gauss = reinterpret_cast<double4 *>(blk + 32);
     FRW_CK(cudaMemsetAsync(d_counter, 0, 8, st));
-    FRW_CK(cudaMemcpyAsync(d_tgt, tg, sizeof(tg), cudaMemcpyHostToDevice, st));
-    rc = launch_gauss(L->dl, (const double *)d_tgt, 1, o.gauss_mode, o.gauss_param, (double *)d_gauss, status, st);
+    rc = launch_gauss_of(L->dl, L->rects.get() + 4 * target, o.gauss_mode, o.gauss_param, (double *)d_gauss, status, st);
     if (rc || walks == 0) return rc;
     WalkParams P{};
     P.job0.L = L->dl;

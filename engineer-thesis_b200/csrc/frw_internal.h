@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/frw.h"
 
@@ -272,6 +273,9 @@ frw_status launch_box_collides(const DevLayout &L, const double *d_boxes, int64_
                                cudaStream_t stream);
 frw_status launch_gauss(const DevLayout &L, const double *d_targets /*[n][4]*/, int n, int mode,
                         double param, double *d_out, uint32_t *d_status, cudaStream_t stream);
+// one target given by value
+frw_status launch_gauss_of(const DevLayout &L, const double target[4], int mode, double param, double *d_out,
+                           uint32_t *d_status, cudaStream_t stream);
 // one Gaussian surface per job, each on its job's layout
 frw_status launch_gauss_jobs(const WalkJob *d_jobs, const double *d_targets, int njobs, int mode, double param,
                              double *d_out, uint32_t *d_status, cudaStream_t stream);
@@ -285,6 +289,24 @@ int walk_max_blocks_per_sm(int threads, bool multi, bool uniform);
 frw_status launch_compact(const unsigned long long *acc_n, const double *acc_s, const double *acc_s2,
                           int64_t rows, int64_t *out_row, unsigned long long *out_n, double *out_s,
                           double *out_s2, unsigned long long *d_count, cudaStream_t stream, int64_t cap = -1);
+
+// A nonzero accumulator row.
+struct RowEntry {
+    int64_t row;
+    unsigned long long n;
+    double s, s2;
+};
+// The same as entries of 32 bytes (room for every nonzero row); the kernel
+// limit word *src, when given, is copied to *dst.
+frw_status launch_compact_entries(const unsigned long long *acc_n, const double *acc_s, const double *acc_s2,
+                                  int64_t rows, RowEntry *out, unsigned long long *d_count, const uint32_t *src,
+                                  uint32_t *dst, cudaStream_t stream);
+// A result header of hdr_bytes at dev with its `room` row entries right behind
+// it, after everything enqueued on `st`: one copy for the header and the
+// entries of a small result, a second one for the rest of a large one.  The
+// count (u64) lies at hdr + count_at.  Entries come sorted by row.
+frw_status read_rows(const void *dev, size_t hdr_bytes, size_t count_at, int64_t room, cudaStream_t st,
+                     const char *what, void *hdr, std::vector<RowEntry> *rows);
 
 // host_green.cpp
 void green_tables(double *g, double *intg, double *wx, double *wy);

@@ -115,6 +115,15 @@ __global__ void k_gauss(DevLayout L, const double4 *__restrict__ targets, int n,
     if (st) atomicOr(status, st);
 }
 
+__global__ void k_gauss_of(DevLayout L, double4 target, int mode, double param, double4 *__restrict__ out,
+                           uint32_t *status) {
+    double o[4];
+    uint32_t st = 0;
+    gauss_one(L, target, mode, param, o, st);
+    *out = make_double4(o[0], o[1], o[2], o[3]);
+    if (st) atomicOr(status, st);
+}
+
 // One job per thread, each on its own layout (batched runs).
 __global__ void k_gauss_jobs(const WalkJob *__restrict__ jobs, const double4 *__restrict__ targets, int n, int mode,
                              double param, double4 *__restrict__ out, uint32_t *status) {
@@ -160,6 +169,13 @@ frw_status launch_box_collides(const DevLayout &L, const double *d_boxes, int64_
                             : make_double4(0, 0, 0, 0);
     k_box<<<(unsigned)((n + T - 1) / T), T, 0, stream>>>(L, (const double4 *)d_boxes, n, has_ignore, ig,
                                                          d_out, d_status);
+    FRW_CK(cudaGetLastError());
+    return FRW_OK;
+}
+
+frw_status launch_gauss_of(const DevLayout &L, const double t[4], int mode, double param, double *d_out,
+                           uint32_t *d_status, cudaStream_t stream) {
+    k_gauss_of<<<1, 1, 0, stream>>>(L, make_double4(t[0], t[1], t[2], t[3]), mode, param, (double4 *)d_out, d_status);
     FRW_CK(cudaGetLastError());
     return FRW_OK;
 }
