@@ -471,9 +471,9 @@ frw_status build_records(const DevLayout &L, const CoarseLists &K, const Grid &G
     if ((rc = B.get(&C.cellids, (size_t)ncells * sizeof(int4), "malloc cell ids"))) return rc;
     if ((rc = B.get(&C.crad, (size_t)ncells * sizeof(float), "malloc cell radii"))) return rc;
     if ((rc = B.get(&tot, 24, "malloc totals"))) return rc;
-    // one entry of list room per cell holds the lists of the benchmark's
-    // densities (0.3 at 16 cells per rect); denser ones take a second pass
-    int64_t room = std::max<int64_t>(ncells, 4096);
+    // half an entry of list room per cell holds the lists of the benchmark's
+    // densities (0.16 at 16 cells per rect); denser ones take a second pass
+    int64_t room = std::max<int64_t>(ncells / 2, 4096);
     unsigned long long h[3] = {0, 0, 0};
     float4 *rects = nullptr;
     int32_t *ids = nullptr;

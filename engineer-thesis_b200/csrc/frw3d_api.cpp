@@ -467,10 +467,7 @@ frw_status frw3_query_batch(const frw3_layout *L, const double *pts, int64_t n, 
     if (rc) return rc;
     rc = check_grid_status(L, st);  // bounded wait for the queries, then the grid status
     if (rc) return rc;
-    if (clear) FRW_CK(cudaMemcpyAsync(clear, dc, cb, cudaMemcpyDeviceToHost, st));
-    if (nearest) FRW_CK(cudaMemcpyAsync(nearest, dn, nbt, cudaMemcpyDeviceToHost, st));
-    FRW_CK(cudaStreamSynchronize(st));
-    return FRW_OK;
+    return copy_out({{clear, dc, cb}, {nearest, dn, nbt}}, L->device, st, "frw3_query_batch");
 }
 
 void frw3_opts_default(frw3_opts *o) {
@@ -677,10 +674,9 @@ frw_status frw3_walk_trace(const frw3_layout *L, int64_t target, uint64_t first_
     rc = wait_stream(st, "frw3_walk_trace");
     if (rc) return rc;
     if (mem == FRW_MEM_HOST) {
-        if (end) FRW_CK(cudaMemcpyAsync(end, P.rec_end, W * 8, cudaMemcpyDeviceToHost, st));
-        if (weight) FRW_CK(cudaMemcpyAsync(weight, P.rec_w, W * 8, cudaMemcpyDeviceToHost, st));
-        if (hops) FRW_CK(cudaMemcpyAsync(hops, P.rec_hops, W * 4, cudaMemcpyDeviceToHost, st));
-        if (bin1) FRW_CK(cudaMemcpyAsync(bin1, P.rec_bin, W * 4, cudaMemcpyDeviceToHost, st));
+        rc = copy_out({{end, P.rec_end, W * 8}, {weight, P.rec_w, W * 8}, {hops, P.rec_hops, W * 4}, {bin1, P.rec_bin, W * 4}},
+                      L->device, st, "frw3_walk_trace");
+        if (rc) return rc;
     }
     unsigned long long done = 0;
     FRW_CK(cudaMemcpyAsync(&done, P.stats + 3, 8, cudaMemcpyDeviceToHost, st));

@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -170,6 +171,16 @@ frw_status wait_event(cudaEvent_t e, const char *what);
 // wait, then a synchronous copy (no allocation).
 frw_status read_back(void *host, const void *dev, size_t bytes, cudaStream_t st, const char *what,
                      bool staged = true);
+
+// Result arrays into pageable host memory, after the work before them on `st`
+// has been waited for: large ones in chunks through pinned buffers of the
+// calling thread, moved on by a few host threads.
+struct HostOut {
+    void *host;
+    const void *dev;
+    size_t bytes;
+};
+frw_status copy_out(std::initializer_list<HostOut> arrays, int device, cudaStream_t st, const char *what);
 
 // CUDA events destroyed at scope exit, error paths included.
 struct Events {

@@ -24,6 +24,7 @@ Names follow the reference (piogrzej/engineer-thesis, randomWalk/):
 from __future__ import annotations
 
 import ctypes as C
+import mmap
 import os
 from dataclasses import dataclass, field
 
@@ -323,6 +324,18 @@ def _ptr(a, t=_VP):
     return None if a is None else C.cast(a.ctypes.data, t)
 
 
+def _row_arrays(cap: int):
+    """conductor, hits, cap, cap_se, sum_w and sum_w2 of a result, `cap` zeros
+    each.  Large ones are demand-zero pages: a result fills the front of rows
+    that are as long as its layout, and clearing 48 MB for the few hundred
+    conductors of a 10^6-rect run takes longer than its walks."""
+    types = (np.int64, np.uint64, np.float64, np.float64, np.float64, np.float64)
+    if cap < 1 << 15:
+        return [np.zeros(cap, t) for t in types]
+    pages = mmap.mmap(-1, 48 * cap)
+    return [np.frombuffer(pages, t, cap, 8 * cap * k) for k, t in enumerate(types)]
+
+
 def version() -> str:
     return lib().frw_version().decode()
 
@@ -518,8 +531,8 @@ class Layout:
     def query(self, pts):
         """drawBiggestSquareAtPoint + checkCollisons(point) for (n,2) points."""
         p = np.ascontiguousarray(pts, dtype=np.float64).reshape(-1, 2)
-        sq = np.zeros((len(p), 4))
-        hit = np.zeros(len(p), dtype=np.int64)
+        sq = np.empty((len(p), 4))
+        hit = np.empty(len(p), dtype=np.int64)
         _check(lib().frw_query_batch(self._h, _ptr(p), len(p), _ptr(sq), _ptr(hit), MEM_HOST, None))
         return sq, hit
 
@@ -551,12 +564,7 @@ class Layout:
     def walk(self, target: int, walks: int, seed: int, o: Opts | None = None, capacity: int | None = None,
              stream: int = 0) -> WalkResult:
         cap = self.n if capacity is None else capacity
-        cond = np.zeros(cap, dtype=np.int64)
-        hits = np.zeros(cap, dtype=np.uint64)
-        c = np.zeros(cap)
-        se = np.zeros(cap)
-        s1 = np.zeros(cap)
-        s2 = np.zeros(cap)
+        cond, hits, c, se, s1, s2 = _row_arrays(cap)
         r = Result()
         r.capacity = cap
         r.conductor = _ptr(cond, _I64)
@@ -597,10 +605,10 @@ class Layout:
         return out
 
     def walk_trace(self, target: int, first: int, walks: int, seed: int, o: Opts | None = None):
-        end = np.zeros(walks, dtype=np.int64)
-        hops = np.zeros(walks, dtype=np.int32)
-        b1 = np.zeros(walks, dtype=np.int32)
-        w = np.zeros(walks)
+        end = np.empty(walks, dtype=np.int64)
+        hops = np.empty(walks, dtype=np.int32)
+        b1 = np.empty(walks, dtype=np.int32)
+        w = np.empty(walks)
         _check(lib().frw_walk_trace(self._h, target, first, walks, seed, C.byref(o) if o else None, _ptr(end),
                                     _ptr(hops), _ptr(b1), _ptr(w), MEM_HOST, None))
         return end, hops, b1, w
@@ -641,12 +649,7 @@ class Batch:
         res = (Result * n)()
         keep = []
         for j in range(n):
-            cond = np.zeros(capacity, dtype=np.int64)
-            hits = np.zeros(capacity, dtype=np.uint64)
-            c = np.zeros(capacity)
-            se = np.zeros(capacity)
-            s1 = np.zeros(capacity)
-            s2 = np.zeros(capacity)
+            cond, hits, c, se, s1, s2 = _row_arrays(capacity)
             keep.append((cond, hits, c, se, s1, s2))
             r = res[j]
             r.capacity = capacity
@@ -878,8 +881,8 @@ class Layout3:
     def query(self, pts):
         """Clearance (L-infinity distance to the nearest box) and that box for (n,3) points."""
         p = np.ascontiguousarray(pts, dtype=np.float64).reshape(-1, 3)
-        d = np.zeros(len(p))
-        k = np.zeros(len(p), dtype=np.int64)
+        d = np.empty(len(p))
+        k = np.empty(len(p), dtype=np.int64)
         _check(lib().frw3_query_batch(self._h, _ptr(p), len(p), _ptr(d), _ptr(k), MEM_HOST, None))
         return d, k
 
@@ -892,12 +895,7 @@ class Layout3:
              stream: int = 0) -> WalkResult:
         o = o or opts3()
         cap = self.n if capacity is None else capacity
-        cond = np.zeros(cap, dtype=np.int64)
-        hits = np.zeros(cap, dtype=np.uint64)
-        c = np.zeros(cap)
-        se = np.zeros(cap)
-        s1 = np.zeros(cap)
-        s2 = np.zeros(cap)
+        cond, hits, c, se, s1, s2 = _row_arrays(cap)
         r = Result3()
         r.capacity = cap
         r.conductor = _ptr(cond, _I64)
@@ -917,8 +915,7 @@ class Layout3:
         t = np.ascontiguousarray(targets, dtype=np.int64)
         cap = self.n if capacity is None else capacity
         T = len(t)
-        arrs = [(np.zeros(cap, np.int64), np.zeros(cap, np.uint64), np.zeros(cap), np.zeros(cap), np.zeros(cap),
-                 np.zeros(cap)) for _ in range(T)]
+        arrs = [_row_arrays(cap) for _ in range(T)]
         rs = (Result3 * T)()
         for r, (cond, hits, c, se, s1, s2) in zip(rs, arrs):
             r.capacity = cap
@@ -949,10 +946,10 @@ class Layout3:
 
     def walk_trace(self, target: int, first: int, walks: int, seed: int, o: Opts3 | None = None):
         o = o or opts3()
-        end = np.zeros(walks, dtype=np.int64)
-        hops = np.zeros(walks, dtype=np.int32)
-        b1 = np.zeros(walks, dtype=np.int32)
-        w = np.zeros(walks)
+        end = np.empty(walks, dtype=np.int64)
+        hops = np.empty(walks, dtype=np.int32)
+        b1 = np.empty(walks, dtype=np.int32)
+        w = np.empty(walks)
         _check(lib().frw3_walk_trace(self._h, target, first, walks, seed, C.byref(o), _ptr(end), _ptr(hops),
                                      _ptr(b1), _ptr(w), MEM_HOST, None))
         return end, hops, b1, w
