@@ -8,10 +8,10 @@
 //      with warp match/ballot + popc instead of shared-memory atomics;
 //   3. a level-synchronous split of Morton ranges: each frontier range is cut
 //      at its next base-4 digit by binary search on the sorted keys (no data
-//      movement); child node ids come from a count -> scan -> emit pass, so
-//      the build is deterministic; single-quadrant ranges are re-split one
-//      level down without emitting a node (path compression); ranges whose
-//      keys are all equal are split by index;
+//      movement); child node ids come from a block scan and an atomic per
+//      block, the level sizes staying on the device; single-quadrant ranges
+//      are re-split one level down without emitting a node (path
+//      compression); ranges whose keys are all equal are split by index;
 //   4. a bottom-up refit of the child boxes, batch by batch in reverse
 //      allocation order (children are always allocated after their parent).
 // Output is the flat node array of frw_internal.h: 64-byte child-box records
@@ -74,30 +74,37 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint32_t *__restri
     hist[threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
 }
 
-// Exclusive scan of up to a few million u32/u64 values with one block.
-template <typename T>
-__global__ void __launch_bounds__(1024) k_scan_excl(T *data, int64_t n, T *total) {
-    __shared__ T part[1024];
-    int t = threadIdx.x;
-    int64_t per = (n + 1023) / 1024;
-    int64_t a = t * per, b = a + per < n ? a + per : n;
-    T s = 0;
-    for (int64_t i = a; i < b; i++) s += data[i];
-    part[t] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        T v = t >= off ? part[t - off] : 0;
+// Exclusive scan of each digit's counts over the tiles (a block per digit, its
+// row of `hist`), the digit's total to tot[digit]; the scatter adds the digits
+// below.  (One block over all 256 rows took 0.1 ms per pass at 10^6 rects.)
+constexpr int kDigitThreads = 512;
+__global__ void __launch_bounds__(kDigitThreads) k_rs_scan(uint32_t *__restrict__ hist, int nblk,
+                                                           uint32_t *__restrict__ tot) {
+    __shared__ uint32_t wt[kDigitThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t *row = hist + (size_t)blockIdx.x * nblk;
+    uint32_t carry = 0;
+    for (int b = 0; b < nblk; b += kDigitThreads) {
+        const int i = b + threadIdx.x;
+        const uint32_t v = i < nblk ? row[i] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wt[w] = x;
         __syncthreads();
-        part[t] += v;
+        uint32_t before = carry, all = 0;
+        for (int k = 0; k < kDigitThreads / 32; k++) {
+            if (k < w) before += wt[k];
+            all += wt[k];
+        }
+        if (i < nblk) row[i] = before + x - v;
+        carry += all;
         __syncthreads();
     }
-    T run = t ? part[t - 1] : 0;
-    for (int64_t i = a; i < b; i++) {
-        T v = data[i];
-        data[i] = run;
-        run += v;
-    }
-    if (t == 1023 && total) *total = part[1023];
+    if (threadIdx.x == 0) tot[blockIdx.x] = carry;
 }
 
 // Stable scatter: warp w of a tile owns kRsChunk consecutive items and walks
@@ -108,11 +115,24 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
                                                            uint32_t *__restrict__ kout,
                                                            int32_t *__restrict__ vout, int n,
                                                            int shift, const uint32_t *__restrict__ hist,
-                                                           int nblk) {
+                                                           const uint32_t *__restrict__ tot, int nblk) {
     __shared__ uint32_t cnt[kRsWarps][256];
+    __shared__ uint32_t wsum[kRsWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int d = threadIdx.x; d < kRsWarps * 256; d += kRsThreads) (&cnt[0][0])[d] = 0;
+    // where this thread's digit starts: the totals of the digits below
+    static_assert(kRsThreads == 256, "a thread per digit");
+    const uint32_t mine = tot[threadIdx.x];
+    uint32_t digit0 = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, digit0, o);
+        if (lane >= o) digit0 += y;
+    }
+    if (lane == 31) wsum[w] = digit0;
     __syncthreads();
+    digit0 -= mine;
+    for (int k = 0; k < w; k++) digit0 += wsum[k];
     const int base = blockIdx.x * kRsTile + w * kRsChunk;
     const uint32_t lt = (1u << lane) - 1u;
     for (int c = 0; c < kRsChunk; c += 32) {
@@ -125,7 +145,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
     __syncthreads();
     {
         int d = threadIdx.x;  // 256 threads == 256 digits
-        uint32_t off = hist[d * nblk + blockIdx.x];
+        uint32_t off = digit0 + hist[d * nblk + blockIdx.x];
         for (int ww = 0; ww < kRsWarps; ww++) {
             uint32_t t = cnt[ww][d];
             cnt[ww][d] = off;
@@ -198,13 +218,6 @@ __device__ __forceinline__ unsigned long long split_count_one(const uint32_t *ke
     return ((unsigned long long)big << 32) | (unsigned long long)big;
 }
 
-__global__ void k_split_count(const uint32_t *__restrict__ keys, Frontier fr, int nfr, int leaf_max,
-                              unsigned long long *__restrict__ cnt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nfr) return;
-    cnt[i] = split_count_one(keys, fr, i, leaf_max);
-}
-
 // Per frontier entry with its scanned offsets: the node's child references
 // and the next frontier's entries.
 __device__ __forceinline__ void split_emit_one(const uint32_t *keys, const Frontier &fr, int i, int leaf_max,
@@ -246,12 +259,62 @@ __device__ __forceinline__ void split_emit_one(const uint32_t *keys, const Front
     nref[node] = make_int4(ref[0], ref[1], ref[2], ref[3]);
 }
 
-__global__ void k_split_emit(const uint32_t *__restrict__ keys, Frontier fr, int nfr, int leaf_max,
-                             const unsigned long long *__restrict__ off, int node_base,
-                             int4 *__restrict__ nref, Frontier nx) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nfr) return;
-    split_emit_one(keys, fr, i, leaf_max, off[i], node_base, nref, nx);
+// Level sizes of a large layout's split, kept on the device: level k's
+// frontier has nfr[k] entries and made nodes[k] nodes (ids from 1 + the earlier
+// levels' nodes on; nodes[-1] is the root).
+constexpr int kMaxLevels = 64;
+struct SplitState {
+    int nfr[kMaxLevels + 2];
+    int made[kMaxLevels + 2];
+};
+
+// Exclusive scan over one block of 1024 threads; every thread gets the total.
+__device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long v, unsigned long long *wt,
+                                                             unsigned long long &total);
+
+// One level of the split: every frontier entry's count, its place by a block
+// scan and one atomic per block and output, and its emission.  Launched for
+// more levels than a layout is deep without asking: an empty frontier is a
+// launch that ends at once, where reading each level's size back (and scanning
+// it in one block) cost 70 us per level, 0.7 of the 1.1 ms of a 10^6-rect
+// tree.  Node ids within a level follow the blocks' order; every query's
+// traversal order is the children's, so its result does not depend on them.
+__global__ void __launch_bounds__(1024) k_split_level(const uint32_t *__restrict__ keys, Frontier fr, Frontier nx,
+                                                     int level, int leaf_max, SplitState *S,
+                                                     int4 *__restrict__ nref) {
+    __shared__ unsigned long long wt[32];
+    __shared__ int s_node, s_next;
+    const int nfr = S->nfr[level];
+    int base = 1;
+    for (int k = 0; k < level; k++) base += S->made[k];
+    for (int b0 = blockIdx.x * 1024; b0 < nfr; b0 += gridDim.x * 1024) {
+        const int i = b0 + threadIdx.x;
+        const unsigned long long v = i < nfr ? split_count_one(keys, fr, i, leaf_max) : 0ull;
+        unsigned long long total;
+        const unsigned long long e = block_scan_u64(v, wt, total);
+        if (threadIdx.x == 0) {
+            s_node = (int)(total >> 32) ? atomicAdd(&S->made[level], (int)(total >> 32)) : 0;
+            s_next = (int)total ? atomicAdd(&S->nfr[level + 1], (int)(total & 0xFFFFFFFFull)) : 0;
+        }
+        __syncthreads();
+        if (i < nfr) {
+            const unsigned long long at =
+                (((e >> 32) + (unsigned)s_node) << 32) | ((e & 0xFFFFFFFFull) + (unsigned)s_next);
+            split_emit_one(keys, fr, i, leaf_max, at, base, nref, nx);
+        }
+        __syncthreads();
+    }
+}
+
+// The child boxes of the nodes made by level `level` (-1: the root).
+__device__ __forceinline__ void refit_one(const float4 *rects, const int4 *nref, float4 *nbox, int node, int c);
+__global__ void k_refit_level(const float4 *__restrict__ rects, const int4 *__restrict__ nref,
+                              float4 *__restrict__ nbox, int level, const SplitState *__restrict__ S) {
+    int a = level < 0 ? 0 : 1;
+    for (int k = 0; k < level; k++) a += S->made[k];
+    const int b = level < 0 ? 1 : a + S->made[level];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * (b - a); t += gridDim.x * blockDim.x)
+        refit_one(rects, nref, nbox, a + (t >> 2), t & 3);
 }
 
 __device__ __forceinline__ float4 box_union(float4 a, float4 b) {
@@ -271,14 +334,6 @@ __device__ __forceinline__ void refit_one(const float4 *rects, const int4 *nref,
         for (int k = 0; k < m; k++) box = box_union(box, rects[f + k]);
     }
     nbox[4 * node + c] = box;
-}
-
-__global__ void k_refit(const float4 *__restrict__ rects, const int4 *__restrict__ nref,
-                        float4 *__restrict__ nbox, int a, int b) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    int node = a + (t >> 2), c = t & 3;
-    if (node >= b) return;
-    refit_one(rects, nref, nbox, node, c);
 }
 
 // Exclusive scan over one block of 1024 threads; every thread gets the total.
@@ -310,7 +365,6 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
 }
 
 constexpr int kSmallBuild = 1 << 16;  // layouts up to this many rects split and refit in one block
-constexpr int kMaxLevels = 64;
 
 // The whole level-synchronous split and the bottom-up refit of a small
 // layout in one block of 1024 threads: the same count -> scan -> emit steps
@@ -516,6 +570,7 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
     int32_t *v0 = nullptr, *v1 = nullptr;
     unsigned long long *cnt = nullptr, *tot = nullptr;
     int32_t *frb = nullptr;
+    void *split = nullptr;
     TreeBuffers T;
     frw_status rc = FRW_OK;
     auto ck = [&](cudaError_t e, const char *what) {
@@ -533,7 +588,7 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
         if (!ck(cudaMallocAsync(&k1, (size_t)n * 4, st), "malloc keys")) break;
         if (!ck(cudaMallocAsync(&v0, (size_t)n * 4, st), "malloc vals")) break;
         if (!ck(cudaMallocAsync(&v1, (size_t)n * 4, st), "malloc vals")) break;
-        if (!ck(cudaMallocAsync(&hist, (size_t)256 * nblk * 4, st), "malloc hist")) break;
+        if (!ck(cudaMallocAsync(&hist, (size_t)256 * (nblk + 1) * 4, st), "malloc hist")) break;
         if (!ck(cudaMallocAsync(&cnt, (size_t)cap_nodes * 8, st), "malloc cnt")) break;
         if (!ck(cudaMallocAsync(&tot, 16, st), "malloc tot")) break;  // scan total, or the small build's result
         if (!ck(cudaMallocAsync(&frb, (size_t)cap_nodes * 8 * 4, st), "malloc frontier")) break;
@@ -544,8 +599,8 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
         if (!ck(cudaGetLastError(), "k_morton")) break;
         for (int shift = 0; shift < 32; shift += 8) {
             k_rs_hist<<<nblk, kRsThreads, 0, st>>>(k0, n, shift, hist, nblk);
-            k_scan_excl<uint32_t><<<1, 1024, 0, st>>>(hist, (int64_t)256 * nblk, nullptr);
-            k_rs_scatter<<<nblk, kRsThreads, 0, st>>>(k0, v0, k1, v1, n, shift, hist, nblk);
+            k_rs_scan<<<256, kDigitThreads, 0, st>>>(hist, nblk, hist + (size_t)256 * nblk);
+            k_rs_scatter<<<nblk, kRsThreads, 0, st>>>(k0, v0, k1, v1, n, shift, hist, hist + (size_t)256 * nblk, nblk);
             if (!ck(cudaGetLastError(), "radix sort")) break;
             std::swap(k0, k1);
             std::swap(v0, v1);
@@ -577,40 +632,49 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
             if (build_ms) *build_ms = ms;
             break;
         }
-        int32_t root[4] = {0, 0, 0, n};
-        if (!ck(cudaMemcpyAsync(fa.node, &root[0], 4, cudaMemcpyHostToDevice, st), "root")) break;
-        if (!ck(cudaMemcpyAsync(fa.level, &root[1], 4, cudaMemcpyHostToDevice, st), "root")) break;
-        if (!ck(cudaMemcpyAsync(fa.start, &root[2], 4, cudaMemcpyHostToDevice, st), "root")) break;
-        if (!ck(cudaMemcpyAsync(fa.end, &root[3], 4, cudaMemcpyHostToDevice, st), "root")) break;
-        int nodes = 1, nfr = 1, depth = 0;
-        std::vector<int> batch = {0, 1};
-        for (int iter = 0; nfr > 0; iter++) {
-            if (iter > kMaxLevels) {
-                set_error("build_tree: too many levels");
-                rc = FRW_E_KERNEL;
-                break;
+        SplitState *S;
+        if (!ck(cudaMallocAsync(&S, sizeof(SplitState), st), "malloc levels")) break;
+        split = S;
+        SplitState h{};
+        h.nfr[0] = 1;
+        const int32_t root[4] = {0, 0, 0, n};
+        if (!ck(cudaMemcpyAsync(S, &h, sizeof(h), cudaMemcpyHostToDevice, st), "levels")) break;
+        for (int k = 0; k < 4 && rc == FRW_OK; k++)
+            ck(cudaMemcpyAsync(frb + (size_t)k * cap_nodes, &root[k], 4, cudaMemcpyHostToDevice, st), "root");
+        if (rc) break;
+        // as many levels as a uniform layout of n rects has and a few more, then
+        // as many again while the frontier is not empty
+        int expect = 4;
+        for (int64_t m = n; m > leaf_max; m >>= 2) expect++;
+        int levels = 0, nfr = 1;
+        while (nfr > 0 && levels < kMaxLevels) {
+            const int to = std::min(kMaxLevels, levels + expect);
+            for (; levels < to; levels++) {
+                // frontier entries are disjoint ranges above leaf_max, four per parent at most
+                const int64_t most = std::min<int64_t>(n / (leaf_max + 1) + 1, 1ll << std::min(2 * levels, 40));
+                k_split_level<<<(unsigned)std::min<int64_t>((most + 1023) / 1024, 296), 1024, 0, st>>>(
+                    k0, fa, fb, levels, leaf_max, S, T.nref);
+                std::swap(fa, fb);
             }
-            k_split_count<<<(nfr + 255) / 256, 256, 0, st>>>(k0, fa, nfr, leaf_max, cnt);
-            k_scan_excl<unsigned long long><<<1, 1024, 0, st>>>(cnt, nfr, tot);
-            unsigned long long h_tot = 0;
-            if ((rc = read_back(&h_tot, tot, 8, st, "build_tree: scan total"))) break;
-            int new_nodes = (int)(h_tot >> 32), next = (int)(h_tot & 0xFFFFFFFFull);
-            k_split_emit<<<(nfr + 255) / 256, 256, 0, st>>>(k0, fa, nfr, leaf_max, cnt, nodes, T.nref, fb);
             if (!ck(cudaGetLastError(), "split")) break;
-            if (new_nodes > 0) {
-                nodes += new_nodes;
-                batch.push_back(nodes);
-                depth++;
-            }
-            std::swap(fa, fb);
-            nfr = next;
+            if ((rc = read_back(&h, S, sizeof(h), st, "build_tree: levels"))) break;
+            nfr = h.nfr[levels];
         }
         if (rc) break;
-        for (int k = (int)batch.size() - 1; k > 0; k--) {
-            int a = batch[k - 1], b = batch[k];
-            int thr = 4 * (b - a);
-            k_refit<<<(thr + 255) / 256, 256, 0, st>>>(T.rects, T.nref, T.nbox, a, b);
+        if (nfr > 0) {
+            set_error("build_tree: too many levels");
+            rc = FRW_E_KERNEL;
+            break;
         }
+        int nodes = 1, depth = 0;
+        for (int k = 0; k < levels; k++) {
+            nodes += h.made[k];
+            depth += h.made[k] > 0;
+        }
+        for (int k = levels - 1; k >= -1; k--)
+            if (k < 0 || h.made[k] > 0)
+                k_refit_level<<<(unsigned)(((k < 0 ? 4 : 4 * (int64_t)h.made[k]) + 255) / 256), 256, 0, st>>>(
+                    T.rects, T.nref, T.nbox, k, S);
         if (!ck(cudaGetLastError(), "refit")) break;
         T.nodes = nodes;
         T.depth = depth;
@@ -622,7 +686,7 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
         if (build_ms) *build_ms = ms;
     } while (0);
     for (void *p : {(void *)k0, (void *)k1, (void *)v0, (void *)v1, (void *)hist, (void *)cnt, (void *)tot,
-                    (void *)frb})
+                    (void *)frb, split})
         if (p) cudaFreeAsync(p, st);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
