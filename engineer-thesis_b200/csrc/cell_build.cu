@@ -44,6 +44,7 @@ __device__ __forceinline__ bool touching(const DevLayout &L, const double B[4], 
     int stk[kStackMax];
     int sp = 1;
     stk[0] = 0;
+    const FloatBox fb = float_box(B);
     while (sp > 0) {
         const int nd = stk[--sp];
         const int4 rf = __ldg(L.nref + nd);
@@ -51,8 +52,7 @@ __device__ __forceinline__ bool touching(const DevLayout &L, const double B[4], 
         for (int c = 0; c < 4; c++) {
             if (ref[c] == kRefEmpty) continue;
             const float4 b = __ldg(L.nbox + 4 * nd + c);
-            if (!((double)b.z >= B[0] && B[2] >= (double)b.x && (double)b.w >= B[1] && B[3] >= (double)b.y))
-                continue;
+            if (!fb.touches(b)) continue;
             if (ref[c] >= 0) {
                 if (sp == kStackMax) return false;
                 stk[sp++] = ref[c];
@@ -61,8 +61,7 @@ __device__ __forceinline__ bool touching(const DevLayout &L, const double B[4], 
             const int f = leaf_first(ref[c]), m = leaf_count(ref[c]);
             for (int k = f; k < f + m; k++) {
                 const float4 r = __ldg(L.rects + k);
-                if ((double)r.z >= B[0] && B[2] >= (double)r.x && (double)r.w >= B[1] && B[3] >= (double)r.y)
-                    if (!visit(k, r)) return true;
+                if (fb.touches(r) && !visit(k, r)) return true;
             }
         }
     }
@@ -217,9 +216,10 @@ __global__ void __launch_bounds__(kRecordThreads)
     // visits the rects touching B in a fixed order
     auto each = [&](auto &&visit) {
         if (!kCoarse || ce.y < 0) return touching(L, B, [&](int k, float4 r) { return visit(L.ids + k, r); });
+        const FloatBox fb = float_box(B);
         for (int k = ce.x; k < ce.x + ce.y; k++) {
             const float4 r = __ldg(K.rects + k);
-            if (touches_box(r, B) && !visit(K.ids + k, r)) break;
+            if (fb.touches(r) && !visit(K.ids + k, r)) break;
         }
         return true;
     };
@@ -231,8 +231,16 @@ __global__ void __launch_bounds__(kRecordThreads)
             ce = __ldg(K.cells + (int64_t)(iy / factor) * K.nx + ix / factor);
         }
         if (kCoarse && ce.y >= 0) {
-            best = bounds_distance(L, p.x, p.y);
-            for (int k = ce.x; k < ce.x + ce.y; k++) best = dmin(best, rect_gap(__ldg(K.rects + k), p.x, p.y));
+            // the clearance in FP32 on a split centre (two roundings of the gap's
+            // own size), raised past its error: a radius a hair larger is as good
+            const float xh = (float)p.x, yh = (float)p.y;
+            const float xl = (float)(p.x - (double)xh), yl = (float)(p.y - (double)yh);
+            float g = 3.0e38f;
+            for (int k = ce.x; k < ce.x + ce.y; k++) {
+                const float4 r = __ldg(K.rects + k);
+                g = fminf(g, fmaxf(fmaxf((r.x - xh) - xl, (xh - r.z) + xl), fmaxf((r.y - yh) - yl, (yh - r.w) + yl)));
+            }
+            best = dmin(bounds_distance(L, p.x, p.y), (double)g + fabs((double)g) * 0x1p-21 + L.delta);
         } else {
             Cands C;
             int hit;

@@ -281,6 +281,18 @@ __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, c
 __device__ __forceinline__ bool touches_box(const float4 r, const double o[4]) {
     return (double)r.z >= o[0] && o[2] >= (double)r.x && (double)r.w >= o[1] && o[3] >= (double)r.y;
 }
+// The same test of FP32 rects without a conversion each: a float is >= an FP64
+// bound exactly when it is >= the bound rounded up to FP32, and <= one when it
+// is <= the bound rounded down.
+struct FloatBox {
+    float x0, y0, x1, y1;
+    __device__ __forceinline__ bool touches(const float4 r) const {
+        return r.z >= x0 && r.x <= x1 && r.w >= y0 && r.y <= y1;
+    }
+};
+__device__ __forceinline__ FloatBox float_box(const double B[4]) {
+    return FloatBox{__double2float_ru(B[0]), __double2float_ru(B[1]), __double2float_rd(B[2]), __double2float_rd(B[3])};
+}
 __device__ __forceinline__ bool collides_listed(const DevLayout &L, const Cands &C, const double o[4]) {
     if (!(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1)) return true;
     const float4 *r = L.rects;
@@ -552,6 +564,7 @@ __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, c
     int stk[kStackMax];
     int sp = 1;
     stk[0] = 0;
+    const FloatBox fb = float_box(B);
     while (sp > 0) {
         const int nd = stk[--sp];
         const int4 rf = __ldg(nref + nd);
@@ -559,8 +572,7 @@ __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, c
         for (int c = 0; c < 4; c++) {
             if (ref[c] == kRefEmpty) continue;
             const float4 b = __ldg(nbox + 4 * nd + c);
-            if (!((double)b.z >= B[0] && B[2] >= (double)b.x && (double)b.w >= B[1] && B[3] >= (double)b.y))
-                continue;
+            if (!fb.touches(b)) continue;
             if (ref[c] >= 0) {
                 if (sp < kStackMax) stk[sp++] = ref[c];
                 else st |= kStStackOverflow;
@@ -569,9 +581,10 @@ __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, c
             const int f = leaf_first(ref[c]), m = leaf_count(ref[c]);
             for (int k = f; k < f + m; k++) {
                 const float4 r = __ldg(rects + k);
+                if (!fb.touches(r)) continue;
                 const double x0 = r.x, y0 = r.y, x1 = r.z, y1 = r.w;
                 if (has_ign && x0 == ign[0] && y0 == ign[1] && x1 == ign[2] && y1 == ign[3]) continue;
-                if (x1 >= B[0] && B[2] >= x0 && y1 >= B[1] && B[3] >= y0) return true;
+                return true;
             }
         }
     }
