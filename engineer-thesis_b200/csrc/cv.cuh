@@ -54,12 +54,14 @@ frw_status launch_forward_tc(const Net &n, const __nv_bfloat16 *x, int64_t rows,
 // tcgen05 training step: each CTA writes its partial gradient to its slot of
 // part ([train_blocks_tc(rows, sms)][kPartStride] floats); launch_reduce_adam_tc
 // then sums the slots in CTA order and applies Adam at step t (1-based), or
-// launch_reduce_sum_tc adds them to a gradient.
+// launch_reduce_sum_tc adds them to a gradient.  after_update: the stream's
+// previous work is launch_reduce_adam_tc, so the step may start its set-up (and
+// read x, y and wt) before that ends.
 constexpr int kPartStride = (kParams + 3) & ~3;  // floats per CTA slot: 16-byte aligned slots
 int train_blocks_tc(int64_t rows, int sms);
 frw_status launch_train_grad_tc(const Net &n, const __nv_bfloat16 *x, const float *y, const float *wt, int64_t rows,
                                 float inv_wsum, float *part, double *loss, uint32_t *status, int sms,
-                                cudaStream_t st);
+                                cudaStream_t st, bool after_update = false);
 frw_status launch_reduce_adam_tc(const Net &n, const float *part, int nb, float *m, float *v, int t, float lr,
                                  cudaStream_t st);
 frw_status launch_reduce_sum_tc(const float *part, int nb, float *grad, cudaStream_t st);

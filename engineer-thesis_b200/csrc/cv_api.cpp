@@ -292,7 +292,7 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
             if (tc) {  // partial gradients per CTA, summed in CTA order with the Adam step
                 const int nb = cv::train_blocks_tc(rows, sms_tc);
                 rc = cv::launch_train_grad_tc(M->net, d_x + 16 * start, d_y + start, d_wt + start, rows, inv, d_part,
-                                              d_loss + s, d_tstatus, sms_tc, st);
+                                              d_loss + s, d_tstatus, sms_tc, st, s > 0);
                 if (!rc) rc = cv::launch_reduce_adam_tc(M->net, d_part, nb, d_m, d_v, s + 1, co.lr, st);
             } else {
                 rc = cv::launch_train_grad(M->net, d_x + 16 * start, d_y + start, d_wt + start, rows, inv, d_grad,
