@@ -623,7 +623,8 @@ __device__ __forceinline__ void point_from_index(const double s[4], int index, b
     const double w2 = __dmul_rn(2.0, w);
     const double per2 = __dadd_rn(w2, __dmul_rn(2.0, h));
     const double v = exact ? __ddiv_rn(per2, (double)FRW_NSAMPLE) : div200((double)__double2int_rz(per2));
-    const double iv = __dmul_rn((double)index, v), jv = __dmul_rn((double)(index - 1), v);
+    const double fi = (double)index;
+    const double iv = __dmul_rn(fi, v), jv = __dmul_rn(__dsub_rn(fi, 1.0), v);
     const double hv = __dmul_rn(v, 0.5);
     const double wh = __dadd_rn(w, h), w2h = __dadd_rn(w2, h);
     // where the index lies, in the reference's order of tests: top, its corner

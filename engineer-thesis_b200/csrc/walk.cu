@@ -40,13 +40,11 @@ constexpr int kWalkThreads = 256;
 // half of the lanes that need one; one hop 6% and three hops 6% slower than
 // two: their draws are needed by some lane in every hop).
 constexpr int kHopsPerRound = 4;
-// Resident blocks per SM: 5 blocks of 256 (40 warps) at 48 registers per
-// thread, for weighted (uniform start) and unweighted walks alike (weighted
-// walks spill a little more there but gain from the extra warps since the
-// loop runs two hops per round; 4 blocks at 64 registers: 1.6% slower) --
-// except weighted walks of many jobs, whose per-job loads need the registers
-// (4 blocks at 64 registers: 6% faster than 5 at 48).
-constexpr int kWalkMinBlocksMultiW = 4;
+// Resident blocks of 256 per SM: 5 at 48 registers for unweighted walks, 4 at 64
+// for weighted (uniform start) ones, whose state is larger (1e7 capacitance
+// walks on 10^4 rects 2.06 -> 1.98 ms, 1e7 control-variate walks 2.12 -> 2.02,
+// 28 batched layouts 2.18 -> 1.94 against 5; unweighted walks equal either way).
+constexpr int kWalkMinBlocksW = 4;
 constexpr int kWalkMinBlocks = 5;
 constexpr int kWarpsPerBlock = kWalkThreads / 32;
 constexpr int kTabSlots = 32;  // per warp
@@ -268,7 +266,7 @@ __device__ __forceinline__ void tab_round(const WalkParams &P, Slot *tab, int la
 // list holds take the whole-tree replay; without it that code is compiled
 // out of the kernel.
 template <bool kMulti, bool kRec, bool kUniform, bool kCV = false, bool kTies = false>
-__global__ void __launch_bounds__(kWalkThreads, kMulti && kUniform ? kWalkMinBlocksMultiW : kWalkMinBlocks)
+__global__ void __launch_bounds__(kWalkThreads, kUniform ? kWalkMinBlocksW : kWalkMinBlocks)
     k_walk(const WalkParams P) {
     __shared__ double s_intg[FRW_NSAMPLE + 1];
     __shared__ double s_wx[FRW_NSAMPLE], s_wy[FRW_NSAMPLE];
@@ -306,6 +304,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMulti && kUniform ? kWalkMinBlo
     const int refill_min = P.refill_min < 1 ? 1 : (P.refill_min > 32 ? 32 : P.refill_min);
     constexpr bool uniform_start = kUniform;
     const bool exact = P.exact_perimeter != 0;
+    const int32_t hop_cap = P.hop_cap < 0x7FFFFFFF ? (int32_t)P.hop_cap : 0x7FFFFFFF;
     const uint64_t seed = P.seed_dev ? *P.seed_dev : P.seed;
     const uint64_t kChunk = P.chunk;
 
@@ -479,7 +478,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMulti && kUniform ? kWalkMinBlo
                 const DevLayout &L = J.L;
                 // distance to the bounds: p is strictly inside exactly when it is
                 // > 0 (each difference is > 0 exactly when p is on that side)
-                const double bd = fmin(fmin(px - L.bx0, L.bx1 - px), fmin(py - L.by0, L.by1 - py));
+                const double bd = dmin(dmin(px - L.bx0, L.bx1 - px), dmin(py - L.by0, L.by1 - py));
                 if (!(bd > 0.0)) {
                     code = -1;  // escaped: left the layer bounds
                 } else {
@@ -489,7 +488,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMulti && kUniform ? kWalkMinBlo
                     st |= query_point<true, !kUniform, kTies>(L, px, py, sq, hit, bd);
                     hops++;
                     if (hit != kNoHit) code = hit;
-                    else if (hops >= P.hop_cap) code = -2;
+                    else if (hops >= hop_cap) code = -2;
                 }
             }
         }
