@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kRecordThreads)
     int2 ce = make_int2(0, -1);
     double B[4] = {0, 0, 0, 0};
     int n = 0;
-    bool tree = false;
+    bool tree = false, near = false;
     // visits the rects touching B in a fixed order
     auto each = [&](auto &&visit) {
         if (!kCoarse || ce.y < 0) return touching(L, B, [&](int k, float4 r) { return visit(L.ids + k, r); });
@@ -225,7 +225,9 @@ __global__ void __launch_bounds__(kRecordThreads)
     };
     if (c >= 0) {
         const double2 p = centre_of(G, c);
-        double best = -1.0;
+        // clearance at the centre: of the bounds, and of the rects (at least)
+        const double bd = bounds_distance(L, p.x, p.y);
+        double gap = 1e300;
         if (kCoarse) {
             const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
             ce = __ldg(K.cells + (int64_t)(iy / factor) * K.nx + ix / factor);
@@ -240,13 +242,16 @@ __global__ void __launch_bounds__(kRecordThreads)
                 const float4 r = __ldg(K.rects + k);
                 g = fminf(g, fmaxf(fmaxf((r.x - xh) - xl, (xh - r.z) + xl), fmaxf((r.y - yh) - yl, (yh - r.w) + yl)));
             }
-            best = dmin(bounds_distance(L, p.x, p.y), (double)g + fabs((double)g) * 0x1p-21 + L.delta);
+            gap = (double)g + fabs((double)g) * 0x1p-21 + L.delta;
         } else {
             Cands C;
             int hit;
-            clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
+            if (bd >= 0.0) clearance(L, p.x, p.y, C, hit, gap, 1e300);
         }
-        const double r = radius_of(L, G, best);
+        // both clearances change by at most the distance moved: no point of a
+        // cell that is not `near` has the bounds as near as its nearest rect or 3
+        near = !(bd - 0.5 * G.side > dmax(gap + 0.5 * G.side, 3.0) + 2.0 * L.delta + G.margin);
+        const double r = radius_of(L, G, dmin(bd, gap));
         grown_box(G, c, r, B);
         // a point of the cell lies within margin/2 of it whatever the rounding of
         // its cell index, so every rect within r - margin of the point is listed
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(kRecordThreads)
         }
     }
     // offsets of the longer lists: a warp scan, the warps' totals, one atomic
-    const unsigned want = !tree && n > kCellSlots ? (unsigned)n : 0u;
+    const unsigned want = !tree && n >= kCellSlots + (near ? 0 : 1) ? (unsigned)n : 0u;
     unsigned x = want;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -286,12 +291,12 @@ __global__ void __launch_bounds__(kRecordThreads)
         s_base = s ? atomicAdd(tot, (unsigned long long)s) : 0ull;
     }
     __syncthreads();
-    if (!want && !tree) return;
+    if (c < 0 || !(want || tree || near)) return;
     unsigned long long at = s_base + (x - want);
     for (int k = 0; k < w; k++) at += s_warp[k];
     float4 *rec = cells + kCellSlots * c;
     rec[kCellSlots - 1] = make_float4(kListRect, __int_as_float(tree ? 0 : (int)at), __int_as_float(tree ? kTreeCell : n), 0.f);
-    if (tree || at + want > (unsigned long long)room) return;
+    if (!want || at + want > (unsigned long long)room) return;
     int m = 0;
     each([&](const int32_t *id, float4 q) {
         crects[at + m] = q;

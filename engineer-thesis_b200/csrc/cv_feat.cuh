@@ -100,10 +100,12 @@ static __device__ __forceinline__ bool nearest_other(const DevLayout &L, double 
         const int32_t *ids = reinterpret_cast<const int32_t *>(L.cellids + cell);
         const float4 last = __ldg(r + kCellSlots - 1);
         int n = kCellSlots;
-        if (last.x > kFarRect) {  // a longer list, or (n < 0) the tree
+        if (last.x > kFarRect) {  // a longer list, a short one near the bounds, or (n < 0) the tree
             n = __float_as_int(last.z);
-            r = L.crects + __float_as_int(last.y);
-            ids = L.cids + __float_as_int(last.y);
+            if (n >= kCellSlots) {
+                r = L.crects + __float_as_int(last.y);
+                ids = L.cids + __float_as_int(last.y);
+            }
         }
         if (n >= 0) {
             double best = 1e300;

@@ -208,7 +208,6 @@ frw_status poll_event(cudaEvent_t ev, const char *what) {
 frw_status status_error(uint32_t h) {
     if (h) {
         std::string m = "kernel reported:";
-        if (h & kStCandOverflow) m += " near-tie candidate list overflow;";
         if (h & kStStackOverflow) m += " traversal stack overflow;";
         if (h & kStReplayCap) m += " bisection replay iteration bound exceeded;";
         if (h & kStBadInput) m += " invalid input;";

@@ -36,12 +36,14 @@ FRW_HD int leaf_first(int ref) { return (-2 - ref) >> kLeafBits; }
 FRW_HD int leaf_count(int ref) { return (-2 - ref) & kLeafCountMax; }
 
 // A cell's record: its rects, unused slots holding a rect too far to matter
-// (kFarRect in every coordinate); or, when it lists more than kCellSlots
-// rects, its first kCellSlots - 1 and a last slot of kListRect and the bits of
-// (first, count, -): all its rects are entries first .. first + count - 1 of
-// the lists, count < 0 when the tree answers the cell's points.  Read as a
-// rect that slot is as far as an unused one (first < kMaxListEntries keeps its
-// bits below kListRect), so the gaps of a record need no test.
+// (kFarRect in every coordinate); or, when it lists more than kCellSlots rects
+// or lies near the bounds (where a point's clearance can be the bounds'), its
+// first kCellSlots - 1 rects and a last slot of kListRect and the bits of
+// (first, count, -): all its rects, when there are kCellSlots or more, are
+// entries first .. first + count - 1 of the lists; count < 0 when the tree
+// answers the cell's points.  Read as a rect that slot is as far as an unused
+// one (first < kMaxListEntries keeps its bits below kListRect), so the gaps of
+// a record need no test.
 constexpr int kCellSlots = 4;
 constexpr float kFarRect = 3.0e38f, kListRect = 3.3e38f;
 constexpr int64_t kMaxListEntries = 0x7F000000;
@@ -77,7 +79,6 @@ struct DevLayout {
 
 // ---- device status word (atomicOr'ed by kernels, read back by the host) ----
 enum : uint32_t {
-    kStCandOverflow = 1u,   // more near-tied rects than the candidate list holds
     kStStackOverflow = 2u,  // traversal stack overflow
     kStReplayCap = 4u,      // bisection replay exceeded its iteration bound
     kStBadInput = 8u,       // a kernel met an input outside its contract

@@ -32,7 +32,8 @@ __global__ void __launch_bounds__(128, kTies ? 8 : 12)
         const double2 p = __ldcs(pts + i);
         double s[4];
         int h;
-        st = query_point<false, false, kTies>(L, p.x, p.y, s, h);
+        if (kTies) st = query_point(L, p.x, p.y, s, h);
+        else query_record<false>(L, p.x, p.y, s, h, st);
         store_square(sq + i, s);
         __stcs((long long *)hit + i, h == kNoHit ? -1ll : (long long)h);
     }

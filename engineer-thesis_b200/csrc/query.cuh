@@ -61,14 +61,12 @@ __device__ __forceinline__ float lb_box_f(const float4 b, float px, float py) {
     return fmaxf(fmaxf(fmaxf(b.x - px, px - b.z), fmaxf(b.y - py, py - b.w)), 0.f);
 }
 
-// One rect of a leaf or a cell list: FP32 screen, then the exact FP64 gap;
+// One rect of a leaf: FP32 screen, then the exact FP64 gap;
 // tightens `best`, keeps the near-tie list and the containing rect.
-// kTies: a full list marks the point (C.first = -2) for the whole-tree
-// replay; otherwise a full list is an error.
-template <bool kTies>
+// A full list marks the point (C.first = -2) for the whole-tree replay.
 __device__ __forceinline__ void scan_rect(const float4 r, int k, const int32_t *ids, double px, double py,
                                           float pxf, float pyf, double r2, float slack, float &limf,
-                                          double &best, int &hit, Cands &C, uint32_t &st) {
+                                          double &best, int &hit, Cands &C) {
     const float gf = fmaxf(fmaxf(r.x - pxf, pxf - r.z), fmaxf(r.y - pyf, pyf - r.w));
     if (gf > limf) return;
     const double x0 = r.x, y0 = r.y, x1 = r.z, y1 = r.w;
@@ -94,13 +92,11 @@ __device__ __forceinline__ void scan_rect(const float4 r, int k, const int32_t *
             C.idx[C.n] = k;
             C.g[C.n] = __double2float_rd(g);
             C.n++;
-        } else if (kTies) {
+        } else {
             // more ties than the list holds (rects with aligned sides tie
             // exactly: a column of equal x0 seen from its left): the replay's
             // boxes near the clearance are then tested against the whole tree
             C.first = -2;
-        } else {
-            st |= kStCandOverflow;
         }
     }
 }
@@ -109,7 +105,6 @@ __device__ __forceinline__ void scan_rect(const float4 r, int k, const int32_t *
 // depth-first, nearest-child-first traversal from the bounds distance in
 // `best`; FP32 screens (errors below slack), the exact FP64 gap only for
 // rects that can matter.
-template <bool kTies>
 __device__ __forceinline__ uint32_t tree_clearance(const float4 *nbox, const int4 *nref, const float4 *rects,
                                                    const int32_t *ids, double px, double py, double r2, float slack,
                                                    Cands &C, int &hit, double &best) {
@@ -138,7 +133,7 @@ __device__ __forceinline__ uint32_t tree_clearance(const float4 *nbox, const int
             if (ref[c] >= kRefEmpty || lb[c] > limf) continue;
             const int f = leaf_first(ref[c]), m = leaf_count(ref[c]);
             for (int k = f; k < f + m; k++)
-                scan_rect<kTies>(__ldg(rects + k), k, ids, px, py, pxf, pyf, r2, slack, limf, best, hit, C, st);
+                scan_rect(__ldg(rects + k), k, ids, px, py, pxf, pyf, r2, slack, limf, best, hit, C);
         }
         // internal children within reach: visit the nearest next, stack the rest
         int next = -1;
@@ -177,12 +172,11 @@ __device__ __forceinline__ uint32_t tree_clearance(const float4 *nbox, const int
 }
 
 // The same, out of line (a call: smaller code where the tree is rare).
-template <bool kTies>
 static __device__ __noinline__ uint32_t tree_clearance_call(const float4 *nbox, const int4 *nref,
                                                             const float4 *rects, const int32_t *ids, double px,
                                                             double py, double r2, float slack, Cands &C, int &hit,
                                                             double &best) {
-    return tree_clearance<kTies>(nbox, nref, rects, ids, px, py, r2, slack, C, hit, best);
+    return tree_clearance(nbox, nref, rects, ids, px, py, r2, slack, C, hit, best);
 }
 
 // The cell of a point inside the bounds (the far edge's cells by clamping).
@@ -243,8 +237,7 @@ __device__ __forceinline__ bool record_clearance(const DevLayout &L, int64_t cel
 // bd: p's distance to the bounds (negative outside).
 // kInside: the caller has checked that p lies inside the bounds.
 // kOutOfLineTree: the tree traversal is a call (smaller code at the caller).
-// kTies: see scan_rect.
-template <bool kInside = false, bool kOutOfLineTree = false, bool kTies = true>
+template <bool kInside = false, bool kOutOfLineTree = false>
 __device__ __forceinline__ uint32_t clearance(const DevLayout &L, double px, double py, Cands &C,
                                               int &hit, double &best, double bd) {
     uint32_t st = 0;
@@ -267,8 +260,8 @@ __device__ __forceinline__ uint32_t clearance(const DevLayout &L, double px, dou
         if (record_clearance(L, cell, r0, r1, r2, r3, px, py, C, hit, best)) return st;
     }
     if (kOutOfLineTree)
-        return tree_clearance_call<kTies>(L.nbox, L.nref, L.rects, L.ids, px, py, r2, L.slack, C, hit, best);
-    return tree_clearance<kTies>(L.nbox, L.nref, L.rects, L.ids, px, py, r2, L.slack, C, hit, best);
+        return tree_clearance_call(L.nbox, L.nref, L.rects, L.ids, px, py, r2, L.slack, C, hit, best);
+    return tree_clearance(L.nbox, L.nref, L.rects, L.ids, px, py, r2, L.slack, C, hit, best);
 }
 
 __device__ __forceinline__ bool tree_box(const float4 *nbox, const int4 *nref, const float4 *rects,
@@ -293,23 +286,49 @@ struct FloatBox {
 __device__ __forceinline__ FloatBox float_box(const double B[4]) {
     return FloatBox{__double2float_ru(B[0]), __double2float_ru(B[1]), __double2float_rd(B[2]), __double2float_rd(B[3])};
 }
-__device__ __forceinline__ bool collides_listed(const DevLayout &L, const Cands &C, const double o[4]) {
-    if (!(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1)) return true;
-    const float4 *r = L.rects;
-    int n = C.n;
-    if (C.first >= 0) {  // the cell's record, or its list when it has one (slots too far touch nothing)
-        r = L.cells + (int64_t)kCellSlots * C.first;
-        n = kCellSlots;
+__device__ __forceinline__ bool leaves_bounds(const DevLayout &L, const double o[4]) {
+    return !(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1);
+}
+// What the boxes within delta of the clearance are tested against: the rects
+// of a cell (its record, or its list when it has one; slots too far touch
+// nothing) ...
+struct RecordTies {
+    int64_t cell;
+    __device__ __forceinline__ bool collides(const DevLayout &L, const double o[4], uint32_t &) const {
+        if (leaves_bounds(L, o)) return true;
+        const float4 *r = L.cells + kCellSlots * cell;
+        int n = kCellSlots - 1;
         const float4 last = __ldg(r + kCellSlots - 1);
         if (last.x > kFarRect) {
-            r = L.crects + __float_as_int(last.y);
-            n = __float_as_int(last.z);
+            if (__float_as_int(last.z) >= kCellSlots) {
+                r = L.crects + __float_as_int(last.y);
+                n = __float_as_int(last.z);
+            }
+        } else if (touches_box(last, o)) {
+            return true;
         }
+        for (int q = 0; q < n; q++)
+            if (touches_box(__ldg(r + q), o)) return true;
+        return false;
     }
-    for (int q = 0; q < n; q++)
-        if (touches_box(__ldg(r + (C.first >= 0 ? q : C.idx[q])), o)) return true;
-    return false;
-}
+};
+// ... the near-tie list of a point answered by the tree (or its cell) ...
+struct ListedTies {
+    const Cands &C;
+    __device__ __forceinline__ bool collides(const DevLayout &L, const double o[4], uint32_t &st) const {
+        if (C.first >= 0) return RecordTies{C.first}.collides(L, o, st);
+        if (leaves_bounds(L, o)) return true;
+        for (int q = 0; q < C.n; q++)
+            if (touches_box(__ldg(L.rects + C.idx[q]), o)) return true;
+        return false;
+    }
+};
+// ... or, when that list overflowed, the whole tree (checkCollisions(box)).
+struct TreeTies {
+    __device__ __forceinline__ bool collides(const DevLayout &L, const double o[4], uint32_t &st) const {
+        return leaves_bounds(L, o) || tree_box(L.nbox, L.nref, L.rects, o, false, nullptr, st);
+    }
+};
 
 // Decision of one box of the replay.  Its four extents (distances from p to
 // its sides) lie within eps << delta of each other, so comparing one extent
@@ -327,19 +346,11 @@ __device__ __forceinline__ Window replay_window(const DevLayout &L, double px, d
     return Window{__dadd_rn(px, __dadd_rn(dstar, L.delta)), __dadd_rn(px, __dsub_rn(dstar, L.delta))};
 }
 
-// kTree: the near-tie list overflowed (C.first == -2) and the exact
-// predicate is the whole tree's checkCollisions(box).
-template <bool kTree>
-__device__ __forceinline__ bool collides_box(const DevLayout &L, const Cands &C, const double o[4],
+template <class Ties>
+__device__ __forceinline__ bool collides_box(const DevLayout &L, const Ties &T, const double o[4],
                                              const Window &W, uint32_t &st) {
     bool c = o[2] > W.hi;
-    if (!c && !(o[2] < W.lo)) {  // rare: within delta of the clearance
-        if (kTree)
-            c = !(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1) ||
-                tree_box(L.nbox, L.nref, L.rects, o, false, nullptr, st);
-        else
-            c = collides_listed(L, C, o);
-    }
+    if (!c && !(o[2] < W.lo)) c = T.collides(L, o, st);  // rare: within delta of the clearance
     return c;
 }
 
@@ -444,8 +455,8 @@ __device__ __forceinline__ void box_at(double px, double py, double h, double o[
 // keeps that.  Its test against the listed rects ran in nearly every round of
 // a warp (1e7 capacitance walks on 10^4 rects 2.22 -> 2.06 ms without it).  Not so where
 // the bounds, which a box may touch, are as near (bd: their distance).
-template <bool kTree = false>
-__device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cands &C, double px,
+template <class Ties>
+__device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Ties &T, double px,
                                                   double py, double dstar, double bd, double o[4]) {
     uint32_t st = 0;
     const bool one = dstar < 1.5;
@@ -453,13 +464,7 @@ __device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cand
     box_at(px, py, h, o);
     const double e = __dsub_rn(dstar, h);
     bool c = e < -L.delta || (e <= 0.0 && bd > 3.0 && fabs(px) >= 4.0 && fabs(py) >= 4.0);
-    if (!c && e <= L.delta) {  // rare: within delta of the clearance
-        if (kTree)
-            c = !(o[1] >= L.by0 && o[0] >= L.bx0 && o[3] <= L.by1 && o[2] <= L.bx1) ||
-                tree_box(L.nbox, L.nref, L.rects, o, false, nullptr, st);
-        else
-            c = collides_listed(L, C, o);
-    }
+    if (!c && e <= L.delta) c = T.collides(L, o, st);  // rare: within delta of the clearance
     if (c) return st;
     box_at(px, py, one ? 2.0 : 1.0, o);
     if (one) return st;  // p +- 1 is free and p +- 2 collides
@@ -479,14 +484,14 @@ __device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cand
     int it = 1;
     // Growth (the reference's maxReached still false): grow by dist, without
     // halving, until a box collides.
-    bool isc = collides_box<kTree>(L, C, o, W, st);
+    bool isc = collides_box(L, T, o, W, st);
     while (!isc) {
         o[0] = __dsub_rn(o[0], dist);
         o[1] = __dsub_rn(o[1], dist);
         o[2] = __dadd_rn(o[2], dist);
         o[3] = __dadd_rn(o[3], dist);
         if (++it > kReplayCap) return st | kStReplayCap;
-        isc = collides_box<kTree>(L, C, o, W, st);
+        isc = collides_box(L, T, o, W, st);
     }
     // Bisection (maxReached): the loop runs while the box collides or dist is
     // above MIN_DIST; a colliding box shrinks by dist, halved first while above
@@ -506,7 +511,7 @@ __device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cand
         o[1] = __dadd_rn(o[1], sd);
         o[2] = __dsub_rn(o[2], sd);
         o[3] = __dsub_rn(o[3], sd);
-        isc = collides_box<kTree>(L, C, o, W, st);
+        isc = collides_box(L, T, o, W, st);
     }
     while (isc) {
         o[0] = __dadd_rn(o[0], dist);
@@ -517,7 +522,7 @@ __device__ __forceinline__ uint32_t replay_square(const DevLayout &L, const Cand
             st |= kStReplayCap;
             break;
         }
-        isc = collides_box<kTree>(L, C, o, W, st);
+        isc = collides_box(L, T, o, W, st);
     }
     return st;
 }
@@ -530,32 +535,82 @@ struct ReplayOut {
 };
 static __device__ __noinline__ ReplayOut replay_tree_call(const DevLayout L, double px, double py,
                                                           double dstar, double bd) {
-    Cands C;
-    C.n = 0;
-    C.first = -2;
     ReplayOut r;
-    r.st = replay_square<true>(L, C, px, py, dstar, bd, r.sq);
+    r.st = replay_square(L, TreeTies{}, px, py, dstar, bd, r.sq);
     return r;
 }
 
-// drawBiggestSquareAtPoint + checkCollisons(point) for one point.  kTies:
-// points with more near ties than the list holds take the whole-tree replay
-// (else they report kStCandOverflow).
-template <bool kInside = false, bool kOutOfLineTree = false, bool kTies = true>
+// drawBiggestSquareAtPoint + checkCollisons(point) for one point; points with
+// more near ties than the list holds take the whole-tree replay.
+template <bool kInside = false, bool kOutOfLineTree = false>
 __device__ __forceinline__ uint32_t query_point(const DevLayout &L, double px, double py, double sq[4],
                                                 int &hit, double bd = -1.0) {
     Cands C;
     double best;
     if (!kInside) bd = fmin(fmin(px - L.bx0, L.bx1 - px), fmin(py - L.by0, L.by1 - py));
-    uint32_t st = clearance<kInside, kOutOfLineTree, kTies>(L, px, py, C, hit, best, bd);
-    if (kTies && C.first == -2) {
+    uint32_t st = clearance<kInside, kOutOfLineTree>(L, px, py, C, hit, best, bd);
+    if (C.first == -2) {
         const ReplayOut r = replay_tree_call(L, px, py, best, bd);
         sq[0] = r.sq[0]; sq[1] = r.sq[1]; sq[2] = r.sq[2]; sq[3] = r.sq[3];
         st |= r.st;
     } else {
-        st |= replay_square(L, C, px, py, best, bd, sq);
+        st |= replay_square(L, ListedTies{C}, px, py, best, bd, sq);
     }
     return st;
+}
+
+// The same where cell records answer every point (no tree_points), without the
+// tree's code.  kWalk: p is a walk's point, which ends the walk (false) when it
+// is not strictly inside the bounds; only cells near them -- whose last slot
+// says so, see cell_build.cu -- look at the bounds at all.  Otherwise p is any
+// point.  (With the tree's code and the bounds in every hop: 2e7 walks on 10^6
+// rects 5.48 ms against 5.09, 1e7 capacitance walks on 10^4 1.98 against 1.89,
+// 1e7 queries 0.452 against 0.439.)
+template <bool kWalk>
+__device__ __forceinline__ bool query_record(const DevLayout &L, double px, double py, double sq[4], int &hit,
+                                             uint32_t &st) {
+    hit = kNoHit;
+    double best = 1e300, bd = 1e300;
+    int64_t cell = 0;
+    auto bounds = [&]() { return dmin(dmin(px - L.bx0, L.bx1 - px), dmin(py - L.by0, L.by1 - py)); };
+    bool in = true;
+    if (!kWalk) {
+        in = px >= L.bx0 && py >= L.by0 && px <= L.bx1 && py <= L.by1;
+        bd = best = in ? bounds() : -1.0;
+    }
+    if (in) {
+        cell = cell_of(L, px, py);
+        float4 r0, r1, r2, r3;
+        load_pair(L.cells + kCellSlots * cell, r0, r1);
+        load_pair(L.cells + kCellSlots * cell + 2, r2, r3);
+        const double g0 = rect_gap(r0, px, py), g1 = rect_gap(r1, px, py), g2 = rect_gap(r2, px, py),
+                     g3 = rect_gap(r3, px, py);
+        const double g = dmin(dmin(g0, g1), dmin(g2, g3));
+        best = kWalk ? g : dmin(best, g);
+        if (!(g > 0.0)) {  // p may lie in listed rects: the lowest layer index
+            const int4 id = __ldg(L.cellids + cell);
+            if (g0 <= 0.0) hit = min(hit, id.x);
+            if (g1 <= 0.0) hit = min(hit, id.y);
+            if (g2 <= 0.0) hit = min(hit, id.z);
+            if (g3 <= 0.0) hit = min(hit, id.w);
+        }
+        if (r3.x > kFarRect) {  // near the bounds, or a longer list
+            if (kWalk) {
+                bd = bounds();
+                if (!(bd > 0.0)) return false;
+                best = dmin(best, bd);
+            }
+            const int n = __float_as_int(r3.z);
+            for (int k = kCellSlots - 1; k < n; k++) {
+                const int i = __float_as_int(r3.y) + k;
+                const double gk = rect_gap(__ldg(L.crects + i), px, py);
+                if (gk <= 0.0) hit = min(hit, __ldg(L.cids + i));
+                best = dmin(best, gk);
+            }
+        }
+    }
+    st |= replay_square(L, RecordTies{cell}, px, py, best, bd, sq);
+    return true;
 }
 
 // Tree::checkCollisions(box, ignore) for an arbitrary box (complete DFS).

@@ -262,9 +262,8 @@ __device__ __forceinline__ void tab_round(const WalkParams &P, Slot *tab, int la
 // the Green-CDF start every weight is 0, so the weight, its inputs and the
 // weight sums are compiled out.  kCV: the control variate's sums (P.cv_phi,
 // P.cv_sums) are kept beside the rows.  kTies: the tree answers some points
-// (P.tree_points), and those with more exact near ties than its candidate
-// list holds take the whole-tree replay; without it that code is compiled
-// out of the kernel.
+// (P.tree_points); without it cell records answer every point and the tree's
+// code is compiled out of the kernel.
 template <bool kMulti, bool kRec, bool kUniform, bool kCV = false, bool kTies = false>
 __global__ void __launch_bounds__(kWalkThreads, kUniform ? kWalkMinBlocksW : kWalkMinBlocks)
     k_walk(const WalkParams P) {
@@ -476,16 +475,22 @@ __global__ void __launch_bounds__(kWalkThreads, kUniform ? kWalkMinBlocksW : kWa
             if (go) {
                 const WalkJob &J = job_of<kMulti>(P, job);
                 const DevLayout &L = J.L;
-                // distance to the bounds: p is strictly inside exactly when it is
-                // > 0 (each difference is > 0 exactly when p is on that side)
-                const double bd = dmin(dmin(px - L.bx0, L.bx1 - px), dmin(py - L.by0, L.by1 - py));
-                if (!(bd > 0.0)) {
+                int hit;
+                bool in = true;
+                if (kTies) {
+                    // distance to the bounds: p is strictly inside exactly when it is
+                    // > 0 (each difference is > 0 exactly when p is on that side)
+                    const double bd = dmin(dmin(px - L.bx0, L.bx1 - px), dmin(py - L.by0, L.by1 - py));
+                    in = bd > 0.0;
+                    // the tree traversal is a call in the 48-register kernel, whose
+                    // code it would otherwise crowd
+                    if (in) st |= query_point<true, !kUniform>(L, px, py, sq, hit, bd);
+                } else {
+                    in = query_record<true>(L, px, py, sq, hit, st);
+                }
+                if (!in) {
                     code = -1;  // escaped: left the layer bounds
                 } else {
-                    int hit;
-                    // the rare tree traversal (overflowed cells) is a call in the
-                    // 48-register kernel, whose code it would otherwise crowd
-                    st |= query_point<true, !kUniform, kTies>(L, px, py, sq, hit, bd);
                     hops++;
                     if (hit != kNoHit) code = hit;
                     else if (hops >= hop_cap) code = -2;

@@ -62,3 +62,27 @@ def test_lists_past_the_first_buffer():
                 assert c.overflow_cells == 0 and c.entries > c.cells
             sq, hit = L.query(p)
             assert np.array_equal(sq, ref) and np.array_equal(hit, hit_ref)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 9])
+@pytest.mark.parametrize("margin", [0.0, 2.5, 40.0, 900.0])
+def test_walks_near_the_bounds(k, margin):
+    """Walks of few rects in bounds from touching them to far away: cells near
+    the bounds look at them, the others do not; most walks escape.  Per-walk
+    records equal the oracle's for both start modes."""
+    r = row_of(k)
+    b = np.array([r[:, 0].min() - margin, r[:, 1].min() - margin, r[:, 2].max() + margin, r[:, 3].max() + margin])
+    G = O.Grid(r, b)
+    escaped = 0
+    with frw.Layout.from_rects(r, b) as L:
+        for o in (frw.opts(), frw.capacitance_opts(1.0)):
+            for cells_per_rect in (16.0, 300.0):
+                L.set_cells(cells_per_rect)
+                end, hops, b1, w = L.walk_trace(k - 1, 0, 3000, 11, o)
+                cfg = G.walk_cfg(target=k - 1, gauss_mode=o.gauss_mode, gauss_param=o.gauss_param,
+                                 start_mode=o.start_mode, hop_cap=o.hop_cap, seed=11)
+                ref = G.walks(cfg, 0, 3000)
+                for x, y in zip((end, hops, b1, w), ref):
+                    assert np.array_equal(x, y)
+                escaped += int((end == -1).sum())
+    assert escaped > 0
