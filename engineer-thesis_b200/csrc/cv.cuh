@@ -36,8 +36,20 @@ frw_status net_refresh_bf16(const Net &n, cudaStream_t st);
 // features of points p (first-hop points) w.r.t. a target rect: the
 // (dx, dy) from p to the nearest point of each edge of the target and of
 // the nearest other conductor, divided by a0 and clamped to [-16, 16].
-frw_status launch_features(const DevLayout &L, double4 target_rect, int target_id, const double4 *rec,
-                           int64_t n, __nv_bfloat16 *xb, float *xf, cudaStream_t st);
+// The conductors around a target: every rect of its layer but the target itself
+// (layer index of each) that comes within `reach` of the target rect; n < 0
+// when no reach has few enough of them.  Points near the target look their
+// nearest other conductor up here.
+constexpr int kNeighbours = 64;
+struct Neighbours {
+    int n;
+    double reach;
+    float4 rects[kNeighbours];
+    int32_t ids[kNeighbours];
+};
+frw_status launch_neighbours(const DevLayout &L, double4 target_rect, int target_id, Neighbours *out, cudaStream_t st);
+frw_status launch_features(const DevLayout &L, double4 target_rect, int target_id, const Neighbours *nb,
+                           const double4 *rec, int64_t n, __nv_bfloat16 *xb, float *xf, cudaStream_t st);
 // The MLP kernels: tcgen05 / TMEM tiles of 128 rows (cv_umma.cu, the
 // default) or mma.sync tiles of 16 rows (cv.cu); frw_mlp_set_kernels picks.
 // status: device word, kStDeviceWait set when a tcgen05 completion wait
@@ -68,13 +80,13 @@ frw_status launch_reduce_sum_tc(const float *part, int nb, float *grad, cudaStre
 int device_sm_count();
 frw_status launch_adam(const Net &n, float *grad, float *m, float *v, int *step, float lr, cudaStream_t st);
 // exact mean E[f] over every (grid start, first-hop bin) pair, accumulated into *sum
-frw_status launch_quad_mean(const DevLayout &L, double4 target_rect, int target_id, const double4 *gauss, uint32_t Q,
-                            const double *pi_exact, const double *wx, const double *wy, double eps,
+frw_status launch_quad_mean(const DevLayout &L, double4 target_rect, int target_id, const Neighbours *nb,
+                            const double4 *gauss, uint32_t Q, const double *pi_exact, const double *wx, const double *wy, double eps,
                             bool exact_perimeter, const Net &net, double *sum,
                             float *phi_out /*nullable: Q*200 phi values, item q*200+i*/, uint32_t *status,
                             cudaStream_t st);
-frw_status launch_quad_mean_tc(const DevLayout &L, double4 trect, int tid, const double4 *gauss, const double4 *sqs,
-                               const int *sides, uint32_t Q, const double *pi_exact, const double *wx,
+frw_status launch_quad_mean_tc(const DevLayout &L, double4 trect, int tid, const Neighbours *nb,
+                               const double4 *gauss, const double4 *sqs, const int *sides, uint32_t Q, const double *pi_exact, const double *wx,
                                const double *wy, double eps, bool exact, const Net &net, double *sum, float *phi_out,
                                uint32_t *status, int sms, cudaStream_t st);
 // per walk record (end, weight factor c, q*200+i1 or -1): the sums of

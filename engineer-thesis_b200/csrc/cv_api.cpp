@@ -223,6 +223,7 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
         Buf B(st);
         int64_t *d_end;
         double4 *d_rec;
+        cv::Neighbours *d_near;
         __nv_bfloat16 *d_x;
         float *d_y, *d_wt, *d_grad, *d_m, *d_v, *d_part = nullptr;
         double *d_wsum, *d_loss;
@@ -233,6 +234,7 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
         cudaError_t e = cudaSuccess;
         if (e == cudaSuccess) e = B.get(&d_end, N * 8);
         if (e == cudaSuccess) e = B.get(&d_rec, N * 32);
+        if (e == cudaSuccess) e = B.get(&d_near, sizeof(cv::Neighbours));
         if (e == cudaSuccess) e = B.get(&d_x, N * 32);
         if (e == cudaSuccess) e = B.get(&d_y, N * 4);
         if (e == cudaSuccess) e = B.get(&d_wt, N * 4);
@@ -257,7 +259,8 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
         if (rc) return fail(rc);
         const double *r = v.rects + 4 * target;
         const double4 trect = make_double4(r[0], r[1], r[2], r[3]);
-        rc = cv::launch_features(v.dl, trect, (int)target, d_rec, N, d_x, nullptr, st);
+        rc = cv::launch_neighbours(v.dl, trect, (int)target, d_near, st);
+        if (!rc) rc = cv::launch_features(v.dl, trect, (int)target, d_near, d_rec, N, d_x, nullptr, st);
         if (!rc) {
             cudaMemsetAsync(d_wsum, 0, 8, st);
             rc = cv::launch_targets(d_end, d_rec, N, (int)target, d_y, d_wt, d_wsum, st);
@@ -318,11 +321,13 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
         const uint32_t Q = walk_opts->start_grid;
         const int64_t nq = (int64_t)Q * FRW_NSAMPLE;
         double4 *d_gauss, *d_tgt;
+        cv::Neighbours *d_near;
         double *d_pi, *d_mu;
         uint32_t *d_status;
         cudaError_t e = cudaSuccess;
         if (e == cudaSuccess) e = B.get(&d_gauss, 32);
         if (e == cudaSuccess) e = B.get(&d_tgt, 32);
+        if (e == cudaSuccess) e = B.get(&d_near, sizeof(cv::Neighbours));
         if (e == cudaSuccess) e = B.get(&d_pi, FRW_NSAMPLE * 8);
         if (e == cudaSuccess) e = B.get(&d_mu, 8);
         if (e == cudaSuccess) e = B.get(&d_status, 4);
@@ -341,8 +346,9 @@ frw_status frw_cv_train(const frw_layout *layout, int64_t target, const frw_opts
             e = cudaMallocAsync(&M->phi, (size_t)nq * sizeof(float), st);
             if (e != cudaSuccess) return fail(cuda_fail(e, "frw_cv_train: phi table"));
         }
+        if (!rc) rc = cv::launch_neighbours(v.dl, trect, (int)target, d_near, st);
         if (!rc)
-            rc = cv::launch_quad_mean(v.dl, trect, (int)target, d_gauss, Q, d_pi, tables + FRW_NSAMPLE + 1,
+            rc = cv::launch_quad_mean(v.dl, trect, (int)target, d_near, d_gauss, Q, d_pi, tables + FRW_NSAMPLE + 1,
                                       tables + 2 * FRW_NSAMPLE + 1, walk_opts->permittivity,
                                       walk_opts->exact_perimeter != 0, M->net, d_mu, M->phi, d_status, st);
         if (rc) return fail(rc);
@@ -566,12 +572,16 @@ frw_status frw_cv_features(const frw_layout *layout, int64_t target, const doubl
     cudaStream_t st = nullptr;
     Buf B(st);
     double4 *d_rec;
+    cv::Neighbours *d_near;
     float *d_f;
     FRW_CK(B.get(&d_rec, n * 32));
     FRW_CK(B.get(&d_f, n * 64));
+    FRW_CK(B.get(&d_near, sizeof(cv::Neighbours)));
     FRW_CK(cudaMemcpyAsync(d_rec, rec4, n * 32, cudaMemcpyHostToDevice, st));
     const double *r = v.rects + 4 * target;
-    rc = cv::launch_features(v.dl, make_double4(r[0], r[1], r[2], r[3]), (int)target, d_rec, n, nullptr, d_f, st);
+    const double4 trect = make_double4(r[0], r[1], r[2], r[3]);
+    rc = cv::launch_neighbours(v.dl, trect, (int)target, d_near, st);
+    if (!rc) rc = cv::launch_features(v.dl, trect, (int)target, d_near, d_rec, n, nullptr, d_f, st);
     if (rc) return rc;
     return read_back(out, d_f, n * 64, st, "frw_cv_features");
 }

@@ -352,7 +352,8 @@ __global__ void __launch_bounds__(kThreads) k_forward_tc(const float *__restrict
 // 128 feature rows go through forward_tile, and sum += weight * phi in FP64;
 // phi of every item is kept for the walks' look-up.
 __global__ void __launch_bounds__(kThreads) k_quad_mean_tc(
-    DevLayout L, double4 trect, int target_id, const double4 *__restrict__ gauss, const double4 *__restrict__ sqs,
+    DevLayout L, double4 trect, int target_id, const Neighbours *__restrict__ nb,
+    const double4 *__restrict__ gauss, const double4 *__restrict__ sqs,
     const int *__restrict__ sides, uint32_t Q, const double *__restrict__ pi_exact, const double *__restrict__ wx,
     const double *__restrict__ wy, double eps, bool exact, const float *__restrict__ p,
     const __nv_bfloat16 *__restrict__ w1, const __nv_bfloat16 *__restrict__ w2, double *sum,
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) k_quad_mean_tc(
             wgt = c * pi_exact[i] / (double)Q;
             edge_feats(x1, y1, trect.x, trect.y, trect.z, trect.w, a0, f);
             float4 o;
-            if (nearest_other(L, x1, y1, target_id, o)) {
+            if (nearest_other(L, trect, nb, x1, y1, target_id, o)) {
                 edge_feats(x1, y1, o.x, o.y, o.z, o.w, a0, f + 8);
             } else {
 #pragma unroll
@@ -757,14 +758,14 @@ frw_status launch_reduce_sum_tc(const float *part, int nb, float *grad, cudaStre
     return FRW_OK;
 }
 
-frw_status launch_quad_mean_tc(const DevLayout &L, double4 trect, int tid, const double4 *gauss, const double4 *sqs,
-                               const int *sides, uint32_t Q, const double *pi_exact, const double *wx,
+frw_status launch_quad_mean_tc(const DevLayout &L, double4 trect, int tid, const Neighbours *nb,
+                               const double4 *gauss, const double4 *sqs, const int *sides, uint32_t Q, const double *pi_exact, const double *wx,
                                const double *wy, double eps, bool exact, const Net &net, double *sum, float *phi_out,
                                uint32_t *status, int sms, cudaStream_t st) {
     FRW_CK(cudaFuncSetAttribute(k_quad_mean_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdMap::Smem));
     const int64_t tiles = ((int64_t)Q * FRW_NSAMPLE + kThreads - 1) / kThreads;
     const int blocks = (int)std::min<int64_t>(tiles, FwdMap::PerSm * (int64_t)sms);
-    k_quad_mean_tc<<<blocks, kThreads, FwdMap::Smem, st>>>(L, trect, tid, gauss, sqs, sides, Q, pi_exact, wx, wy, eps, exact,
+    k_quad_mean_tc<<<blocks, kThreads, FwdMap::Smem, st>>>(L, trect, tid, nb, gauss, sqs, sides, Q, pi_exact, wx, wy, eps, exact,
                                                     net.p, net.w1, net.w2, sum, phi_out, status);
     FRW_CK(cudaGetLastError());
     return FRW_OK;

@@ -86,3 +86,29 @@ def test_walks_near_the_bounds(k, margin):
                     assert np.array_equal(x, y)
                 escaped += int((end == -1).sum())
     assert escaped > 0
+
+
+@pytest.mark.parametrize("cells_per_rect", [0.2, 1.0, 16.0, 400.0, 20000.0])
+@pytest.mark.parametrize("kind", ["alone", "pair", "ring", "nested", "columns", "layer"])
+def test_nearest_other_conductor(kind, cells_per_rect):
+    """The nearest conductor other than the target, in the control variate's
+    features: in the lists of the cells around the point, near or at the
+    bounds' cells, several rings away, beyond them (the tree) or nowhere."""
+    b = np.array([0.0, 0.0, 400.0, 400.0])
+    r = {"alone": np.array([[200.0, 200, 210, 210]]),
+         "pair": np.array([[3.0, 3, 8, 8], [380.0, 390, 390, 397]]),
+         "ring": row_of(33),
+         "nested": np.array([[100.0, 100, 200, 200], [120.0, 120, 140, 140], [90.0, 90, 210, 210]]),
+         "columns": np.array([[x, y, x + 10, y + 10] for x in range(20, 380, 30) for y in range(20, 380, 30)], float),
+         "layer": frw.generate_layout(5, 16, 400.0).astype(np.float64)}[kind]
+    rng = np.random.default_rng(len(r))
+    t = r[0]
+    p = np.concatenate([rng.uniform(0, 400, (600, 2)), rng.uniform(t[:2] - 3, t[2:] + 3, (600, 2)),
+                        np.round(rng.uniform(0, 400, (300, 2)))]).clip(0, 400)
+    rec = np.zeros((len(p), 4))
+    rec[:, :2] = p
+    rec[:, 2] = rng.choice([1.0, 2.5, 7.0], len(p))
+    with frw.Layout.from_rects(r, b) as L:
+        L.set_cells(cells_per_rect)
+        got = L.cv_features(0, rec)
+    assert np.array_equal(got, O.cv_features(r, 0, rec))
