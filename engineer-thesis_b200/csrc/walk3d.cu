@@ -651,15 +651,18 @@ __device__ __forceinline__ void land(const Walk3Params &P, const double *s_offs,
         j = r - i * P.n;
     }
     const double hi_ = __dmul_rn(h, s_offs[i]), hj = __dmul_rn(h, s_offs[j]);
-    const double x = W.px, y = W.py, z = W.pz;
-    switch (k) {
-    case 0: W.px = __dadd_rn(x, hi_); W.py = __dadd_rn(y, hj); W.pz = __dsub_rn(z, h); break;
-    case 1: W.px = __dadd_rn(x, h); W.py = __dadd_rn(y, hi_); W.pz = __dadd_rn(z, hj); break;
-    case 2: W.px = __dsub_rn(x, hj); W.py = __dadd_rn(y, h); W.pz = __dadd_rn(z, hi_); break;
-    case 3: W.px = __dsub_rn(x, hi_); W.py = __dsub_rn(y, hj); W.pz = __dadd_rn(z, h); break;
-    case 4: W.px = __dsub_rn(x, h); W.py = __dsub_rn(y, hi_); W.pz = __dsub_rn(z, hj); break;
-    default: W.px = __dadd_rn(x, hj); W.py = __dsub_rn(y, h); W.pz = __dsub_rn(z, hi_); break;
-    }
+    // faces k and k + 3 are each other's negatives; x + (-d) rounds exactly as
+    // x - d, so the six faces are one addition per coordinate of selected
+    // offsets: lanes land on all of them, and a branch each ran one by one
+    // (10^7 walks on 10^4 boxes 3.46 -> 3.30 ms)
+    const int sign = k >= 3 ? (int)0x80000000 : 0, m = k >= 3 ? k - 3 : k;
+    const double dx = m == 0 ? hi_ : (m == 1 ? h : -hj);
+    const double dy = m == 0 ? hj : (m == 1 ? hi_ : h);
+    const double dz = m == 0 ? -h : (m == 1 ? hj : hi_);
+    auto signed_by = [&](double d) { return __hiloint2double(__double2hiint(d) ^ sign, __double2loint(d)); };
+    W.px = __dadd_rn(W.px, signed_by(dx));
+    W.py = __dadd_rn(W.py, signed_by(dy));
+    W.pz = __dadd_rn(W.pz, signed_by(dz));
 }
 
 // kMulti: a batch of targets of one layout (jobs); every lane keeps its
