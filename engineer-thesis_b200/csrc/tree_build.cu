@@ -180,32 +180,36 @@ struct Frontier {
     int32_t *node, *level, *start, *end;
 };
 
-__device__ __forceinline__ int lower_digit(const uint32_t *keys, int s, int e, int shift, uint32_t d) {
-    // first index in [s, e) whose digit at `shift` is >= d (digits are sorted there)
-    int lo = s, hi = e;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (((keys[mid] >> shift) & 3u) < d) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
+// The four children's key ranges [b[c], b[c + 1]): the first index in [s, e)
+// whose digit at this level is >= 1, 2, 3 (digits are sorted there).  The three
+// binary searches run side by side: each is a chain of loads, and one after
+// another they were most of a level (see k_split_level).
 __device__ __forceinline__ void child_bounds(const uint32_t *keys, int level, int s, int e, int b[5]) {
     b[0] = s;
     b[4] = e;
     if (level < 16) {
-        int shift = 30 - 2 * level;
-        for (int d = 1; d < 4; d++) b[d] = lower_digit(keys, s, e, shift, (uint32_t)d);
+        const int shift = 30 - 2 * level;
+        int lo[3] = {s, s, s}, hi[3] = {e, e, e};
+        while (lo[0] < hi[0] || lo[1] < hi[1] || lo[2] < hi[2]) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const int mid = (lo[d] + hi[d]) >> 1;
+                // (a finished search reads nothing and stays: mid == lo == hi)
+                const bool below = lo[d] < hi[d] && ((__ldg(keys + mid) >> shift) & 3u) <= (uint32_t)d;
+                if (below) lo[d] = mid + 1;
+                else hi[d] = mid;
+            }
+        }
+        for (int d = 0; d < 3; d++) b[d + 1] = lo[d];
     } else {  // identical keys: split by index
         for (int d = 1; d < 4; d++) b[d] = s + (int)((int64_t)(e - s) * d / 4);
     }
 }
 
-// Per frontier entry: (new nodes << 32) | (next-frontier entries).
+// Per frontier entry: (new nodes << 32) | (next-frontier entries), and its
+// children's bounds.
 __device__ __forceinline__ unsigned long long split_count_one(const uint32_t *keys, const Frontier &fr, int i,
-                                                              int leaf_max) {
-    int b[5];
+                                                              int leaf_max, int b[5]) {
     int level = fr.level[i];
     child_bounds(keys, level, fr.start[i], fr.end[i], b);
     int nonempty = 0, big = 0;
@@ -220,12 +224,10 @@ __device__ __forceinline__ unsigned long long split_count_one(const uint32_t *ke
 
 // Per frontier entry with its scanned offsets: the node's child references
 // and the next frontier's entries.
-__device__ __forceinline__ void split_emit_one(const uint32_t *keys, const Frontier &fr, int i, int leaf_max,
+__device__ __forceinline__ void split_emit_one(const int b[5], const Frontier &fr, int i, int leaf_max,
                                                unsigned long long o, int node_base, int4 *nref,
                                                const Frontier &nx) {
-    int b[5];
     int level = fr.level[i], node = fr.node[i];
-    child_bounds(keys, level, fr.start[i], fr.end[i], b);
     int nonempty = 0, big = 0;
     for (int c = 0; c < 4; c++) {
         int m = b[c + 1] - b[c];
@@ -277,7 +279,8 @@ __device__ __forceinline__ unsigned long long block_scan_u64(unsigned long long 
 // more levels than a layout is deep without asking: an empty frontier is a
 // launch that ends at once, where reading each level's size back (and scanning
 // it in one block) cost 70 us per level, 0.7 of the 1.1 ms of a 10^6-rect
-// tree.  Node ids within a level follow the blocks' order; every query's
+// tree.  What is left of a level is its searches' chain of loads (20 -> 11 us
+// with the three side by side and once per level).  Node ids within a level follow the blocks' order; every query's
 // traversal order is the children's, so its result does not depend on them.
 __global__ void __launch_bounds__(1024) k_split_level(const uint32_t *__restrict__ keys, Frontier fr, Frontier nx,
                                                      int level, int leaf_max, SplitState *S,
@@ -289,7 +292,8 @@ __global__ void __launch_bounds__(1024) k_split_level(const uint32_t *__restrict
     for (int k = 0; k < level; k++) base += S->made[k];
     for (int b0 = blockIdx.x * 1024; b0 < nfr; b0 += gridDim.x * 1024) {
         const int i = b0 + threadIdx.x;
-        const unsigned long long v = i < nfr ? split_count_one(keys, fr, i, leaf_max) : 0ull;
+        int cb[5];
+        const unsigned long long v = i < nfr ? split_count_one(keys, fr, i, leaf_max, cb) : 0ull;
         unsigned long long total;
         const unsigned long long e = block_scan_u64(v, wt, total);
         if (threadIdx.x == 0) {
@@ -300,7 +304,7 @@ __global__ void __launch_bounds__(1024) k_split_level(const uint32_t *__restrict
         if (i < nfr) {
             const unsigned long long at =
                 (((e >> 32) + (unsigned)s_node) << 32) | ((e & 0xFFFFFFFFull) + (unsigned)s_next);
-            split_emit_one(keys, fr, i, leaf_max, at, base, nref, nx);
+            split_emit_one(cb, fr, i, leaf_max, at, base, nref, nx);
         }
         __syncthreads();
     }
@@ -405,7 +409,8 @@ __global__ void __launch_bounds__(1024) k_build_small(const uint32_t *__restrict
             if (t == 0) s_over = 1;
             break;
         }
-        for (int i = t; i < nfr; i += 1024) cnt[i] = split_count_one(keys, fa, i, leaf_max);
+        int cb[5];
+        for (int i = t; i < nfr; i += 1024) cnt[i] = split_count_one(keys, fa, i, leaf_max, cb);
         __syncthreads();
         unsigned long long carry = 0;
         for (int b0 = 0; b0 < nfr; b0 += 1024) {
@@ -418,7 +423,11 @@ __global__ void __launch_bounds__(1024) k_build_small(const uint32_t *__restrict
         }
         __syncthreads();
         const int node_base = s_nodes;
-        for (int i = t; i < nfr; i += 1024) split_emit_one(keys, fa, i, leaf_max, cnt[i], node_base, nref, fb);
+        for (int i = t; i < nfr; i += 1024) {
+            // (a thread that counted one entry has its bounds)
+            if (nfr > 1024) child_bounds(keys, fa.level[i], fa.start[i], fa.end[i], cb);
+            split_emit_one(cb, fa, i, leaf_max, cnt[i], node_base, nref, fb);
+        }
         __syncthreads();
         if (t == 0) {
             const int new_nodes = (int)(carry >> 32);
