@@ -33,8 +33,8 @@ namespace {
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-// rect indices staged per coarse cell by the count pass
-constexpr int kStage = 4;
+// rects that a thread of the coarse pass keeps
+constexpr int kStage = 12;
 
 // Visits the tree's rects touching the closed box B, in tree order, until
 // visit() returns false.  Returns false when the traversal stack overflowed
@@ -73,7 +73,7 @@ struct Grid {
     int nx, ny;
 };
 
-// The count pass visits the cells in tiles of 8 x 4, one tile per warp, so
+// The passes visit the cells in tiles of 8 x 4, one tile per warp, so
 // that a warp's tree traversals start from neighbouring points and take
 // similar paths: thread t gets cell (tile_x * 8 + t % 8, tile_y * 4 + t % 32
 // / 8) of tile t / 32, or -1 past the grid's edge.
@@ -124,66 +124,84 @@ __device__ __forceinline__ double2 centre_of(const Grid &G, int64_t c) {
     return make_double2(G.gx0 + ix * G.side + 0.5 * G.side, G.gy0 + iy * G.side + 0.5 * G.side);
 }
 
-// Coarse cells, from the tree (L without cells).  Per cell: its list length,
-// or -1 (in cells[c].y) when it exceeds cap or the enumeration was incomplete;
-// cnt[c] = entries to reserve; rad[c] its radius (one margin above the
-// Lipschitz bound r_cell <= r_coarse) and stage[kStage c ..] the tree positions
-// of its first kStage rects, for the fill pass.
-__global__ void k_cell_count(DevLayout L, Grid G, int cap, int64_t *__restrict__ cnt, int2 *__restrict__ cells,
-                             double *__restrict__ rad, int32_t *__restrict__ stage, int64_t nthreads) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nthreads) return;
-    const int64_t c = tiled_cell(G, t);
-    if (c < 0) return;
-    const double2 p = centre_of(G, c);
-    Cands C;
-    int hit;
-    double best;
-    clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
-    const double r = radius_of(L, G, best) + G.margin;
-    double B[4];
-    grown_box(G, c, r, B);
-    rad[c] = r;
-    int n = 0;
-    int32_t *sg = stage + kStage * c;
-    const bool complete = touching(L, B, [&](int k, float4) {
-        if (n < kStage) sg[n] = k;
-        return ++n <= cap;
-    });
-    const bool ok = complete && n <= cap;
-    cnt[c] = ok ? n : 0;
-    cells[c] = make_int2(0, ok ? n : -1);
+// The place of this thread's `want` entries in a buffer with cursor *tot: a
+// scan over the block, one atomic.  Every thread of the block calls it.
+__device__ __forceinline__ unsigned long long block_offset(unsigned want, unsigned long long *tot,
+                                                           unsigned *s_warp, unsigned long long *s_base, int warps) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned x = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[w] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned s = 0;
+        for (int k = 0; k < warps; k++) s += s_warp[k];
+        *s_base = s ? atomicAdd(tot, (unsigned long long)s) : 0ull;
+    }
+    __syncthreads();
+    unsigned long long at = *s_base + (x - want);
+    for (int k = 0; k < w; k++) at += s_warp[k];
+    return at;
 }
 
-// Writes the coarse lists that did not overflow: the staged rects, or for
-// longer lists the enumeration of the same grown box again (its order is
-// deterministic, so it meets the same rects as the count).
-__global__ void k_cell_fill(DevLayout L, Grid G, const int64_t *__restrict__ start, const double *__restrict__ rad,
-                            const int32_t *__restrict__ stage, int2 *__restrict__ cells, float4 *__restrict__ crects,
-                            int32_t *__restrict__ cids, int64_t ncells) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncells) return;
-    const int m = cells[c].y;
-    if (m < 0) return;
-    const int64_t s = start[c];
-    if (m <= kStage) {
-        for (int i = 0; i < m; i++) {
-            const int k = stage[kStage * c + i];
-            crects[s + i] = __ldg(L.rects + k);
-            cids[s + i] = __ldg(L.ids + k);
+// Coarse cells, from the tree (L without cells): every rect touching the cell
+// grown by its radius, one margin above the Lipschitz bound r_cell <= r_coarse;
+// (0, -1) when there are more than cap or the enumeration was incomplete.  The
+// lists go to the shared buffers at offsets from a global cursor (tot), a block
+// scan and one atomic per block; past `room` entries they are counted, not
+// written (the caller runs the pass again with room for tot).  A thread keeps
+// its first kStage rects in shared memory and enumerates longer lists again.
+// Bound by the traversals' chains of loads, two per cell; a count pass, a scan
+// and a fill pass with 48 bytes per cell between them took 0.69 ms for 10^6
+// rects' 10^6 coarse cells, this one 0.55.
+constexpr int kCoarseThreads = 128;
+__global__ void __launch_bounds__(kCoarseThreads)
+    k_coarse_lists(DevLayout L, Grid G, int cap, int2 *__restrict__ cells, float4 *__restrict__ crects,
+                   int32_t *__restrict__ cids, int64_t room, unsigned long long *tot, int64_t nthreads) {
+    __shared__ int32_t s_stage[kStage][kCoarseThreads];
+    __shared__ unsigned s_warp[kCoarseThreads / 32];
+    __shared__ unsigned long long s_base;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t c = t < nthreads ? tiled_cell(G, t) : -1;
+    double B[4] = {0, 0, 0, 0};
+    int n = 0;
+    bool ok = false;
+    if (c >= 0) {
+        const double2 p = centre_of(G, c);
+        Cands C;
+        int hit;
+        double best;
+        clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
+        grown_box(G, c, radius_of(L, G, best) + G.margin, B);
+        const bool complete = touching(L, B, [&](int k, float4) {
+            if (n < kStage) s_stage[n][threadIdx.x] = k;
+            return ++n <= cap;
+        });
+        ok = complete && n <= cap;
+    }
+    const unsigned want = ok ? (unsigned)n : 0u;
+    const unsigned long long at = block_offset(want, tot, s_warp, &s_base, kCoarseThreads / 32);
+    if (c < 0) return;
+    cells[c] = make_int2(ok ? (int)at : 0, ok ? n : -1);
+    if (!want || at + want > (unsigned long long)room) return;
+    if (n <= kStage) {
+        for (int i = 0; i < n; i++) {
+            const int k = s_stage[i][threadIdx.x];
+            crects[at + i] = __ldg(L.rects + k);
+            cids[at + i] = __ldg(L.ids + k);
         }
     } else {
-        double B[4];
-        grown_box(G, c, rad[c], B);
-        int n = 0;
+        int m = 0;
         touching(L, B, [&](int k, float4 r) {
-            if (n >= m) return false;
-            crects[s + n] = r;
-            cids[s + n] = __ldg(L.ids + k);
-            return ++n < m;
+            crects[at + m] = r;
+            cids[at + m] = __ldg(L.ids + k);
+            return ++m < n;
         });
     }
-    cells[c] = make_int2((int)s, m);
 }
 
 constexpr int kRecordThreads = 256;
@@ -207,7 +225,6 @@ __global__ void __launch_bounds__(kRecordThreads)
     __shared__ unsigned s_warp[kRecordThreads / 32];
     __shared__ unsigned long long s_base;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t c = t < nthreads ? tiled_cell(G, t) : -1;
     int2 ce = make_int2(0, -1);
     double B[4] = {0, 0, 0, 0};
@@ -271,29 +288,16 @@ __global__ void __launch_bounds__(kRecordThreads)
             rid[k] = -1;
         }
     }
-    // offsets of the longer lists: a warp scan, the warps' totals, one atomic
+    // totals, and the offsets of the longer lists
     const unsigned want = !tree && n >= kCellSlots + (near ? 0 : 1) ? (unsigned)n : 0u;
-    unsigned x = want;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[w] = x;
     const unsigned kept = __reduce_add_sync(0xFFFFFFFFu, tree ? 0u : (unsigned)n);
     const unsigned trees = __popc(__ballot_sync(0xFFFFFFFFu, tree));
-    if (lane == 0 && kept) atomicAdd(tot + 1, (unsigned long long)kept);
-    if (lane == 0 && trees) atomicAdd(tot + 2, (unsigned long long)trees);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned s = 0;
-        for (int k = 0; k < kRecordThreads / 32; k++) s += s_warp[k];
-        s_base = s ? atomicAdd(tot, (unsigned long long)s) : 0ull;
+    if ((threadIdx.x & 31) == 0) {
+        if (kept) atomicAdd(tot + 1, (unsigned long long)kept);
+        if (trees) atomicAdd(tot + 2, (unsigned long long)trees);
     }
-    __syncthreads();
+    const unsigned long long at = block_offset(want, tot, s_warp, &s_base, kRecordThreads / 32);
     if (c < 0 || !(want || tree || near)) return;
-    unsigned long long at = s_base + (x - want);
-    for (int k = 0; k < w; k++) at += s_warp[k];
     float4 *rec = cells + kCellSlots * c;
     rec[kCellSlots - 1] = make_float4(kListRect, __int_as_float(tree ? 0 : (int)at), __int_as_float(tree ? kTreeCell : n), 0.f);
     if (!want || at + want > (unsigned long long)room) return;
@@ -432,35 +436,33 @@ struct BuildBufs {
     }
 };
 
-// Count -> scan -> fill of coarse cells over the tree of L.
+// Coarse cells over the tree of L.
 frw_status build_coarse(const DevLayout &L, const Grid &G, cudaStream_t st, BuildBufs &B, CoarseLists *K) {
-    const int64_t ncells = (int64_t)G.nx * G.ny, tiles = scan_i64_tiles(ncells), nt = tiled_threads(G.nx, G.ny);
-    int64_t *cnt, *start, *sums, *grand;
-    double *rad;
-    int32_t *stage;
+    const int64_t ncells = (int64_t)G.nx * G.ny, nt = tiled_threads(G.nx, G.ny);
     frw_status rc;
+    unsigned long long *tot;
     if ((rc = B.get(&K->cells, (size_t)ncells * sizeof(int2), "malloc coarse cells"))) return rc;
-    if ((rc = B.get(&cnt, (size_t)ncells * 8, "malloc cell counts"))) return rc;
-    if ((rc = B.get(&start, (size_t)ncells * 8, "malloc cell starts"))) return rc;
-    if ((rc = B.get(&rad, (size_t)ncells * 8, "malloc cell radii (build)"))) return rc;
-    if ((rc = B.get(&stage, (size_t)ncells * kStage * 4, "malloc staged rects"))) return rc;
-    if ((rc = B.get(&sums, (size_t)tiles * 8, "malloc tile sums"))) return rc;
-    if ((rc = B.get(&grand, 8, "malloc total"))) return rc;
-    k_cell_count<<<(unsigned)((nt + 127) / 128), 128, 0, st>>>(L, G, kCoarseCap, cnt, K->cells, rad, stage, nt);
-    launch_scan_i64(cnt, ncells, start, sums, grand, st);
-    FRW_CK(cudaGetLastError());
-    int64_t total = 0;
-    if ((rc = read_back(&total, grand, 8, st, "build_cells: coarse list total"))) return rc;
-    if (total > INT32_MAX) {
-        set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
-        return FRW_E_ARG;
+    if ((rc = B.get(&tot, 8, "malloc total"))) return rc;
+    // room for 12 rects a cell (8 to 9 at the benchmark's densities); denser layouts take a second pass
+    int64_t room = std::max<int64_t>(12 * ncells, 4096);
+    for (int pass = 0; pass < 2; pass++) {
+        if ((rc = B.get(&K->rects, (size_t)room * 16, "malloc coarse rects"))) return rc;
+        if ((rc = B.get(&K->ids, (size_t)room * 4, "malloc coarse ids"))) return rc;
+        FRW_CK(cudaMemsetAsync(tot, 0, 8, st));
+        k_coarse_lists<<<(unsigned)((nt + kCoarseThreads - 1) / kCoarseThreads), kCoarseThreads, 0, st>>>(
+            L, G, kCoarseCap, K->cells, K->rects, K->ids, room, tot, nt);
+        FRW_CK(cudaGetLastError());
+        unsigned long long total = 0;
+        if ((rc = read_back(&total, tot, 8, st, "build_cells: coarse list total"))) return rc;
+        if (total > INT32_MAX) {
+            set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
+            return FRW_E_ARG;
+        }
+        if ((int64_t)total <= room) break;
+        B.drop(K->rects);
+        B.drop(K->ids);
+        room = (int64_t)total;
     }
-    if ((rc = B.get(&K->rects, (size_t)total * 16, "malloc coarse rects"))) return rc;
-    if ((rc = B.get(&K->ids, (size_t)total * 4, "malloc coarse ids"))) return rc;
-    if (total > 0)
-        k_cell_fill<<<(unsigned)((ncells + 127) / 128), 128, 0, st>>>(L, G, start, rad, stage, K->cells, K->rects,
-                                                                      K->ids, ncells);
-    FRW_CK(cudaGetLastError());
     K->nx = G.nx;
     K->ny = G.ny;
     return FRW_OK;
