@@ -40,12 +40,13 @@ constexpr int kWalkThreads = 256;
 // half of the lanes that need one; one hop 6% and three hops 6% slower than
 // two: their draws are needed by some lane in every hop).
 constexpr int kHopsPerRound = 4;
-// Resident blocks of 256 per SM: 5 at 48 registers for unweighted walks, 4 at 64
-// for weighted (uniform start) ones, whose state is larger (1e7 capacitance
-// walks on 10^4 rects 2.06 -> 1.98 ms, 1e7 control-variate walks 2.12 -> 2.02,
-// 28 batched layouts 2.18 -> 1.94 against 5; unweighted walks equal either way).
-constexpr int kWalkMinBlocksW = 4;
-constexpr int kWalkMinBlocks = 5;
+// Resident blocks of 256 per SM: 4, at 64 registers.  The walk is bound by
+// instruction issue once 32 warps are resident, and 48 registers for a fifth
+// block spill (1e7 capacitance walks on 10^4 rects 2.06 -> 1.98 ms, 28 batched
+// layouts 2.18 -> 1.94 against 5; Green-function starts 2e7 walks on 10^6 rects
+// 5.09 -> 5.03, 3e6 on 10^4 0.86 -> 0.81, 10^5 0.21 -> 0.20; 3 blocks and 6 are
+// slower).
+constexpr int kWalkMinBlocks = 4;
 constexpr int kWarpsPerBlock = kWalkThreads / 32;
 constexpr int kTabSlots = 32;  // per warp
 constexpr unsigned long long kEmptyKey = ~0ull;
@@ -265,7 +266,7 @@ __device__ __forceinline__ void tab_round(const WalkParams &P, Slot *tab, int la
 // (P.tree_points); without it cell records answer every point and the tree's
 // code is compiled out of the kernel.
 template <bool kMulti, bool kRec, bool kUniform, bool kCV = false, bool kTies = false>
-__global__ void __launch_bounds__(kWalkThreads, kUniform ? kWalkMinBlocksW : kWalkMinBlocks)
+__global__ void __launch_bounds__(kWalkThreads, kWalkMinBlocks)
     k_walk(const WalkParams P) {
     __shared__ double s_intg[FRW_NSAMPLE + 1];
     __shared__ double s_wx[FRW_NSAMPLE], s_wy[FRW_NSAMPLE];
@@ -482,8 +483,8 @@ __global__ void __launch_bounds__(kWalkThreads, kUniform ? kWalkMinBlocksW : kWa
                     // > 0 (each difference is > 0 exactly when p is on that side)
                     const double bd = dmin(dmin(px - L.bx0, L.bx1 - px), dmin(py - L.by0, L.by1 - py));
                     in = bd > 0.0;
-                    // the tree traversal is a call in the 48-register kernel, whose
-                    // code it would otherwise crowd
+                    // the tree traversal is a call unless the walks are weighted (a
+                    // call was slower for those)
                     if (in) st |= query_point<true, !kUniform>(L, px, py, sq, hit, bd);
                 } else {
                     in = query_record<true>(L, px, py, sq, hit, st);
