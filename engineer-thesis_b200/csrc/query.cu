@@ -17,13 +17,16 @@ __device__ __forceinline__ void store_square(double4 *p, const double s[4]) {
 // many exact ties can reach the whole-tree replay (compiled out otherwise).
 // Random points: bound by the reads of their records, in L2 for 10^4 rects (a
 // warp's 32 records are 64 separate 32-byte reads; 16-byte reads doubled the
-// L1 lookups, 1e7 points 0.304 -> 0.228 ms; 12 blocks per SM against 10:
-// 0.240, 16 spill: 0.242) and in HBM for 10^6 (150 bytes read and 40 written
-// per point, 0.545 -> 0.453 ms).  Records fetched ahead of their points --
-// through shared memory by asynchronous copies, or the coordinates alone in a
-// persistent grid -- were slower (1.05 and 0.59 ms).
+// L1 lookups, 1e7 points 0.304 -> 0.228 ms) and in HBM for 10^6 (150 bytes read
+// and 40 written per point, 0.545 -> 0.432 ms by now).  24 blocks of 64 per SM:
+// a block ends with its slowest lane, so small ones refill the SM sooner (0.216
+// -> 0.208 and 0.436 -> 0.432 ms against 12 of 128; 10 of 128: 0.229; 28 of 64
+// spill: 0.267).  Records fetched ahead of their points -- through shared memory
+// by asynchronous copies, or the coordinates alone in a persistent grid -- were
+// slower (1.05 and 0.59 ms).
+constexpr int kQueryThreads = 64;
 template <bool kTies>
-__global__ void __launch_bounds__(128, kTies ? 8 : 12)
+__global__ void __launch_bounds__(kQueryThreads, kTies ? 16 : 24)
     k_query(DevLayout L, const double2 *__restrict__ pts, int64_t n, double4 *__restrict__ sq,
             int64_t *__restrict__ hit, uint32_t *status) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -151,7 +154,7 @@ frw_status launch_gauss_jobs(const WalkJob *d_jobs, const double *d_targets, int
 frw_status launch_query(const DevLayout &L, const double *d_pts, int64_t n, double *d_sq, int64_t *d_hit,
                         uint32_t *d_status, cudaStream_t stream) {
     if (n <= 0) return FRW_OK;
-    const int T = 128;
+    const int T = kQueryThreads;
     const unsigned g = (unsigned)((n + T - 1) / T);
     if (L.tree_points)
         k_query<true><<<g, T, 0, stream>>>(L, (const double2 *)d_pts, n, (double4 *)d_sq, d_hit, d_status);
