@@ -49,7 +49,7 @@ WORKLOAD = dict(workload="frw-c3-1e6-rects-1e8-walks", rects=1_000_000, domain=1
                 start="Green-CDF bin on the Gaussian perimeter (reference RandomWalk)",
                 estimator="per-conductor end counts, fraction ending elsewhere (reference getAvgPathLen)",
                 layout_seed=0xF4A7 + 3,
-                l2="working set above the 126 MB L2 (cell lists 0.8 GB); the GPU arm also writes 256 MiB "
+                l2="working set above the 126 MB L2 (cell records 1.4 GB); the GPU arm also writes 256 MiB "
                    "between steps")
 METRIC = "walks/s (plain FRW, 10^6-rect layout, 1e8 walks/step, reference surface, start and estimator)"
 PROFILE = os.path.join(ROOT, "profiles", "walk_kernel_c3.md")

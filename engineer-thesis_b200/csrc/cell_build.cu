@@ -15,8 +15,8 @@
 // writes its record (up to kCellSlots rects in place; a longer list goes to
 // the shared list buffer at an offset from a global cursor, one atomic per
 // block).  Large grids first build coarse cells (4 x 4 cells each) from the
-// tree -- count, scan, fill -- and answer each cell's clearance and enumeration
-// from its coarse cell's list.  Cells with more than max_per_cell rects are
+// tree, in one pass of the same kind, and answer each cell's clearance and
+// enumeration from its coarse cell's list.  Cells with more than max_per_cell rects are
 // left to the tree.
 #include <cuda_runtime.h>
 

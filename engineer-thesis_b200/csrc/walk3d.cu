@@ -13,14 +13,14 @@
 //     boxes that its cells can need into shared memory and every lane finds
 //     its cell's nearest box and list among them;
 //   * the walk kernel is persistent (SM count x resident blocks); a warp
-//     claims walks in chunks from one global counter and refills each idle
-//     lane before every hop, so lanes stay busy while walks of very different
+//     claims walks in chunks from one global counter and refills its idle
+//     lanes every four hops, so lanes stay busy while walks of very different
 //     lengths finish;
 //   * random numbers are Philox4x32-10 words keyed by (seed) with counter
 //     (t / 4, walk, stream): the trajectory of a walk depends only on its
 //     index, so the CPU oracle replays every walk bit for bit;
 //   * the landing bin comes from a 2^14-entry guide in shared memory and the
-//     32-bit CDF thresholds (L1-resident) -- one or two compares;
+//     32-bit CDF thresholds (shared memory, or L1) -- one or two compares;
 //   * FP64 geometry with explicitly rounded operations (no contraction):
 //     exactly the oracle's arithmetic.
 #include <math.h>
