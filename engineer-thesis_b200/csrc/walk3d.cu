@@ -249,28 +249,36 @@ __device__ void sort_entries(float4 *e, int64_t m) {
 // runs the pass again with room for tot[0]).
 // Why: a thread per cell walked its own bins -- 7 of 32 lanes active -- twice,
 // counting and then filling, and ordered 32-byte entries in place in global
-// memory: 10^5 boxes 5.3 -> 1.5 ms (bins and read-backs included).
+// memory: 10^5 boxes 5.3 -> 1.5 ms (bins and read-backs included; 1.3 by now).
 constexpr int kBrickX = 4, kBrickY = 4, kBrickZ = 2;
 constexpr int kBrickWarps = 2;     // per block
-constexpr int kBrickCand = 256;    // candidates a warp keeps (about 75 at 8 cells per box)
-constexpr int kBrickKeys = 40;     // list entries a lane orders in shared memory
+constexpr int kBrickKeys = 32;     // list entries a lane orders in shared memory
+// Candidates a warp keeps.  The finest level's bricks have about 75, and its
+// warps are as many as their shared memory allows: 128 there against 256, and 32
+// keys against 40.  Coarser levels have few cells, far from every box, each with
+// many candidates in reach: 256 (128: 1e5 boxes no faster than before; 512 and
+// 768 as 256).  Grids of 1e5 boxes 1.46 -> 1.31 ms, of 3e5 (two passes) 8.9
+// -> 7.3.
+constexpr int kFineCand = 128, kCoarseCand = 256;
 
+template <int kBrickCand>
 struct BrickShared {
     float4 box[2 * kBrickCand];  // (x0, y0, z0, index), (x1, y1, z1, -)
     float key[kBrickKeys][32];   // per lane: rounded-down distances, in order
     uint16_t at[kBrickKeys][32]; // and their candidates
 };
 
+template <int kBrickCand>
 __global__ void __launch_bounds__(kBrickWarps * 32)
     k3_cell_lists(const float *__restrict__ boxes, Grid3 G, const int64_t *__restrict__ bstart,
                   const int32_t *__restrict__ items, const uint8_t *__restrict__ need, uint8_t *__restrict__ need_up,
                   int upnx, int upny, uint2 *__restrict__ cells, float4 *__restrict__ lists, int64_t room,
                   unsigned long long *__restrict__ tot, int64_t nbricks) {
-    __shared__ BrickShared s_brick[kBrickWarps];
+    __shared__ BrickShared<kBrickCand> s_brick[kBrickWarps];
     const int lane = threadIdx.x & 31;
     const int64_t brick = (int64_t)blockIdx.x * kBrickWarps + (threadIdx.x >> 5);
     if (brick >= nbricks) return;
-    BrickShared &S = s_brick[threadIdx.x >> 5];
+    BrickShared<kBrickCand> &S = s_brick[threadIdx.x >> 5];
     const int bnx = (G.n[0] + kBrickX - 1) / kBrickX, bny = (G.n[1] + kBrickY - 1) / kBrickY;
     const int c0[3] = {(int)(brick % bnx) * kBrickX, (int)(brick / bnx % bny) * kBrickY,
                        (int)(brick / ((int64_t)bnx * bny)) * kBrickZ};
@@ -938,15 +946,18 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         // the fill uses bcnt as its cursor: start it at the bin starts
         if (!ck(cudaMemcpyAsync(bcnt, bstart, cb, cudaMemcpyDeviceToDevice, st), "cursor")) break;
         k3_bin_fill<<<nb, 256, 0, st>>>(d_boxes, n, G, (unsigned long long *)bcnt, items);
-        // room for the lists of the default density (7 to 8 entries per cell);
+        // room for the lists of the default density (7 to 9.2 entries per cell, the
+        // more the larger the layout: 3e5 boxes passed 9 and
+        // took a second pass, 7.3 -> 4.4 ms);
         // longer ones take a second pass, and a buffer mostly unused a copy
-        int64_t room = 9 * ncells + 4096;
+        int64_t room = 10 * ncells + 4096;
         unsigned long long h[3] = {0, 0, 0};
         for (int pass = 0; pass < 2; pass++) {
             // (a query may read one entry past a list)
             if (!ck(cudaMallocAsync(&out->lists, (size_t)(room + 1) * 32, st), "malloc lists")) break;
             if (!ck(cudaMemsetAsync(tot, 0, 24, st), "memset")) break;
-            k3_cell_lists<<<(unsigned)((nbricks + kBrickWarps - 1) / kBrickWarps), kBrickWarps * 32, 0, st>>>(
+            const auto kernel = need ? k3_cell_lists<kCoarseCand> : k3_cell_lists<kFineCand>;
+            kernel<<<(unsigned)((nbricks + kBrickWarps - 1) / kBrickWarps), kBrickWarps * 32, 0, st>>>(
                 d_boxes, G, bstart, items, need, need_up, upnx, upny, out->cells, out->lists, room, tot, nbricks);
             if (!ck(cudaGetLastError(), "cell lists")) break;
             if ((rc = read_back(h, tot, 24, st, "build_grid3: list total"))) break;
