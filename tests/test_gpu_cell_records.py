@@ -112,3 +112,20 @@ def test_nearest_other_conductor(kind, cells_per_rect):
         L.set_cells(cells_per_rect)
         got = L.cv_features(0, rec)
     assert np.array_equal(got, O.cv_features(r, 0, rec))
+
+
+@pytest.mark.parametrize("width", [60, 200, 900, 4000])
+def test_coarse_lists_longer_than_their_room(width):
+    """Long thin rects on a grid built through coarse cells: few rects per
+    coarse cell, more than there is room for at first (the pass runs again),
+    and more than a coarse cell keeps (its cells take them from the tree)."""
+    n = 4200
+    y = np.arange(n) * 4.0
+    r = np.stack([np.zeros(n), y, np.full(n, float(width)), y + 2], 1)
+    b = np.array([-50.0, -50.0, width + 50.0, 4.0 * n + 50.0])
+    rng = np.random.default_rng(width)
+    p = np.concatenate([rng.uniform(b[:2], b[2:], (4000, 2)), np.round(rng.uniform(b[:2], b[2:], (1000, 2)))])
+    ref, hit_ref = O.Grid(r, b).query_batch(p)
+    with frw.Layout.from_rects(r, b) as L:
+        sq, hit = L.query(p)
+    assert np.array_equal(sq, ref) and np.array_equal(hit, hit_ref)
