@@ -328,12 +328,13 @@ def _row_arrays(cap: int):
     """conductor, hits, cap, cap_se, sum_w and sum_w2 of a result, `cap` zeros
     each.  Large ones are demand-zero pages: a result fills the front of rows
     that are as long as its layout, and clearing 48 MB for the few hundred
-    conductors of a 10^6-rect run takes longer than its walks."""
+    conductors of a 10^6-rect run takes longer than its walks.  Each column has
+    private pages of its own: a forked child's writes stay its own, and a
+    column kept alone keeps no other's pages."""
     types = (np.int64, np.uint64, np.float64, np.float64, np.float64, np.float64)
     if cap < 1 << 15:
         return [np.zeros(cap, t) for t in types]
-    pages = mmap.mmap(-1, 48 * cap)
-    return [np.frombuffer(pages, t, cap, 8 * cap * k) for k, t in enumerate(types)]
+    return [np.frombuffer(mmap.mmap(-1, 8 * cap, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), t) for t in types]
 
 
 def version() -> str:
