@@ -179,30 +179,59 @@ __device__ __forceinline__ void st_group_raw(unsigned char *buf, int g, int r, u
     *reinterpret_cast<uint4 *>(buf + g * kGrp + (r >> 3) * 128 + (r & 7) * 16) = q;
 }
 
+// Loads of what the kernels of an overlapped chain write for each other (the
+// weights, the moments, the partial sums).  A kernel of the chain may start
+// while the kernel that writes them still runs, so they are no constants of the
+// launch: strong loads, past L1, in volatile statements, which stay behind
+// wait_previous(), itself one.
+__device__ __forceinline__ float ld_chain(const float *p) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_chain(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
+}
+
 // The weights as B operands (K-major core-matrix grids) and the FP32 vectors.
+// All of a thread's loads are issued before its first store.
 template <class M>
 __device__ void load_weights(unsigned char *sm, const float *p, const __nv_bfloat16 *w1, const __nv_bfloat16 *w2,
                              const __nv_bfloat16 *w2t, bool need_w2t) {
-    const uint4 *w1q = reinterpret_cast<const uint4 *>(w1);
+    constexpr int kW2Each = 64 * 8 / kThreads;
+    static_assert(kThreads == 64 * 2, "a thread per chunk of W1");
+    const int t = threadIdx.x, j = t & (kHid - 1);
     const uint4 *w2q = reinterpret_cast<const uint4 *>(w2);
     const uint4 *w2tq = reinterpret_cast<const uint4 *>(w2t);
-    for (int c = threadIdx.x; c < 64 * 2; c += blockDim.x) {  // W1[n][k]: 64 rows x 2 chunks of 8
-        const int n = c >> 1, kc = c & 1;
-        *reinterpret_cast<uint4 *>(sm + M::W1 + (n >> 3) * 256 + kc * 128 + (n & 7) * 16) = w1q[c];
+    const uint4 q1 = ld_chain(reinterpret_cast<const uint4 *>(w1) + t);
+    uint4 q2[kW2Each], q2t[kW2Each];
+#pragma unroll
+    for (int k = 0; k < kW2Each; k++) {
+        q2[k] = ld_chain(w2q + k * kThreads + t);
+        if (need_w2t) q2t[k] = ld_chain(w2tq + k * kThreads + t);
     }
-    for (int c = threadIdx.x; c < 64 * 8; c += blockDim.x) {  // W2[n][k] and W2T[n][k]: 64 rows x 8 chunks
-        const int n = c >> 3, kc = c & 7;
+    const float b1 = ld_chain(p + oB1 + j), b2 = ld_chain(p + oB2 + j), w3 = ld_chain(p + oW3 + j),
+                b3 = ld_chain(p + oB3);
+    // W1[n][k]: 64 rows x 2 chunks of 8
+    *reinterpret_cast<uint4 *>(sm + M::W1 + (t >> 4) * 256 + (t & 1) * 128 + ((t >> 1) & 7) * 16) = q1;
+#pragma unroll
+    for (int k = 0; k < kW2Each; k++) {  // W2[n][k] and W2T[n][k]: 64 rows x 8 chunks
+        const int c = k * kThreads + t, n = c >> 3, kc = c & 7;
         const uint32_t off = (n >> 3) * 1024 + kc * 128 + (n & 7) * 16;
-        *reinterpret_cast<uint4 *>(sm + M::W2 + off) = w2q[c];
-        if (need_w2t) *reinterpret_cast<uint4 *>(sm + M::W2T + off) = w2tq[c];
+        *reinterpret_cast<uint4 *>(sm + M::W2 + off) = q2[k];
+        if (need_w2t) *reinterpret_cast<uint4 *>(sm + M::W2T + off) = q2t[k];
     }
     float *par = reinterpret_cast<float *>(sm + M::Par);
-    for (int i = threadIdx.x; i < kHid; i += blockDim.x) {
-        par[i] = p[oB1 + i];
-        par[64 + i] = p[oB2 + i];
-        par[128 + i] = p[oW3 + i];
+    if (t < kHid) {
+        par[t] = b1;
+        par[64 + t] = b2;
+        par[128 + t] = w3;
     }
-    if (threadIdx.x == 0) par[192] = p[oB3];
+    if (t == 0) par[192] = b3;
 }
 
 // ---------------------------------------------------------------- forward
@@ -414,13 +443,13 @@ __global__ void __launch_bounds__(kThreads) k_quad_mean_tc(
 
 // ---------------------------------------------------------------- training
 // grad += d/dparams sum_r wt_r (f(x_r) - y_r)^2 * inv_wsum; loss += the sum.
-__global__ void __launch_bounds__(kThreads) k_train_grad_tc(const float *__restrict__ p,
-                                                            const __nv_bfloat16 *__restrict__ w1,
-                                                            const __nv_bfloat16 *__restrict__ w2,
-                                                            const __nv_bfloat16 *__restrict__ w2t,
+// (p, w1, w2, w2t: written by the update before while this kernel may already
+// run, hence without __restrict__, see ld_chain)
+__global__ void __launch_bounds__(kThreads) k_train_grad_tc(const float *p, const __nv_bfloat16 *w1,
+                                                            const __nv_bfloat16 *w2, const __nv_bfloat16 *w2t,
                                                             const __nv_bfloat16 *__restrict__ x,
                                                             const float *__restrict__ y, const float *__restrict__ wt,
-                                                            int64_t rows, float inv_wsum, float *__restrict__ part,
+                                                            int64_t rows, float inv_wsum, float *part,
                                                             double *__restrict__ loss_out, uint32_t *status) {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -638,7 +667,9 @@ __global__ void __launch_bounds__(kThreads) k_train_grad_tc(const float *__restr
 // training run of 124 steps of 32,768 rows 4.03 -> 3.16 ms with this, the
 // overlapped launches and SiLU's derivative kept from its forward pass.)
 constexpr int kReduceThreads = 256, kReduceParams = 32, kReduceSlots = 256;
-__device__ __forceinline__ float sum_slots(const float *__restrict__ part, int nb, int i) {
+// part: written by the kernel before, see ld_chain; a slot or parameter past the
+// last is read as the last one and not used.
+__device__ __forceinline__ float sum_slots(const float *part, int nb, int i) {
     __shared__ float s[kReduceSlots][kReduceParams];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int kWarps = kReduceThreads / 32, kEach = kReduceSlots / kWarps;
@@ -648,8 +679,8 @@ __device__ __forceinline__ float sum_slots(const float *__restrict__ part, int n
         float v[kEach];
 #pragma unroll
         for (int k = 0; k < kEach; k++) {
-            const int b = k * kWarps + w;
-            v[k] = b < n && i < kParams ? __ldcg(part + (size_t)(b0 + b) * kPartStride + i) : 0.f;
+            const int b = min(k * kWarps + w, n - 1);
+            v[k] = ld_chain(part + (size_t)(b0 + b) * kPartStride + min(i, kParams - 1));
         }
 #pragma unroll
         for (int k = 0; k < kEach; k++) s[k * kWarps + w][lane] = v[k];
@@ -661,21 +692,23 @@ __device__ __forceinline__ float sum_slots(const float *__restrict__ part, int n
     }
     return g;
 }
-__global__ void __launch_bounds__(kReduceThreads) k_reduce_adam(const float *__restrict__ part, int nb, float *__restrict__ p, float *__restrict__ m,
-                              float *__restrict__ v, int t, float lr, __nv_bfloat16 *__restrict__ w1,
-                              __nv_bfloat16 *__restrict__ w2, __nv_bfloat16 *__restrict__ w2t) {
+__global__ void __launch_bounds__(kReduceThreads) k_reduce_adam(const float *part, int nb, float *p, float *m, float *v,
+                                                                int t, float lr, __nv_bfloat16 *w1, __nv_bfloat16 *w2,
+                                                                __nv_bfloat16 *w2t) {
     const int i = blockIdx.x * kReduceParams + (threadIdx.x & 31);
     let_next_start();
     wait_previous();
     const float gi = sum_slots(part, nb, i);
     if (threadIdx.x >= 32 || i >= kParams) return;
     const float b1 = 0.9f, b2 = 0.999f;
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    // (the update before this one wrote them; it may still run when this one starts)
+    const float m0 = ld_chain(m + i), v0 = ld_chain(v + i), p0 = ld_chain(p + i);
+    const float mi = b1 * m0 + (1.f - b1) * gi;
+    const float vi = b2 * v0 + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
     const float mh = mi / (1.f - powf(b1, (float)t)), vh = vi / (1.f - powf(b2, (float)t));
-    const float pi = p[i] - lr * mh / (sqrtf(vh) + 1e-8f);
+    const float pi = p0 - lr * mh / (sqrtf(vh) + 1e-8f);
     p[i] = pi;
     if (i < oB1) w1[i] = __float2bfloat16_rn(pi);
     else if (i >= oW2 && i < oB2) {
@@ -686,7 +719,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce_adam(const float *__r
 }
 
 // grad += the CTAs' partial sums, in CTA order.
-__global__ void __launch_bounds__(kReduceThreads) k_reduce_sum(const float *__restrict__ part, int nb, float *__restrict__ grad) {
+__global__ void __launch_bounds__(kReduceThreads) k_reduce_sum(const float *part, int nb, float *__restrict__ grad) {
     const int i = blockIdx.x * kReduceParams + (threadIdx.x & 31);
     const float g = sum_slots(part, nb, i);
     if (threadIdx.x < 32 && i < kParams) grad[i] += g;
