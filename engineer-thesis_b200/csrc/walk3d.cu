@@ -1199,7 +1199,10 @@ frw_status launch_walk3_as(Walk3Params P, int sms, int bps, cudaStream_t st) {
     const bool big = bps == 0 && thr <= kW3ThrBytes && P.walks >= warps * 32;
     P.chunk = P.walks < warps * 128 ? 32 : 128;
     if (big) {
-        cudaError_t e = cudaFuncSetAttribute(k_walk3<kMulti, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)thr);
+        // the largest table's size, whichever table this launch has: the attribute
+        // is the kernel's, and another host thread's launch may have a longer one
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_walk3<kMulti, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kW3ThrBytes);
         if (e != cudaSuccess) return cuda_fail(e, "k_walk3: shared memory");
         k_walk3<kMulti, true><<<sms, kW3BigThreads, thr, st>>>(P);
     } else {
