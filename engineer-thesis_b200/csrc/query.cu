@@ -24,9 +24,16 @@ __device__ __forceinline__ void store_square(double4 *p, const double s[4]) {
 // spill: 0.267).  Records fetched ahead of their points -- through shared memory
 // by asynchronous copies, or the coordinates alone in a persistent grid -- were
 // slower (1.05 and 0.59 ms).
+// With the tree's code (kTies) a point's chain of nodes is what its warp waits
+// for: 24 blocks as well, at 40 registers (4e6 points on 10^4 rects 1.318 ->
+// 1.215 ms, on 3e5 1.49 -> 1.33, partly overflowed cells 0.70 -> 0.59; 16 blocks
+// 1.375, 1.54 and 0.69), but the spills lengthen the chain, so points that are
+// all resident at once anyway take 16 at 64 registers (1000 points on 10^4
+// rects 55 us a call against 65).
 constexpr int kQueryThreads = 64;
-template <bool kTies>
-__global__ void __launch_bounds__(kQueryThreads, kTies ? 16 : 24)
+constexpr int64_t kTreeWave = 148 * 16 * kQueryThreads;
+template <bool kTies, int kBlocks>
+__global__ void __launch_bounds__(kQueryThreads, kBlocks)
     k_query(DevLayout L, const double2 *__restrict__ pts, int64_t n, double4 *__restrict__ sq,
             int64_t *__restrict__ hit, uint32_t *status) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -156,10 +163,8 @@ frw_status launch_query(const DevLayout &L, const double *d_pts, int64_t n, doub
     if (n <= 0) return FRW_OK;
     const int T = kQueryThreads;
     const unsigned g = (unsigned)((n + T - 1) / T);
-    if (L.tree_points)
-        k_query<true><<<g, T, 0, stream>>>(L, (const double2 *)d_pts, n, (double4 *)d_sq, d_hit, d_status);
-    else
-        k_query<false><<<g, T, 0, stream>>>(L, (const double2 *)d_pts, n, (double4 *)d_sq, d_hit, d_status);
+    const auto kernel = !L.tree_points ? k_query<false, 24> : n <= kTreeWave ? k_query<true, 16> : k_query<true, 24>;
+    kernel<<<g, T, 0, stream>>>(L, (const double2 *)d_pts, n, (double4 *)d_sq, d_hit, d_status);
     FRW_CK(cudaGetLastError());
     return FRW_OK;
 }
