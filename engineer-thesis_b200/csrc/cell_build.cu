@@ -14,7 +14,8 @@
 // the clearance at each cell centre, enumerates the rects of its grown box and
 // writes its record (up to kCellSlots rects in place; a longer list goes to
 // the shared list buffer at an offset from a global cursor, one atomic per
-// block).  Large grids first build coarse cells (4 x 4 cells each) from the
+// block; lists past the buffer's first room are written by a second pass over
+// their cells).  Large grids first build coarse cells (4 x 4 cells each) from the
 // tree, in one pass of the same kind, and answer each cell's clearance and
 // enumeration from its coarse cell's list.  Cells with more than max_per_cell rects are
 // left to the tree.
@@ -211,12 +212,34 @@ constexpr int kRecordThreads = 256;
 // holds every rect the clearance at the centre and the grown box can need --
 // unless it overflowed; else from the tree.  tot[0]: list entries reserved,
 // tot[1]: entries of all cells (records included), tot[2]: cells left to the
-// tree.  Lists past `room` entries are counted, not written (the caller runs
-// the pass again with room for tot[0]).
+// tree.  Lists past `room` entries have their place and radius in the record but
+// are not written (k_fill_lists does).
 // Bound by its writes (84 bytes a cell: 16e6 cells at 10^6 rects take 0.2 ms
 // at the copy rate) and the FP64 gaps of the coarse lists (about 6 rects,
 // twice); it replaces a count pass, a scan and a fill pass with 84 bytes of
 // counts, radii and staged positions per cell between them.
+
+// Visits the rects touching B in a fixed order: those of the coarse cell ce, or
+// the tree's.  visit(layer index, rect) says whether to go on; false when the
+// enumeration was incomplete.
+template <bool kCoarse, typename F>
+__device__ __forceinline__ bool each_touching(const DevLayout &L, const CoarseLists &K, int2 ce, const double B[4],
+                                              F &&visit) {
+    if (!kCoarse || ce.y < 0) return touching(L, B, [&](int k, float4 r) { return visit(L.ids + k, r); });
+    const FloatBox fb = float_box(B);
+    for (int k = ce.x; k < ce.x + ce.y; k++) {
+        const float4 r = __ldg(K.rects + k);
+        if (fb.touches(r) && !visit(K.ids + k, r)) break;
+    }
+    return true;
+}
+
+// The coarse cell covering cell c.
+__device__ __forceinline__ int2 coarse_of(const CoarseLists &K, const Grid &G, int factor, int64_t c) {
+    const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
+    return __ldg(K.cells + (int64_t)(iy / factor) * K.nx + ix / factor);
+}
+
 template <bool kCoarse>
 __global__ void __launch_bounds__(kRecordThreads)
     k_cell_records(DevLayout L, CoarseLists K, Grid G, int factor, int cap, float4 *__restrict__ cells,
@@ -230,25 +253,14 @@ __global__ void __launch_bounds__(kRecordThreads)
     double B[4] = {0, 0, 0, 0};
     int n = 0;
     bool tree = false, near = false;
-    // visits the rects touching B in a fixed order
-    auto each = [&](auto &&visit) {
-        if (!kCoarse || ce.y < 0) return touching(L, B, [&](int k, float4 r) { return visit(L.ids + k, r); });
-        const FloatBox fb = float_box(B);
-        for (int k = ce.x; k < ce.x + ce.y; k++) {
-            const float4 r = __ldg(K.rects + k);
-            if (fb.touches(r) && !visit(K.ids + k, r)) break;
-        }
-        return true;
-    };
+    float radius = 0.f;
+    auto each = [&](auto &&visit) { return each_touching<kCoarse>(L, K, ce, B, visit); };
     if (c >= 0) {
         const double2 p = centre_of(G, c);
         // clearance at the centre: of the bounds, and of the rects (at least)
         const double bd = bounds_distance(L, p.x, p.y);
         double gap = 1e300;
-        if (kCoarse) {
-            const int ix = (int)(c % G.nx), iy = (int)(c / G.nx);
-            ce = __ldg(K.cells + (int64_t)(iy / factor) * K.nx + ix / factor);
-        }
+        if (kCoarse) ce = coarse_of(K, G, factor, c);
         if (kCoarse && ce.y >= 0) {
             // the clearance in FP32 on a split centre (two roundings of the gap's
             // own size), raised past its error: a radius a hair larger is as good
@@ -268,11 +280,12 @@ __global__ void __launch_bounds__(kRecordThreads)
         // both clearances change by at most the distance moved: no point of a
         // cell that is not `near` has the bounds as near as its nearest rect or 3
         near = !(bd - 0.5 * G.side > dmax(gap + 0.5 * G.side, 3.0) + 2.0 * L.delta + G.margin);
-        const double r = radius_of(L, G, dmin(bd, gap));
-        grown_box(G, c, r, B);
+        // (raised to FP32: the record keeps it)
+        radius = __double2float_ru(radius_of(L, G, dmin(bd, gap)));
+        grown_box(G, c, (double)radius, B);
         // a point of the cell lies within margin/2 of it whatever the rounding of
-        // its cell index, so every rect within r - margin of the point is listed
-        crad[c] = __double2float_rd(r - G.margin);
+        // its cell index, so every rect within radius - margin of the point is listed
+        crad[c] = __double2float_rd((double)radius - G.margin);
         float4 *rec = cells + kCellSlots * c;
         int32_t *rid = reinterpret_cast<int32_t *>(cellids + c);
         const bool complete = each([&](const int32_t *id, float4 q) {
@@ -299,7 +312,8 @@ __global__ void __launch_bounds__(kRecordThreads)
     const unsigned long long at = block_offset(want, tot, s_warp, &s_base, kRecordThreads / 32);
     if (c < 0 || !(want || tree || near)) return;
     float4 *rec = cells + kCellSlots * c;
-    rec[kCellSlots - 1] = make_float4(kListRect, __int_as_float(tree ? 0 : (int)at), __int_as_float(tree ? kTreeCell : n), 0.f);
+    rec[kCellSlots - 1] = make_float4(kListRect, __int_as_float(tree ? 0 : (int)at), __int_as_float(tree ? kTreeCell : n),
+                                      radius);
     if (!want || at + want > (unsigned long long)room) return;
     int m = 0;
     each([&](const int32_t *id, float4 q) {
@@ -307,6 +321,33 @@ __global__ void __launch_bounds__(kRecordThreads)
         cids[at + m] = __ldg(id);
         return ++m < n;
     });
+}
+
+// The lists that k_cell_records had no room for: cells whose list ends past
+// `room` take their rects again, by the radius in their record, and write them
+// at their place (the lists before it are copied).  Only these cells do any
+// work: running the whole pass again made layouts of long lists slower to build
+// than a count and a fill pass had been (clustered 3e5 rects 2.25 -> 1.96 ms
+// with this, 300,000 at one cell per rect 0.64 -> 0.52).
+template <bool kCoarse>
+__global__ void __launch_bounds__(kRecordThreads)
+    k_fill_lists(DevLayout L, CoarseLists K, Grid G, int factor, const float4 *__restrict__ cells,
+                 float4 *__restrict__ crects, int32_t *__restrict__ cids, int64_t room, int64_t nthreads) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t c = t < nthreads ? tiled_cell(G, t) : -1;
+    if (c < 0) return;
+    const float4 last = cells[kCellSlots * c + kCellSlots - 1];
+    const int at = __float_as_int(last.y), n = __float_as_int(last.z);
+    if (!(last.x > kFarRect) || n < kCellSlots || (int64_t)at + n <= room) return;
+    double B[4];
+    grown_box(G, c, (double)last.w, B);
+    int m = 0;
+    each_touching<kCoarse>(L, K, kCoarse ? coarse_of(K, G, factor, c) : make_int2(0, -1), B,
+                           [&](const int32_t *id, float4 q) {
+                               crects[at + m] = q;
+                               cids[at + m] = __ldg(id);
+                               return ++m < n;
+                           });
 }
 
 // Exclusive scan of int64 values: tile sums, a one-block scan of the tile
@@ -487,40 +528,36 @@ frw_status build_records(const DevLayout &L, const CoarseLists &K, const Grid &G
     if ((rc = B.get(&C.crad, (size_t)ncells * sizeof(float), "malloc cell radii"))) return rc;
     if ((rc = B.get(&tot, 24, "malloc totals"))) return rc;
     // half an entry of list room per cell holds the lists of the benchmark's
-    // densities (0.16 at 16 cells per rect); denser ones take a second pass
-    int64_t room = std::max<int64_t>(ncells / 2, 4096);
+    // densities (0.16 at 16 cells per rect); k_fill_lists writes those past it
+    const int64_t room = std::max<int64_t>(ncells / 2, 4096);
     unsigned long long h[3] = {0, 0, 0};
     float4 *rects = nullptr;
     int32_t *ids = nullptr;
-    for (int pass = 0; pass < 2; pass++) {
-        if ((rc = B.get(&rects, (size_t)room * 16, "malloc cell rects"))) return rc;
-        if ((rc = B.get(&ids, (size_t)room * 4, "malloc cell ids"))) return rc;
-        FRW_CK(cudaMemsetAsync(tot, 0, 24, st));
-        const unsigned blocks = (unsigned)((nt + kRecordThreads - 1) / kRecordThreads);
-        if (K.cells)
-            k_cell_records<true><<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, cap, C.cells, C.cellids, C.crad,
-                                                                    rects, ids, room, tot, nt);
-        else
-            k_cell_records<false><<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, cap, C.cells, C.cellids,
-                                                                     C.crad, rects, ids, room, tot, nt);
-        FRW_CK(cudaGetLastError());
-        if ((rc = read_back(h, tot, 24, st, "build_cells: list total"))) return rc;
-        if (h[0] >= (unsigned long long)kMaxListEntries) {
-            set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
-            return FRW_E_ARG;
-        }
-        if ((int64_t)h[0] <= room) break;
-        B.drop(rects);
-        B.drop(ids);
-        room = (int64_t)h[0];
+    if ((rc = B.get(&rects, (size_t)room * 16, "malloc cell rects"))) return rc;
+    if ((rc = B.get(&ids, (size_t)room * 4, "malloc cell ids"))) return rc;
+    FRW_CK(cudaMemsetAsync(tot, 0, 24, st));
+    const unsigned blocks = (unsigned)((nt + kRecordThreads - 1) / kRecordThreads);
+    const auto records = K.cells ? k_cell_records<true> : k_cell_records<false>;
+    records<<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, cap, C.cells, C.cellids, C.crad, rects, ids, room, tot,
+                                               nt);
+    FRW_CK(cudaGetLastError());
+    if ((rc = read_back(h, tot, 24, st, "build_cells: list total"))) return rc;
+    if (h[0] >= (unsigned long long)kMaxListEntries) {
+        set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
+        return FRW_E_ARG;
     }
     // the lists in buffers of their size
-    const int64_t total = (int64_t)h[0];
+    const int64_t total = (int64_t)h[0], written = std::min(total, room);
     if ((rc = B.get(&C.crects, (size_t)total * 16, "malloc cell rects"))) return rc;
     if ((rc = B.get(&C.cids, (size_t)total * 4, "malloc cell ids"))) return rc;
-    if (total) {
-        FRW_CK(cudaMemcpyAsync(C.crects, rects, (size_t)total * 16, cudaMemcpyDeviceToDevice, st));
-        FRW_CK(cudaMemcpyAsync(C.cids, ids, (size_t)total * 4, cudaMemcpyDeviceToDevice, st));
+    if (written) {
+        FRW_CK(cudaMemcpyAsync(C.crects, rects, (size_t)written * 16, cudaMemcpyDeviceToDevice, st));
+        FRW_CK(cudaMemcpyAsync(C.cids, ids, (size_t)written * 4, cudaMemcpyDeviceToDevice, st));
+    }
+    if (total > room) {
+        const auto fill = K.cells ? k_fill_lists<true> : k_fill_lists<false>;
+        fill<<<blocks, kRecordThreads, 0, st>>>(L, K, G, kCoarse, C.cells, C.crects, C.cids, room, nt);
+        FRW_CK(cudaGetLastError());
     }
     C.entries = (int64_t)h[1];
     C.overflow = (int64_t)h[2];

@@ -39,7 +39,7 @@ FRW_HD int leaf_count(int ref) { return (-2 - ref) & kLeafCountMax; }
 // (kFarRect in every coordinate); or, when it lists more than kCellSlots rects
 // or lies near the bounds (where a point's clearance can be the bounds'), its
 // first kCellSlots - 1 rects and a last slot of kListRect and the bits of
-// (first, count, -): all its rects, when there are kCellSlots or more, are
+// (first, count, radius): all its rects, when there are kCellSlots or more, are
 // entries first .. first + count - 1 of the lists; count < 0 when the tree
 // answers the cell's points.  Read as a rect that slot is as far as an unused
 // one (first < kMaxListEntries keeps its bits below kListRect), so the gaps of
