@@ -153,16 +153,17 @@ __device__ __forceinline__ unsigned long long block_offset(unsigned want, unsign
 // grown by its radius, one margin above the Lipschitz bound r_cell <= r_coarse;
 // (0, -1) when there are more than cap or the enumeration was incomplete.  The
 // lists go to the shared buffers at offsets from a global cursor (tot), a block
-// scan and one atomic per block; past `room` entries they are counted, not
-// written (the caller runs the pass again with room for tot).  A thread keeps
-// its first kStage rects in shared memory and enumerates longer lists again.
+// scan and one atomic per block; past `room` entries they have their place and
+// radius but are not written (k_fill_coarse does).  A thread keeps its first
+// kStage rects in shared memory and enumerates longer lists again.
 // Bound by the traversals' chains of loads, two per cell; a count pass, a scan
 // and a fill pass with 48 bytes per cell between them took 0.69 ms for 10^6
 // rects' 10^6 coarse cells, this one 0.55.
 constexpr int kCoarseThreads = 128;
 __global__ void __launch_bounds__(kCoarseThreads)
-    k_coarse_lists(DevLayout L, Grid G, int cap, int2 *__restrict__ cells, float4 *__restrict__ crects,
-                   int32_t *__restrict__ cids, int64_t room, unsigned long long *tot, int64_t nthreads) {
+    k_coarse_lists(DevLayout L, Grid G, int cap, int2 *__restrict__ cells, float *__restrict__ crad,
+                   float4 *__restrict__ crects, int32_t *__restrict__ cids, int64_t room, unsigned long long *tot,
+                   int64_t nthreads) {
     __shared__ int32_t s_stage[kStage][kCoarseThreads];
     __shared__ unsigned s_warp[kCoarseThreads / 32];
     __shared__ unsigned long long s_base;
@@ -177,7 +178,9 @@ __global__ void __launch_bounds__(kCoarseThreads)
         int hit;
         double best;
         clearance(L, p.x, p.y, C, hit, best, bounds_distance(L, p.x, p.y));
-        grown_box(G, c, radius_of(L, G, best) + G.margin, B);
+        const float radius = __double2float_ru(radius_of(L, G, best) + G.margin);
+        crad[c] = radius;
+        grown_box(G, c, (double)radius, B);
         const bool complete = touching(L, B, [&](int k, float4) {
             if (n < kStage) s_stage[n][threadIdx.x] = k;
             return ++n <= cap;
@@ -203,6 +206,28 @@ __global__ void __launch_bounds__(kCoarseThreads)
             return ++m < n;
         });
     }
+}
+
+// The lists that k_coarse_lists had no room for, one traversal each: k_coarse_lists
+// run again, two or three traversals each, made dense layouts slower to build than
+// its count and fill passes had been (3e5 overlapping rects, 16 a coarse cell,
+// 1.95 -> 1.40 ms in all against 1.42).
+__global__ void __launch_bounds__(kCoarseThreads)
+    k_fill_coarse(DevLayout L, Grid G, const int2 *__restrict__ cells, const float *__restrict__ crad,
+                  float4 *__restrict__ crects, int32_t *__restrict__ cids, int64_t room, int64_t nthreads) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t c = t < nthreads ? tiled_cell(G, t) : -1;
+    if (c < 0) return;
+    const int2 ce = cells[c];
+    if (ce.y <= 0 || (int64_t)ce.x + ce.y <= room) return;
+    double B[4];
+    grown_box(G, c, (double)crad[c], B);
+    int m = 0;
+    touching(L, B, [&](int k, float4 r) {
+        crects[ce.x + m] = r;
+        cids[ce.x + m] = __ldg(L.ids + k);
+        return ++m < ce.y;
+    });
 }
 
 constexpr int kRecordThreads = 256;
@@ -326,9 +351,9 @@ __global__ void __launch_bounds__(kRecordThreads)
 // The lists that k_cell_records had no room for: cells whose list ends past
 // `room` take their rects again, by the radius in their record, and write them
 // at their place (the lists before it are copied).  Only these cells do any
-// work: running the whole pass again made layouts of long lists slower to build
-// than a count and a fill pass had been (clustered 3e5 rects 2.25 -> 1.96 ms
-// with this, 300,000 at one cell per rect 0.64 -> 0.52).
+// work: the whole pass run again made layouts of long lists slower to build than
+// a count and a fill pass had been (3e5 clustered rects 3.28 -> 1.96 ms against
+// 2.25, 3e5 rects at one cell each 0.72 -> 0.52 against 0.64).
 template <bool kCoarse>
 __global__ void __launch_bounds__(kRecordThreads)
     k_fill_lists(DevLayout L, CoarseLists K, Grid G, int factor, const float4 *__restrict__ cells,
@@ -481,28 +506,37 @@ struct BuildBufs {
 frw_status build_coarse(const DevLayout &L, const Grid &G, cudaStream_t st, BuildBufs &B, CoarseLists *K) {
     const int64_t ncells = (int64_t)G.nx * G.ny, nt = tiled_threads(G.nx, G.ny);
     frw_status rc;
-    unsigned long long *tot;
+    unsigned long long *tot, total = 0;
+    float *crad;
     if ((rc = B.get(&K->cells, (size_t)ncells * sizeof(int2), "malloc coarse cells"))) return rc;
+    if ((rc = B.get(&crad, (size_t)ncells * sizeof(float), "malloc coarse radii"))) return rc;
     if ((rc = B.get(&tot, 8, "malloc total"))) return rc;
-    // room for 12 rects a cell (8 to 9 at the benchmark's densities); denser layouts take a second pass
-    int64_t room = std::max<int64_t>(12 * ncells, 4096);
-    for (int pass = 0; pass < 2; pass++) {
-        if ((rc = B.get(&K->rects, (size_t)room * 16, "malloc coarse rects"))) return rc;
-        if ((rc = B.get(&K->ids, (size_t)room * 4, "malloc coarse ids"))) return rc;
-        FRW_CK(cudaMemsetAsync(tot, 0, 8, st));
-        k_coarse_lists<<<(unsigned)((nt + kCoarseThreads - 1) / kCoarseThreads), kCoarseThreads, 0, st>>>(
-            L, G, kCoarseCap, K->cells, K->rects, K->ids, room, tot, nt);
+    // room for 12 rects a cell (8 to 9 at the benchmark's densities); k_fill_coarse writes the lists past it
+    const int64_t room = std::max<int64_t>(12 * ncells, 4096);
+    float4 *rects;
+    int32_t *ids;
+    if ((rc = B.get(&rects, (size_t)room * 16, "malloc coarse rects"))) return rc;
+    if ((rc = B.get(&ids, (size_t)room * 4, "malloc coarse ids"))) return rc;
+    FRW_CK(cudaMemsetAsync(tot, 0, 8, st));
+    const unsigned blocks = (unsigned)((nt + kCoarseThreads - 1) / kCoarseThreads);
+    k_coarse_lists<<<blocks, kCoarseThreads, 0, st>>>(L, G, kCoarseCap, K->cells, crad, rects, ids, room, tot, nt);
+    FRW_CK(cudaGetLastError());
+    if ((rc = read_back(&total, tot, 8, st, "build_cells: coarse list total"))) return rc;
+    if (total > INT32_MAX) {
+        set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
+        return FRW_E_ARG;
+    }
+    K->rects = rects;
+    K->ids = ids;
+    if ((int64_t)total > room) {
+        if ((rc = B.get(&K->rects, (size_t)total * 16, "malloc coarse rects"))) return rc;
+        if ((rc = B.get(&K->ids, (size_t)total * 4, "malloc coarse ids"))) return rc;
+        FRW_CK(cudaMemcpyAsync(K->rects, rects, (size_t)room * 16, cudaMemcpyDeviceToDevice, st));
+        FRW_CK(cudaMemcpyAsync(K->ids, ids, (size_t)room * 4, cudaMemcpyDeviceToDevice, st));
+        B.drop(rects);
+        B.drop(ids);
+        k_fill_coarse<<<blocks, kCoarseThreads, 0, st>>>(L, G, K->cells, crad, K->rects, K->ids, room, nt);
         FRW_CK(cudaGetLastError());
-        unsigned long long total = 0;
-        if ((rc = read_back(&total, tot, 8, st, "build_cells: coarse list total"))) return rc;
-        if (total > INT32_MAX) {
-            set_error("build_cells: more than 2^31 list entries; use fewer cells per rect");
-            return FRW_E_ARG;
-        }
-        if ((int64_t)total <= room) break;
-        B.drop(K->rects);
-        B.drop(K->ids);
-        room = (int64_t)total;
     }
     K->nx = G.nx;
     K->ny = G.ny;
