@@ -48,6 +48,7 @@ struct Dev3Layout {
     float fslack;          // absolute part of the FP32 screen's error (nearest3)
     int nx, ny, nz;
     int nup;               // coarser levels
+    int max_list;          // longest list of any level
     const Level3 *up;      // [nup] device array
     uint32_t *status;      // kSt3* bits (device word of the layout)
     double b[6];           // bounds (x0,y0,z0,x1,y1,z1), open

@@ -453,6 +453,35 @@ __global__ void __launch_bounds__(kBrickWarps * 32)
 }
 
 // ---- query -----------------------------------------------------------------
+// A point as floats and their remainders: a gap lo - p = (lo - ph) - pl carries
+// two roundings of its own size and the remainder's (2^-22 of the gap + 2^-46 of
+// the coordinates; lo - ph is exact when the two are close).
+struct Split3 {
+    float xh, yh, zh, xl, yl, zl;
+    __device__ __forceinline__ float gap(const float4 &lo, const float4 &hi) const {
+        const float gx = fmaxf((lo.x - xh) - xl, (xh - hi.x) + xl);
+        const float gy = fmaxf((lo.y - yh) - yl, (yh - hi.y) + yl);
+        const float gz = fmaxf((lo.z - zh) - zl, (zh - hi.z) + zl);
+        return fmaxf(fmaxf(gx, gy), fmaxf(gz, 0.f));
+    }
+    // (a point far outside the bounds has gaps of its own size, so the relative
+    // slack covers its remainder's rounding; one past FP32's range, or NaN, is
+    // left to FP64)
+    __device__ __forceinline__ bool usable() const { return fabsf(xh) + fabsf(yh) + fabsf(zh) < 1e37f; }
+};
+__device__ __forceinline__ Split3 split3(double px, double py, double pz) {
+    Split3 s;
+    s.xh = (float)px;
+    s.yh = (float)py;
+    s.zh = (float)pz;
+    s.xl = (float)__dsub_rn(px, (double)s.xh);
+    s.yl = (float)__dsub_rn(py, (double)s.yh);
+    s.zl = (float)__dsub_rn(pz, (double)s.zh);
+    return s;
+}
+
+// kLong: for layouts with long lists (kLongQuery, kLongWalk), see below.
+template <bool kLong>
 __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double py, double pz, double &best,
                                          int &bid) {
     const int ix = cell_axis(px, L.g0x, L.ginv, L.nx);
@@ -479,57 +508,74 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
         }
     }
     e += 2 * (size_t)cr.x;
-    // The nearest entry in FP32: p as a float and its remainder, so a gap
-    // lo - p = (lo - ph) - pl carries two roundings of its own size and the
-    // remainder's (2^-22 of the gap + 2^-46 of the coordinates; lo - ph is
-    // exact when the two are close).  An entry is skipped when its distance
-    // from the cell centre (hi.w, rounded down) leaves it farther than the best;
-    // later ones are too.  A winner ahead by more than the errors is the FP64
-    // winner, and only its distance is taken in FP64; else (ties, touching
-    // boxes) the list is scanned again in FP64.
-    // Why: an FP64 gap costs conversions and compares, six of each per entry
+    best = INFINITY;
+    bid = 0x7FFFFFFF;
+    // The nearest entry in FP32 on a split point.  An entry is skipped when its
+    // distance from the cell centre (hi.w, rounded down) leaves it farther than
+    // the best; later ones are too.  A winner ahead by more than the errors is
+    // the FP64 winner, and only its distance is taken in FP64.  Where two are
+    // closer (ties, touching boxes), a list is scanned again in FP64; with kLong,
+    // where that costs as much as the first scan and clusters of aligned boxes
+    // seen from afar tie often, the two are compared in FP64 on the spot, so that
+    // the best is the FP64 winner of the entries so far (a block of 4096 aligned
+    // boxes in wide bounds, 3e5 points: 14.6 -> 6.2 ms against 8.1 for one FP64
+    // scan, 3e4 walks 140 -> 91 ms against 156).
+    // Why FP32: an FP64 gap costs conversions and compares, six of each per entry
     // and about 60 instructions, on lists whose longest of a warp sets the
     // pace (3 entries scanned on average, 7.5 by the slowest lane, at 8 cells
     // per box): 1e7 walks on 10^4 boxes 4.29 -> 4.20 ms, 1e7 queries 0.312 ->
     // 0.302 ms, then 4.12 and 0.300 ms with two entries read at a time.
-    const float xh = (float)px, yh = (float)py, zh = (float)pz;
-    const float xl = (float)__dsub_rn(px, (double)xh), yl = (float)__dsub_rn(py, (double)yh),
-                zl = (float)__dsub_rn(pz, (double)zh);
-    const float hqf = __double2float_ru(hq);
-    float b1 = 3.0e38f, b2 = 3.0e38f, lim = 3.0e38f;
-    uint32_t w = 0;
-    auto take = [&](uint32_t k, const float4 &lo, const float4 &hi) {
-        const float gx = fmaxf((lo.x - xh) - xl, (xh - hi.x) + xl);
-        const float gy = fmaxf((lo.y - yh) - yl, (yh - hi.y) + yl);
-        const float gz = fmaxf((lo.z - zh) - zl, (zh - hi.z) + zl);
-        const float g = fmaxf(fmaxf(gx, gy), fmaxf(gz, 0.f));
-        b2 = fminf(b2, fmaxf(g, b1));
-        if (g < b1) {
+    const Split3 S = split3(px, py, pz);
+    if (!kLong || S.usable()) {
+        const float hqf = __double2float_ru(hq);
+        float b1 = 3.0e38f, b2 = 3.0e38f, lim = 3.0e38f;  // b2: the second nearest; kLong: past it clearly farther
+        uint32_t w = 0;
+        bool exact = false;  // kLong: best and bid are the best entry's
+        auto take = [&](uint32_t k, const float4 &lo, const float4 &hi) {
+            const float g = S.gap(lo, hi);
+            if (kLong) {
+                if (g > b2) return;
+                if (g * 1.000001f + L.fslack < b1) {
+                    exact = false;
+                } else {
+                    if (!exact) {
+                        const float4 blo = __ldg(e + 2 * w), bhi = __ldg(e + 2 * w + 1);
+                        best = box_dist_finite(px, py, pz, blo, bhi);
+                        bid = __float_as_int(blo.w);
+                        exact = true;
+                    }
+                    const double d = box_dist_finite(px, py, pz, lo, hi);
+                    const int id = __float_as_int(lo.w);
+                    if (d > best || (d == best && id > bid)) return;
+                    best = d;
+                    bid = id;
+                }
+                b2 = g * 1.000001f + L.fslack;
+            } else {
+                b2 = fminf(b2, fmaxf(g, b1));
+                if (!(g < b1)) return;
+            }
             b1 = g;
             w = k;
             lim = (b1 + hqf) * 1.000002f + L.fslack;
+        };
+        for (uint32_t k = 0; k < cr.y; k += 2) {  // two entries in flight (the lists end in a spare one)
+            float4 lo, hi, lo2, hi2;
+            load_pair(e + 2 * k, lo, hi);
+            load_pair(e + 2 * k + 2, lo2, hi2);
+            if (hi.w > lim) break;
+            take(k, lo, hi);
+            if (k + 1 >= cr.y || hi2.w > lim) break;
+            take(k + 1, lo2, hi2);
         }
-    };
-    for (uint32_t k = 0; k < cr.y; k += 2) {  // two entries in flight (the lists end in a spare one)
-        float4 lo, hi, lo2, hi2;
-        load_pair(e + 2 * k, lo, hi);
-        load_pair(e + 2 * k + 2, lo2, hi2);
-        if (hi.w > lim) break;
-        take(k, lo, hi);
-        if (k + 1 >= cr.y || hi2.w > lim) break;
-        take(k + 1, lo2, hi2);
-    }
-    best = INFINITY;
-    bid = 0x7FFFFFFF;
-    // (a point far outside the bounds has gaps of its own size, so the relative
-    // slack covers its remainder's rounding; one past FP32's range, or NaN, is
-    // left to FP64)
-    if (b2 > b1 * 1.000001f + L.fslack && fabsf(xh) + fabsf(yh) + fabsf(zh) < 1e37f) {
-        float4 lo, hi;
-        load_pair(e + 2 * w, lo, hi);
-        best = box_dist_finite(px, py, pz, lo, hi);
-        bid = __float_as_int(lo.w);
-        return;
+        if (kLong && (exact || !cr.y)) return;
+        if (kLong || (b2 > b1 * 1.000001f + L.fslack && S.usable())) {
+            float4 lo, hi;
+            load_pair(e + 2 * w, lo, hi);
+            best = box_dist_finite(px, py, pz, lo, hi);
+            bid = __float_as_int(lo.w);
+            return;
+        }
     }
     for (uint32_t k = 0; k < cr.y; k++) {
         const float4 lo = __ldg(e + 2 * k), hi = __ldg(e + 2 * k + 1);
@@ -550,16 +596,23 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
 // random cells in L2.  Blocks of 64: a block ends with its slowest lane, so
 // smaller ones refill the SM sooner, and 24 of them keep the 40 registers (1e7
 // points: 0.299 -> 0.286 ms on 10^4 boxes, 0.468 -> 0.435 on 10^5 against blocks
-// of 256; 32 registers for full occupancy 0.312 and 0.424).
+// of 256; 32 registers for full occupancy 0.312 and 0.424).  Layouts with longer
+// lists than those of uniform boxes (39 entries at most among 10^5) compare ties
+// on the spot, at the 64 registers that takes (3e5 points on 64 aligned boxes in
+// wide bounds, lists of 64: 0.283 -> 0.138 ms against 0.160 for one FP64 scan; 10^5
+// boxes at half a cell each, lists of 108: 0.063 -> 0.056; uniform ones 2-10%
+// slower with it).
+constexpr int kLongQuery = 48;
 constexpr int kQuery3Threads = 64;
-__global__ void __launch_bounds__(kQuery3Threads, 24)
+template <bool kLong>
+__global__ void __launch_bounds__(kQuery3Threads, kLong ? 16 : 24)
     k3_query(const Dev3Layout L, const double *__restrict__ pts, int64_t n, double *__restrict__ clear,
              int64_t *__restrict__ nearest) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double d;
     int id;
-    nearest3(L, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], d, id);
+    nearest3<kLong>(L, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], d, id);
     if (clear) clear[i] = d;
     if (nearest) nearest[i] = id;
 }
@@ -705,7 +758,7 @@ __device__ __forceinline__ void flush_job(const Walk3Params &P, int job, unsigne
     ts = ts2 = 0.0;
 }
 
-template <bool kMulti, bool kBig>
+template <bool kMulti, bool kBig, bool kLong>
 __global__ void __launch_bounds__(kBig ? kW3BigThreads : kW3Threads, kBig ? 1 : kW3MinBlocks)
     k_walk3(const Walk3Params P) {
     __shared__ uint16_t s_guide[1 << kGuide3Bits];
@@ -774,7 +827,7 @@ __global__ void __launch_bounds__(kBig ? kW3BigThreads : kW3Threads, kBig ? 1 : 
                 end = -1;
             } else {
                 int id;
-                nearest3(P.L, W.px, W.py, W.pz, d, id);
+                nearest3<kLong>(P.L, W.px, W.py, W.pz, d, id);
                 W.hops++;
                 if (d <= P.shell) end = id;
                 else if (W.hops >= P.hop_cap) end = -2;
@@ -896,6 +949,7 @@ void attach_grid3(Dev3Layout &L, const Grid3Buffers &g, const double bounds[6]) 
         M = std::max(M, std::fabs(bounds[c]));
     }
     L.fslack = (float)std::ldexp(M, -43);
+    L.max_list = g.max_list;
 }
 
 namespace {
@@ -1180,7 +1234,8 @@ frw_status build_grid3(const float *d_boxes, int64_t n, const double bounds[6], 
 frw_status launch_query3(const Dev3Layout &L, const double *d_pts, int64_t n, double *d_clear, int64_t *d_nearest,
                          cudaStream_t st) {
     if (n <= 0) return FRW_OK;
-    k3_query<<<(unsigned)((n + kQuery3Threads - 1) / kQuery3Threads), kQuery3Threads, 0, st>>>(L, d_pts, n, d_clear, d_nearest);
+    const auto kernel = L.max_list > kLongQuery ? k3_query<true> : k3_query<false>;
+    kernel<<<(unsigned)((n + kQuery3Threads - 1) / kQuery3Threads), kQuery3Threads, 0, st>>>(L, d_pts, n, d_clear, d_nearest);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k3_query");
 }
@@ -1191,8 +1246,13 @@ namespace {
 // spread over more SMs in small blocks), unless the caller asks for a number of
 // blocks or the table is too long.  A warp claims 32 walks at a time in runs of
 // a few walks per lane -- claims of 128 put four walks one after another on a
-// lane: 30,000 walks 0.37 -> 0.22 ms -- and 128 in long ones.
-template <bool kMulti>
+// lane: 30,000 walks 0.37 -> 0.22 ms -- and 128 in long ones.  Layouts with lists
+// past kLongWalk take the kernels that compare ties on the spot: they spill twice
+// as much (uniform boxes 8-10% slower, lists of 300 6-10%), which lists of 8065
+// with ties pay back (1e5 walks on a block over a plane 3.63 -> 2.17 ms, 3.29
+// for one FP64 scan).
+constexpr int kLongWalk = 512;
+template <bool kMulti, bool kLong>
 frw_status launch_walk3_as(Walk3Params P, int sms, int bps, cudaStream_t st) {
     const size_t thr = (size_t)P.nb * sizeof(uint32_t);
     const uint64_t warps = (uint64_t)sms * (kW3BigThreads / 32);
@@ -1202,13 +1262,13 @@ frw_status launch_walk3_as(Walk3Params P, int sms, int bps, cudaStream_t st) {
         // the largest table's size, whichever table this launch has: the attribute
         // is the kernel's, and another host thread's launch may have a longer one
         const cudaError_t e =
-            cudaFuncSetAttribute(k_walk3<kMulti, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kW3ThrBytes);
+            cudaFuncSetAttribute(k_walk3<kMulti, true, kLong>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kW3ThrBytes);
         if (e != cudaSuccess) return cuda_fail(e, "k_walk3: shared memory");
-        k_walk3<kMulti, true><<<sms, kW3BigThreads, thr, st>>>(P);
+        k_walk3<kMulti, true, kLong><<<sms, kW3BigThreads, thr, st>>>(P);
     } else {
         const uint64_t need = std::max<uint64_t>((P.walks + kW3Threads - 1) / kW3Threads, 1);
         const int full = sms * (bps > 0 ? std::min(bps, kW3MinBlocks) : kW3MinBlocks);
-        k_walk3<kMulti, false><<<(unsigned)std::min<uint64_t>(need, full), kW3Threads, 0, st>>>(P);
+        k_walk3<kMulti, false, kLong><<<(unsigned)std::min<uint64_t>(need, full), kW3Threads, 0, st>>>(P);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k_walk3");
@@ -1216,11 +1276,13 @@ frw_status launch_walk3_as(Walk3Params P, int sms, int bps, cudaStream_t st) {
 }  // namespace
 
 frw_status launch_walk3(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t st) {
-    return launch_walk3_as<false>(P, sms, blocks_per_sm, st);
+    return P.L.max_list > kLongWalk ? launch_walk3_as<false, true>(P, sms, blocks_per_sm, st)
+                          : launch_walk3_as<false, false>(P, sms, blocks_per_sm, st);
 }
 
 frw_status launch_walk3_batch(const Walk3Params &P, int sms, int blocks_per_sm, cudaStream_t st) {
-    return launch_walk3_as<true>(P, sms, blocks_per_sm, st);
+    return P.L.max_list > kLongWalk ? launch_walk3_as<true, true>(P, sms, blocks_per_sm, st)
+                          : launch_walk3_as<true, false>(P, sms, blocks_per_sm, st);
 }
 
 }  // namespace frw

@@ -67,3 +67,26 @@ def test_walk_counts_and_launch_shapes(walks):
     k, n = np.unique(end[end >= 0], return_counts=True)
     assert np.array_equal(r.conductor, k) and np.array_equal(r.hits, n)
     assert np.allclose(r.sum_w, [w[end == c].sum() for c in k], rtol=1e-11, atol=1e-11 * np.abs(w).sum())
+
+
+@pytest.mark.parametrize("k,step", [(3, 0), (4, 0), (7, 0), (9, 0), (9, 1e-7), (9, 1e-3)])
+def test_long_lists_of_ties(k, step):
+    """A block of aligned boxes in wide bounds: the lists of distant cells hold
+    all of it (from 27 entries, scanned again on ties, to 729, compared on the
+    spot), and whole faces of it tie, exactly or nearly.  Queries and walks."""
+    b = boxes_at(1.0, 0.0, k)
+    b[1:, :3] += np.float32(step) * np.arange(len(b) - 1, dtype=np.float32)[:, None] / len(b)
+    bounds = np.array([-300.0, -250, -200, 300, 320, 280])
+    rng = np.random.default_rng(k)
+    p = bounds[:3] + rng.random((5000, 3)) * (bounds[3:] - bounds[:3])
+    p[:2000] = np.round(p[:2000])
+    p[2000:2500] = 1.5 * k + rng.choice([-150.0, 150.0], (500, 3))  # on the diagonals
+    B = O.Boxes3(b, bounds)
+    d_o, k_o = B.nearest(p)
+    with frw.Layout3.from_boxes(b, bounds) as L:
+        assert L.info.max_list == k**3
+        d, near = L.query(p)
+        got = L.walk_trace(k, 0, 1500, 9)
+    assert np.array_equal(d, d_o) and np.array_equal(near, k_o)
+    for x, y in zip(got, B.walks(B.cfg(target=k, offset=1.0, seed=9), 0, 1500)):
+        assert np.array_equal(x, y)
