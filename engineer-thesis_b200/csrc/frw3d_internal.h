@@ -49,6 +49,7 @@ struct Dev3Layout {
     int nx, ny, nz;
     int nup;               // coarser levels
     int max_list;          // longest list of any level
+    int64_t list_bytes;    // of the finest level's lists
     const Level3 *up;      // [nup] device array
     uint32_t *status;      // kSt3* bits (device word of the layout)
     double b[6];           // bounds (x0,y0,z0,x1,y1,z1), open

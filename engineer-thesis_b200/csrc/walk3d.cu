@@ -480,8 +480,10 @@ __device__ __forceinline__ Split3 split3(double px, double py, double pz) {
     return s;
 }
 
-// kLong: for layouts with long lists (kLongQuery, kLongWalk), see below.
-template <bool kLong>
+// kLong: for layouts with long lists (kLongQuery, kLongWalk), see below.  kKeep:
+// entries one at a time, the best one kept in registers instead of read again:
+// fewer reads, more registers.
+template <bool kLong, bool kKeep = false>
 __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double py, double pz, double &best,
                                          int &bid) {
     const int ix = cell_axis(px, L.g0x, L.ginv, L.nx);
@@ -531,6 +533,8 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
         float b1 = 3.0e38f, b2 = 3.0e38f, lim = 3.0e38f;  // b2: the second nearest; kLong: past it clearly farther
         uint32_t w = 0;
         bool exact = false;  // kLong: best and bid are the best entry's
+        float4 klo, khi;     // kKeep: the best entry
+        if (kKeep) klo = khi = make_float4(0.f, 0.f, 0.f, 0.f);
         auto take = [&](uint32_t k, const float4 &lo, const float4 &hi) {
             const float g = S.gap(lo, hi);
             if (kLong) {
@@ -539,7 +543,7 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
                     exact = false;
                 } else {
                     if (!exact) {
-                        const float4 blo = __ldg(e + 2 * w), bhi = __ldg(e + 2 * w + 1);
+                        const float4 blo = kKeep ? klo : __ldg(e + 2 * w), bhi = kKeep ? khi : __ldg(e + 2 * w + 1);
                         best = box_dist_finite(px, py, pz, blo, bhi);
                         bid = __float_as_int(blo.w);
                         exact = true;
@@ -557,23 +561,27 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
             }
             b1 = g;
             w = k;
+            if (kKeep) {
+                klo = lo;
+                khi = hi;
+            }
             lim = (b1 + hqf) * 1.000002f + L.fslack;
         };
-        for (uint32_t k = 0; k < cr.y; k += 2) {  // two entries in flight (the lists end in a spare one)
+        for (uint32_t k = 0; k < cr.y; k += kKeep ? 1 : 2) {  // two entries in flight (the lists end in a spare one)
             float4 lo, hi, lo2, hi2;
             load_pair(e + 2 * k, lo, hi);
-            load_pair(e + 2 * k + 2, lo2, hi2);
+            if (!kKeep) load_pair(e + 2 * k + 2, lo2, hi2);
             if (hi.w > lim) break;
             take(k, lo, hi);
+            if (kKeep) continue;
             if (k + 1 >= cr.y || hi2.w > lim) break;
             take(k + 1, lo2, hi2);
         }
         if (kLong && (exact || !cr.y)) return;
         if (kLong || (b2 > b1 * 1.000001f + L.fslack && S.usable())) {
-            float4 lo, hi;
-            load_pair(e + 2 * w, lo, hi);
-            best = box_dist_finite(px, py, pz, lo, hi);
-            bid = __float_as_int(lo.w);
+            if (!kKeep) load_pair(e + 2 * w, klo, khi);
+            best = box_dist_finite(px, py, pz, klo, khi);
+            bid = __float_as_int(klo.w);
             return;
         }
     }
@@ -601,18 +609,24 @@ __device__ __forceinline__ void nearest3(const Dev3Layout &L, double px, double 
 // on the spot, at the 64 registers that takes (3e5 points on 64 aligned boxes in
 // wide bounds, lists of 64: 0.283 -> 0.138 ms against 0.160 for one FP64 scan; 10^5
 // boxes at half a cell each, lists of 108: 0.063 -> 0.056; uniform ones 2-10%
-// slower with it).
+// slower with it).  Lists of twice the L2 and more are read from HBM, whose
+// requests bound them: the best entry stays in registers, 20 blocks at 48 (1e7
+// points: on 2e5 boxes, 445 MB, 0.82 -> 0.73 ms against 0.80 for one FP64 scan; on
+// 3e5 1.14 -> 1.00 against 1.03; on 6e5 2.11 -> 1.85 against 1.78; on 10^5, 200 MB,
+// 0.44 -> 0.50).
 constexpr int kLongQuery = 48;
+constexpr int64_t kFarLists = int64_t(256) << 20;
+enum : int { kQueryShort = 0, kQueryLong = 1, kQueryFar = 2 };
 constexpr int kQuery3Threads = 64;
-template <bool kLong>
-__global__ void __launch_bounds__(kQuery3Threads, kLong ? 16 : 24)
+template <int kKind>
+__global__ void __launch_bounds__(kQuery3Threads, kKind == kQueryShort ? 24 : kKind == kQueryLong ? 16 : 20)
     k3_query(const Dev3Layout L, const double *__restrict__ pts, int64_t n, double *__restrict__ clear,
              int64_t *__restrict__ nearest) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double d;
     int id;
-    nearest3<kLong>(L, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], d, id);
+    nearest3<kKind != kQueryShort, kKind == kQueryFar>(L, pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], d, id);
     if (clear) clear[i] = d;
     if (nearest) nearest[i] = id;
 }
@@ -950,6 +964,7 @@ void attach_grid3(Dev3Layout &L, const Grid3Buffers &g, const double bounds[6]) 
     }
     L.fslack = (float)std::ldexp(M, -43);
     L.max_list = g.max_list;
+    L.list_bytes = g.entries * 32;
 }
 
 namespace {
@@ -1234,7 +1249,9 @@ frw_status build_grid3(const float *d_boxes, int64_t n, const double bounds[6], 
 frw_status launch_query3(const Dev3Layout &L, const double *d_pts, int64_t n, double *d_clear, int64_t *d_nearest,
                          cudaStream_t st) {
     if (n <= 0) return FRW_OK;
-    const auto kernel = L.max_list > kLongQuery ? k3_query<true> : k3_query<false>;
+    const auto kernel = L.list_bytes > kFarLists   ? k3_query<kQueryFar>
+                        : L.max_list > kLongQuery ? k3_query<kQueryLong>
+                                                  : k3_query<kQueryShort>;
     kernel<<<(unsigned)((n + kQuery3Threads - 1) / kQuery3Threads), kQuery3Threads, 0, st>>>(L, d_pts, n, d_clear, d_nearest);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FRW_OK : cuda_fail(e, "k3_query");

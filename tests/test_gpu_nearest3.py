@@ -90,3 +90,20 @@ def test_long_lists_of_ties(k, step):
     assert np.array_equal(d, d_o) and np.array_equal(near, k_o)
     for x, y in zip(got, B.walks(B.cfg(target=k, offset=1.0, seed=9), 0, 1500)):
         assert np.array_equal(x, y)
+
+
+def test_lists_past_the_l2():
+    """A layout whose lists are read from HBM takes the kernel that keeps the best
+    entry in registers: nearest boxes, ties of lined-up boxes included, equal the
+    oracle's."""
+    b = frw.generate_layout3(3, 150_000, 20.0 * 150_000**0.5, 400.0, 5, 50, 5, 20, 2)
+    B = O.Boxes3(b, grid=True)
+    rng = np.random.default_rng(0)
+    p = B.bounds[:3] + rng.random((60_000, 3)) * (B.bounds[3:] - B.bounds[:3])
+    p[:20_000] = np.round(p[:20_000])
+    p[20_000:30_000] = b[rng.integers(0, len(b), 10_000), 3:]
+    with frw.Layout3.from_boxes(b) as L:
+        assert L.info.list_entries * 32 > 256 << 20
+        d, near = L.query(p)
+    d_o, k_o = B.nearest(p)
+    assert np.array_equal(d, d_o) and np.array_equal(near, k_o)
