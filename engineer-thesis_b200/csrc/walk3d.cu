@@ -208,26 +208,31 @@ __device__ __forceinline__ void entry_swap(float4 *e, int64_t a, int64_t b) {
     e[2 * b] = lo;
     e[2 * b + 1] = hi;
 }
-__device__ __forceinline__ void sift_down(float4 *e, int64_t root, int64_t end) {
-    for (int64_t c = 2 * root + 1; c < end; c = 2 * root + 1) {
-        if (c + 1 < end && entry_less(e, c, c + 1)) c++;
-        if (!entry_less(e, root, c)) return;
-        entry_swap(e, root, c);
-        root = c;
-    }
-}
-// One thread's list, in place: insertion for short lists (the usual case),
-// heapsort for the long ones of coarse cells facing a dense cluster.
-__device__ void sort_entries(float4 *e, int64_t m) {
-    if (m <= 32) {
-        for (int64_t a = 1; a < m; a++)
-            for (int64_t b = a; b > 0 && entry_less(e, b, b - 1); b--) entry_swap(e, b, b - 1);
-        return;
-    }
-    for (int64_t r = m / 2 - 1; r >= 0; r--) sift_down(e, r, m);
-    for (int64_t end = m - 1; end > 0; end--) {
-        entry_swap(e, 0, end);
-        sift_down(e, 0, end);
+// The lists left unordered (of the cells in `todo`), a block each, in place: a
+// bitonic network whose merges start mirrored, so every comparator orders
+// upwards and those past the list's end are left out.  (A lane per list, by
+// heapsort in global memory, was bound by its chain of loads and slower still in a
+// kernel that leaves the L1 little room: grids of 4096 boxes in wide bounds 323 ->
+// 57 ms, of 10^5 boxes at half a cell each 3.13 -> 1.73, 300 and 2.15 with the
+// heapsort in a kernel without shared memory.)
+constexpr int kSortThreads = 128;
+__global__ void __launch_bounds__(kSortThreads)
+    k3_sort_lists(const uint2 *__restrict__ cells, const int32_t *__restrict__ todo, float4 *lists) {
+    const uint2 cr = cells[todo[blockIdx.x]];
+    float4 *e = lists + 2 * (int64_t)cr.x;
+    const int64_t m = cr.y;
+    auto step = [&](int lg, bool mirrored) {  // comparators of sequences of 2^lg entries
+        const int64_t size = 1ll << lg, half = size >> 1;
+        for (int64_t t = threadIdx.x;; t += kSortThreads) {
+            const int64_t at = (t >> (lg - 1)) << lg, o = t & (half - 1), p = at + (mirrored ? size - 1 - o : half + o);
+            if (at >= m) break;
+            if (p < m && entry_less(e, p, at + o)) entry_swap(e, at + o, p);
+        }
+        __syncthreads();
+    };
+    for (int lg = 1; (1ll << (lg - 1)) < m; lg++) {
+        step(lg, true);
+        for (int k = lg - 1; k > 0; k--) step(k, false);
     }
 }
 
@@ -245,7 +250,8 @@ __device__ void sort_entries(float4 *e, int64_t m) {
 // needed; cells outside `need` (when given) are unused.  More candidates than
 // fit (coarse cells facing a dense cluster) pass through in chunks.  Lists go to the shared
 // buffer at an offset from a global cursor, ordered by (distance from the
-// centre, index); past `room` entries they are counted, not written (the caller
+// centre, index) -- longer ones by k3_sort_lists, their cells in todo[0 .. tot[3])
+// --; past `room` entries they are counted, not written (the caller
 // runs the pass again with room for tot[0]).
 // Why: a thread per cell walked its own bins -- 7 of 32 lanes active -- twice,
 // counting and then filling, and ordered 32-byte entries in place in global
@@ -273,7 +279,7 @@ __global__ void __launch_bounds__(kBrickWarps * 32)
     k3_cell_lists(const float *__restrict__ boxes, Grid3 G, const int64_t *__restrict__ bstart,
                   const int32_t *__restrict__ items, const uint8_t *__restrict__ need, uint8_t *__restrict__ need_up,
                   int upnx, int upny, uint2 *__restrict__ cells, float4 *__restrict__ lists, int64_t room,
-                  unsigned long long *__restrict__ tot, int64_t nbricks) {
+                  int32_t *__restrict__ todo, unsigned long long *__restrict__ tot, int64_t nbricks) {
     __shared__ BrickShared<kBrickCand> s_brick[kBrickWarps];
     const int lane = threadIdx.x & 31;
     const int64_t brick = (int64_t)blockIdx.x * kBrickWarps + (threadIdx.x >> 5);
@@ -436,7 +442,13 @@ __global__ void __launch_bounds__(kBrickWarps * 32)
             out[2 * k + 1] = hi;
         }
     if (__all_sync(kFull, ordered)) return;
-    // long lists: written as they come, then ordered in place
+    // long lists: written as they come, ordered by k3_sort_lists
+    const bool later = lists_here && !ordered && m > 1;
+    const unsigned l = __ballot_sync(kFull, later);
+    unsigned long long t0 = 0;
+    if (lane == 0 && l) t0 = atomicAdd(tot + 3, (unsigned long long)__popc(l));
+    t0 = __shfl_sync(kFull, t0, 0);
+    if (later) todo[t0 + __popc(l & ((1u << lane) - 1u))] = (int32_t)c;
     int w = 0;
     candidates([&](int n) {
         for (int k = 0; k < n; k++) {
@@ -449,7 +461,6 @@ __global__ void __launch_bounds__(kBrickWarps * 32)
             w++;
         }
     });
-    if (lists_here && !ordered) sort_entries(out, m);
 }
 
 // ---- query -----------------------------------------------------------------
@@ -983,8 +994,8 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
     const int64_t nbricks = (int64_t)((G.n[0] + kBrickX - 1) / kBrickX) * ((G.n[1] + kBrickY - 1) / kBrickY) *
                             ((G.n[2] + kBrickZ - 1) / kBrickZ);
     int64_t *bcnt = nullptr, *bstart = nullptr, *sums = nullptr, *grand = nullptr;
-    int32_t *items = nullptr;
-    unsigned long long *tot = nullptr;  // list entries, longest list, deferred cells
+    int32_t *items = nullptr, *todo = nullptr;
+    unsigned long long *tot = nullptr;  // list entries, longest list, deferred cells, lists to sort
     const int64_t tiles = scan_i64_tiles(ncells + 1);
     frw_status rc = FRW_OK;
     auto ck = [&](cudaError_t e, const char *what) {
@@ -997,7 +1008,8 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         if (!ck(cudaMallocAsync(&bstart, cb, st), "malloc bin starts")) break;
         if (!ck(cudaMallocAsync(&sums, (size_t)tiles * 8, st), "malloc tile sums")) break;
         if (!ck(cudaMallocAsync(&grand, 8, st), "malloc totals")) break;
-        if (!ck(cudaMallocAsync(&tot, 24, st), "malloc stats")) break;
+        if (!ck(cudaMallocAsync(&tot, 32, st), "malloc stats")) break;
+        if (!ck(cudaMallocAsync(&todo, (size_t)ncells * 4, st), "malloc lists to sort")) break;
         if (!ck(cudaMallocAsync(&out->cells, (size_t)ncells * sizeof(uint2), st), "malloc cells")) break;
         if (!ck(cudaMemsetAsync(bcnt, 0, cb, st), "memset")) break;
         const unsigned nb = (unsigned)((n + 255) / 256);
@@ -1020,16 +1032,17 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         // took a second pass, 7.3 -> 4.4 ms);
         // longer ones take a second pass, and a buffer mostly unused a copy
         int64_t room = 10 * ncells + 4096;
-        unsigned long long h[3] = {0, 0, 0};
+        unsigned long long h[4] = {0, 0, 0, 0};
         for (int pass = 0; pass < 2; pass++) {
             // (a query may read one entry past a list)
             if (!ck(cudaMallocAsync(&out->lists, (size_t)(room + 1) * 32, st), "malloc lists")) break;
-            if (!ck(cudaMemsetAsync(tot, 0, 24, st), "memset")) break;
+            if (!ck(cudaMemsetAsync(tot, 0, 32, st), "memset")) break;
             const auto kernel = need ? k3_cell_lists<kCoarseCand> : k3_cell_lists<kFineCand>;
             kernel<<<(unsigned)((nbricks + kBrickWarps - 1) / kBrickWarps), kBrickWarps * 32, 0, st>>>(
-                d_boxes, G, bstart, items, need, need_up, upnx, upny, out->cells, out->lists, room, tot, nbricks);
+                d_boxes, G, bstart, items, need, need_up, upnx, upny, out->cells, out->lists, room, todo, tot,
+                nbricks);
             if (!ck(cudaGetLastError(), "cell lists")) break;
-            if ((rc = read_back(h, tot, 24, st, "build_grid3: list total"))) break;
+            if ((rc = read_back(h, tot, 32, st, "build_grid3: list total"))) break;
             if (h[0] > (unsigned long long)INT32_MAX) {
                 set_error("build_grid3: more than 2^31 list entries; use fewer cells per box");
                 rc = FRW_E_ARG;
@@ -1044,6 +1057,10 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         out->entries = (int64_t)h[0];
         out->max_list = h[1];
         out->deferred = (int64_t)h[2];
+        if (h[3]) {
+            k3_sort_lists<<<(unsigned)h[3], kSortThreads, 0, st>>>(out->cells, todo, out->lists);
+            if (!ck(cudaGetLastError(), "list order")) break;
+        }
         if (out->entries < room - room / 3) {
             float4 *exact = nullptr;
             if (!ck(cudaMallocAsync(&exact, (size_t)(out->entries + 1) * 32, st), "malloc lists")) break;
@@ -1054,7 +1071,7 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
             if (!ck(e, "lists")) break;
         }
     } while (0);
-    for (void *p : {(void *)bcnt, (void *)bstart, (void *)sums, (void *)grand, (void *)items, (void *)tot})
+    for (void *p : {(void *)bcnt, (void *)bstart, (void *)sums, (void *)grand, (void *)items, (void *)todo, (void *)tot})
         if (p) cudaFreeAsync(p, st);
     if (rc != FRW_OK) {
         if (out->cells) cudaFreeAsync(out->cells, st);
