@@ -1038,7 +1038,9 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         // room for the lists of the default density (7 to 9.2 entries per cell, the
         // more the larger the layout: 3e5 boxes passed 9 and
         // took a second pass, 7.3 -> 4.4 ms);
-        // longer ones take a second pass, and a buffer mostly unused a copy
+        // longer ones take a second pass, and a buffer mostly unused a copy.  Where
+        // there is no memory for that room, the first pass counts only and the
+        // second has the lists' own; without memory for the copy the buffer stays.
         int64_t room = 10 * ncells + 4096;
         unsigned long long h[4] = {0, 0, 0, 0};
         // the bricks' first search: a little over two cells, or little more than the
@@ -1047,7 +1049,13 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         const double first_radius = (nitems > 4 * ncells ? 2.5 : 5.0) * G.h;
         for (int pass = 0; pass < 2; pass++) {
             // (a query may read one entry past a list)
-            if (!ck(cudaMallocAsync(&out->lists, (size_t)(room + 1) * 32, st), "malloc lists")) break;
+            cudaError_t e = cudaMallocAsync(&out->lists, (size_t)(room + 1) * 32, st);
+            if (e == cudaErrorMemoryAllocation && pass == 0) {
+                cudaGetLastError();
+                room = 0;
+                e = cudaMallocAsync(&out->lists, 32, st);
+            }
+            if (!ck(e, "malloc lists")) break;
             if (!ck(cudaMemsetAsync(tot, 0, 32, st), "memset")) break;
             const auto kernel = need ? k3_cell_lists<kCoarseCand> : k3_cell_lists<kFineCand>;
             kernel<<<(unsigned)((nbricks + kBrickWarps - 1) / kBrickWarps), kBrickWarps * 32, 0, st>>>(
@@ -1075,12 +1083,15 @@ frw_status build_level(const float *d_boxes, int64_t n, const Grid3 &G, const ui
         }
         if (out->entries < room - room / 3) {
             float4 *exact = nullptr;
-            if (!ck(cudaMallocAsync(&exact, (size_t)(out->entries + 1) * 32, st), "malloc lists")) break;
-            const cudaError_t e =
-                cudaMemcpyAsync(exact, out->lists, (size_t)out->entries * 32, cudaMemcpyDeviceToDevice, st);
-            cudaFreeAsync(out->lists, st);
-            out->lists = exact;
-            if (!ck(e, "lists")) break;
+            if (cudaMallocAsync(&exact, (size_t)(out->entries + 1) * 32, st) == cudaSuccess) {
+                const cudaError_t e =
+                    cudaMemcpyAsync(exact, out->lists, (size_t)out->entries * 32, cudaMemcpyDeviceToDevice, st);
+                cudaFreeAsync(out->lists, st);
+                out->lists = exact;
+                if (!ck(e, "lists")) break;
+            } else {
+                cudaGetLastError();
+            }
         }
     } while (0);
     for (void *p : {(void *)bcnt, (void *)bstart, (void *)sums, (void *)grand, (void *)items, (void *)todo, (void *)tot})
