@@ -34,70 +34,86 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
-// The target's neighbours, from the cells around it: a block tries a reach of 8
-// cell sides (twice the mean distance of rects at 16 cells per rect), then
-// halves it while they are too many.  A rect is taken from the one cell of its
-// lowest corner within reach, whose list holds it as it touches that cell.
+// The target's neighbours, from the cells around it, at reaches of 8 cell sides
+// (twice the mean distance of rects at 16 cells per rect), 4, 2, 1 and 1/2 at
+// once: a rect goes to the list of every reach it comes within, so the largest
+// reach with few enough of them is at hand.  Reaches over more than
+// kNeighbourCells cells, and all of them when a cell is left to the tree, are
+// marked full.  A rect is taken from the one cell of its lowest corner within
+// reach, whose list holds it as it touches that cell.
 // Why a list: the target is excluded, so a first hop's nearest other conductor
 // lies beyond its cell's list, and the tree, whose search starts at the target
 // and without a bound, issued 11800 instructions per warp: exact mean of 16384
 // starts on 10^5 rects 0.775 -> 0.415 ms, a training run with 10^6 features 3.09
-// -> 3.02.
-constexpr int kNeighbourThreads = 256, kNeighbourCells = 16384;
+// -> 3.02.  Why all reaches at once, a thread per cell: one block that tried a
+// reach after another took 0.16 ms around a target with hundreds of neighbours,
+// more than the list saves (training on 10^5 walks around a plate of 3000 x 3000
+// units 0.91 -> 0.61 ms against 0.70 without lists).
+constexpr int kNeighbourThreads = 256, kNeighbourCells = 16384, kNeighbourFull = 1 << 30;
+
+// The box of the bounds within a reach of the target, and its cells.
+struct NeighbourBox {
+    double B[4];
+    int x0, y0, w, h;
+};
+__device__ __forceinline__ NeighbourBox neighbour_box(const DevLayout &L, double4 t, double reach) {
+    NeighbourBox b;
+    b.B[0] = dmax(t.x - reach, L.bx0);
+    b.B[1] = dmax(t.y - reach, L.by0);
+    b.B[2] = dmin(t.z + reach, L.bx1);
+    b.B[3] = dmin(t.w + reach, L.by1);
+    const uint2 c0 = cell_xy(L, b.B[0], b.B[1]), c1 = cell_xy(L, b.B[2], b.B[3]);
+    b.x0 = (int)c0.x;
+    b.y0 = (int)c0.y;
+    b.w = (int)(c1.x - c0.x) + 1;
+    b.h = (int)(c1.y - c0.y) + 1;
+    return b;
+}
+
 __global__ void __launch_bounds__(kNeighbourThreads) k_neighbours(DevLayout L, double4 trect, int tid, Neighbours *out) {
-    __shared__ int s_n, s_bad;
-    double reach = 8.0 / L.ginv;
-    for (int pass = 0; L.cells && pass < 5; pass++, reach *= 0.5) {
-        if (threadIdx.x == 0) s_n = s_bad = 0;
-        __syncthreads();
-        const double B[4] = {dmax(trect.x - reach, L.bx0), dmax(trect.y - reach, L.by0), dmin(trect.z + reach, L.bx1),
-                             dmin(trect.w + reach, L.by1)};
-        const FloatBox fb = float_box(B);
-        const int64_t c0 = cell_of(L, B[0], B[1]), c1 = cell_of(L, B[2], B[3]);
-        const int x0 = (int)(c0 % L.gnx), y0 = (int)(c0 / L.gnx);
-        const int w = (int)(c1 % L.gnx) - x0 + 1, h = (int)(c1 / L.gnx) - y0 + 1;
-        if ((int64_t)w * h > kNeighbourCells) continue;
-        for (int i = threadIdx.x; i < w * h; i += kNeighbourThreads) {
-            const int64_t cell = (int64_t)(y0 + i / w) * L.gnx + x0 + i % w;
-            const float4 *r = L.cells + kCellSlots * cell;
-            const int32_t *ids = reinterpret_cast<const int32_t *>(L.cellids + cell);
-            const float4 last = __ldg(r + kCellSlots - 1);
-            int n = kCellSlots;
-            if (last.x > kFarRect) {  // a longer list, a short one near the bounds, or (n < 0) the tree
-                n = __float_as_int(last.z);
-                if (n < 0) s_bad = 1;
-                if (n >= kCellSlots) {
-                    r = L.crects + __float_as_int(last.y);
-                    ids = L.cids + __float_as_int(last.y);
-                }
+    int level = 0;  // the largest reach that is looked at
+    NeighbourBox box = neighbour_box(L, trect, neighbour_reach(L, 0));
+    while ((int64_t)box.w * box.h > kNeighbourCells && ++level < kNeighbourLevels)
+        box = neighbour_box(L, trect, neighbour_reach(L, level));
+    if (blockIdx.x == 0 && threadIdx.x < kNeighbourLevels) out->reach[threadIdx.x] = neighbour_reach(L, threadIdx.x);
+    if (blockIdx.x == 0 && (int)threadIdx.x < level) atomicOr(&out->n[threadIdx.x], kNeighbourFull);
+    if (level == kNeighbourLevels) return;
+    FloatBox fb[kNeighbourLevels];
+#pragma unroll
+    for (int l = 0; l < kNeighbourLevels; l++) fb[l] = float_box(neighbour_box(L, trect, neighbour_reach(L, l)).B);
+    for (int i = blockIdx.x * kNeighbourThreads + threadIdx.x; i < box.w * box.h; i += gridDim.x * kNeighbourThreads) {
+        const int cx = box.x0 + i % box.w, cy = box.y0 + i / box.w;
+        const int64_t cell = (int64_t)cy * L.gnx + cx;
+        const float4 *r = L.cells + kCellSlots * cell;
+        const int32_t *ids = reinterpret_cast<const int32_t *>(L.cellids + cell);
+        const float4 last = __ldg(r + kCellSlots - 1);
+        int n = kCellSlots;
+        if (last.x > kFarRect) {  // a longer list, a short one near the bounds, or (n < 0) the tree
+            n = __float_as_int(last.z);
+            if (n < 0)
+                for (int l = level; l < kNeighbourLevels; l++) atomicOr(&out->n[l], kNeighbourFull);
+            if (n >= kCellSlots) {
+                r = L.crects + __float_as_int(last.y);
+                ids = L.cids + __float_as_int(last.y);
             }
-            for (int k = 0; k < n; k++) {
-                const int id = __ldg(ids + k);
-                if (id < 0 || id == tid) continue;
-                const float4 q = __ldg(r + k);
-                if (!fb.touches(q) || cell_of(L, dmax((double)q.x, B[0]), dmax((double)q.y, B[1])) != cell) continue;
-                const int at = atomicAdd(&s_n, 1);
+        }
+#pragma unroll 4
+        for (int k = 0; k < n; k++) {
+            const int id = __ldg(ids + k);
+            const float4 q = __ldg(r + k);
+            if (id < 0 || id == tid) continue;
+            const uint2 lowest = cell_xy(L, dmax((double)q.x, box.B[0]), dmax((double)q.y, box.B[1]));
+            if ((int)lowest.x != cx || (int)lowest.y != cy) continue;
+#pragma unroll
+            for (int l = 0; l < kNeighbourLevels; l++) {
+                if (l < level || !fb[l].touches(q)) continue;
+                const int at = atomicAdd(&out->n[l], 1);
                 if (at < kNeighbours) {
-                    out->rects[at] = q;
-                    out->ids[at] = id;
+                    out->rects[l][at] = q;
+                    out->ids[l][at] = id;
                 }
             }
         }
-        __syncthreads();
-        const int n = s_n, bad = s_bad;
-        __syncthreads();
-        if (bad) break;
-        if (n <= kNeighbours) {
-            if (threadIdx.x == 0) {
-                out->n = n;
-                out->reach = reach;
-            }
-            return;
-        }
-    }
-    if (threadIdx.x == 0) {
-        out->n = -1;
-        out->reach = 0.0;
     }
 }
 
@@ -725,7 +741,18 @@ frw_status net_upload(Net *n, const float *host, cudaStream_t st) {
 }
 
 frw_status launch_neighbours(const DevLayout &L, double4 trect, int tid, Neighbours *out, cudaStream_t st) {
-    k_neighbours<<<1, kNeighbourThreads, 0, st>>>(L, trect, tid, out);
+    FRW_CK(cudaMemsetAsync(out->n, 0, sizeof(out->n), st));
+    if (!L.cells) return FRW_OK;  // no neighbours: the tree
+    // a thread per cell of the first reach whose cells are not too many (it is the
+    // kernel that decides)
+    double cells = 0;
+    for (int l = 0; l < kNeighbourLevels; l++) {
+        const double r = neighbour_reach(L, l) * 2 * L.ginv + 2;
+        cells = ((trect.z - trect.x) * L.ginv + r) * ((trect.w - trect.y) * L.ginv + r);
+        if (cells <= kNeighbourCells) break;
+    }
+    const int blocks = (int)std::max(1.0, std::min(cells, (double)kNeighbourCells) / kNeighbourThreads + 1);
+    k_neighbours<<<blocks, kNeighbourThreads, 0, st>>>(L, trect, tid, out);
     FRW_CK(cudaGetLastError());
     return FRW_OK;
 }

@@ -33,21 +33,24 @@ void net_free(Net *n, cudaStream_t st);
 frw_status net_upload(Net *n, const float *host_params, cudaStream_t st);
 frw_status net_refresh_bf16(const Net &n, cudaStream_t st);
 
+// The conductors around a target, for each reach l of neighbour_reach: every rect
+// of its layer but the target itself that comes within the reach of the target
+// rect (n[l] of them, the first kNeighbours listed: the list is whole when n[l]
+// is no more).  Points near the target look their nearest other conductor up
+// here.
+constexpr int kNeighbours = 64, kNeighbourLevels = 5;
+struct Neighbours {
+    int n[8];
+    double reach[kNeighbourLevels + 1];
+    int32_t ids[kNeighbourLevels][kNeighbours];
+    float4 rects[kNeighbourLevels][kNeighbours];
+};
+FRW_HD double neighbour_reach(const DevLayout &L, int level) { return 8.0 / L.ginv / (double)(1 << level); }  // reach[level]
+frw_status launch_neighbours(const DevLayout &L, double4 target_rect, int target_id, Neighbours *out, cudaStream_t st);
 // features of points p (first-hop points) w.r.t. a target rect: the
 // (dx, dy) from p to the nearest point of each edge of the target and of
-// the nearest other conductor, divided by a0 and clamped to [-16, 16].
-// The conductors around a target: every rect of its layer but the target itself
-// (layer index of each) that comes within `reach` of the target rect; n < 0
-// when no reach has few enough of them.  Points near the target look their
-// nearest other conductor up here.
-constexpr int kNeighbours = 64;
-struct Neighbours {
-    int n;
-    double reach;
-    float4 rects[kNeighbours];
-    int32_t ids[kNeighbours];
-};
-frw_status launch_neighbours(const DevLayout &L, double4 target_rect, int target_id, Neighbours *out, cudaStream_t st);
+// the nearest other conductor, divided by a0 and clamped to [-16, 16].  nb: the
+// target's neighbours, or null.
 frw_status launch_features(const DevLayout &L, double4 target_rect, int target_id, const Neighbours *nb,
                            const double4 *rec, int64_t n, __nv_bfloat16 *xb, float *xf, cudaStream_t st);
 // The MLP kernels: tcgen05 / TMEM tiles of 128 rows (cv_umma.cu, the

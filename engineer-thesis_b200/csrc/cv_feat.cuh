@@ -91,26 +91,31 @@ static __device__ int nearest_other_tree(const DevLayout &L, double px, double p
     return best_k;
 }
 
-// The same from the list of the target's neighbours (cv.cuh) where it settles
-// the answer: it holds every other rect within reach of the target rect, so a
-// nearest one within reach less p's own distance to the target (two deltas
-// cover the rounding) is the nearest, ties included.
+// The same from the list of the target's neighbours (cv.cuh) at the largest reach
+// that has a whole one, where it settles the answer: it holds every other rect
+// within reach of the target rect, so a nearest one within reach less p's own
+// distance to the target (two deltas cover the rounding) is the nearest, ties
+// included.
 static __device__ __forceinline__ bool nearest_neighbour(const DevLayout &L, double4 target, const Neighbours *nb,
                                                          double px, double py, float4 &o) {
-    const int n = __ldg(&nb->n);
+    int l = 0;
+    while (l < kNeighbourLevels && __ldg(nb->n + l) > kNeighbours) l++;
+    if (l == kNeighbourLevels) return false;
+    const int n = __ldg(nb->n + l);
+    if (n <= 0) return false;
     const double away = dmax(dmax(dmax(target.x - px, px - target.z), dmax(target.y - py, py - target.w)), 0.0);
-    const double within = __ldg(&nb->reach) - away - 2.0 * L.delta;
-    if (n <= 0 || !(within > 0.0)) return false;
+    const double within = __ldg(nb->reach + l) - away - 2.0 * L.delta;
+    if (!(within > 0.0)) return false;
     const float pxf = (float)px, pyf = (float)py;
     float limf = 3.0e38f;
     double best = 1e300;
     int best_id = 0x7FFFFFFF;
 #pragma unroll 4
     for (int k = 0; k < n; k++) {
-        const float4 q = __ldg(nb->rects + k);
+        const float4 q = __ldg(nb->rects[l] + k);
         if (fmaxf(fmaxf(q.x - pxf, pxf - q.z), fmaxf(q.y - pyf, pyf - q.w)) > limf) continue;
         const double g = rect_gap(q, px, py);
-        const int id = __ldg(nb->ids + k);
+        const int id = __ldg(nb->ids[l] + k);
         if (g < best || (g == best && id < best_id)) {
             best = g;
             best_id = id;
@@ -121,13 +126,13 @@ static __device__ __forceinline__ bool nearest_neighbour(const DevLayout &L, dou
     return best <= within;
 }
 
-// The same from the target's neighbours, else from p's cell list when it
+// The same from the target's neighbours (nb, nullable), else from p's cell list when it
 // settles the answer: every rect within crad of p is listed, so a listed
 // nearest other within crad is the nearest (ties included); otherwise the
 // tree.  Writes the rect, false when none.
 static __device__ __forceinline__ bool nearest_other(const DevLayout &L, double4 target, const Neighbours *nb, double px,
                                                      double py, int exclude, float4 &o) {
-    if (nearest_neighbour(L, target, nb, px, py, o)) return true;
+    if (nb && nearest_neighbour(L, target, nb, px, py, o)) return true;
     if (L.cells && px >= L.bx0 && py >= L.by0 && px <= L.bx1 && py <= L.by1) {
         const int64_t cell = cell_of(L, px, py);
         const float4 *r = L.cells + kCellSlots * cell;

@@ -180,10 +180,13 @@ static __device__ __noinline__ uint32_t tree_clearance_call(const float4 *nbox, 
 }
 
 // The cell of a point inside the bounds (the far edge's cells by clamping).
+__device__ __forceinline__ uint2 cell_xy(const DevLayout &L, double px, double py) {
+    return make_uint2(min((unsigned)(int)__dmul_rn(__dsub_rn(px, L.gx0), L.ginv), (unsigned)(L.gnx - 1)),
+                      min((unsigned)(int)__dmul_rn(__dsub_rn(py, L.gy0), L.ginv), (unsigned)(L.gny - 1)));
+}
 __device__ __forceinline__ int64_t cell_of(const DevLayout &L, double px, double py) {
-    const unsigned ix = min((unsigned)(int)__dmul_rn(__dsub_rn(px, L.gx0), L.ginv), (unsigned)(L.gnx - 1));
-    const unsigned iy = min((unsigned)(int)__dmul_rn(__dsub_rn(py, L.gy0), L.ginv), (unsigned)(L.gny - 1));
-    return (int64_t)iy * L.gnx + ix;
+    const uint2 c = cell_xy(L, px, py);
+    return (int64_t)c.y * L.gnx + c.x;
 }
 
 // Two neighbouring rects of a record in one 256-bit read (32-byte aligned).
