@@ -165,13 +165,14 @@ __global__ void __launch_bounds__(256) k3_check_boxes(const float *__restrict__ 
     }
 }
 
-// Boxes of one bin compared pairwise, a thread per bin entry against the later
-// ones of its bin up to the first that overlaps it (interiors meet): *pair =
-// min over the pairs found of (lower index << 32 | higher).  Two overlapping
-// boxes share a bin.
+// Boxes of one bin compared pairwise, a thread per bin entry against those of its
+// bin with a higher index (interiors meet): *pair = the lowest overlapping pair
+// (lower index << 32 | higher), whatever order the bins were filled in.  Two
+// overlapping boxes share a bin.  A thread whose box is above the lower one of a
+// pair found has nothing to add, so layouts full of overlaps end soon.
 __global__ void __launch_bounds__(256) k3_overlaps(const float *__restrict__ boxes, const int64_t *__restrict__ bstart,
                                                    int64_t nbins, const int32_t *__restrict__ items,
-                                                   unsigned long long *__restrict__ pair) {
+                                                   unsigned long long *pair) {
     const int64_t total = bstart[nbins];
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total; u += (int64_t)gridDim.x * blockDim.x) {
         int64_t a = 0, b = nbins;  // the bin of entry u: bstart[a] <= u < bstart[a + 1]
@@ -180,17 +181,20 @@ __global__ void __launch_bounds__(256) k3_overlaps(const float *__restrict__ box
             if (bstart[m] <= u) a = m;
             else b = m;
         }
-        const int64_t e = bstart[a + 1];
+        const int64_t s = bstart[a], e = bstart[a + 1];
         const int i = items[u];
         float4 lo, hi;
         load_box(boxes, i, lo, hi);
-        for (int64_t v = u + 1; v < e; v++) {
+        int lowest = INT32_MAX;  // box of the bin that overlaps box i
+        for (int64_t v = s; v < e; v++) {
+            if (((v - s) & 31) == 0 && (unsigned long long)i > (*(volatile unsigned long long *)pair >> 32)) break;
             const int j = items[v];
+            if (j <= i || j >= lowest) continue;
             float4 l2, h2;
             load_box(boxes, j, l2, h2);
             if (lo.x < h2.x && l2.x < hi.x && lo.y < h2.y && l2.y < hi.y && lo.z < h2.z && l2.z < hi.z) {
-                atomicMin(pair, ((unsigned long long)(unsigned)min(i, j) << 32) | (unsigned)max(i, j));
-                break;
+                lowest = j;
+                atomicMin(pair, ((unsigned long long)(unsigned)i << 32) | (unsigned)j);
             }
         }
     }
