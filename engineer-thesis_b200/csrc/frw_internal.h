@@ -308,8 +308,9 @@ struct RowEntry {
     unsigned long long n;
     double s, s2;
 };
-// The same as entries of 32 bytes (room for every nonzero row); the kernel
-// limit word *src, when given, is copied to *dst.
+// The same as entries of 32 bytes (room for every nonzero row); a status word
+// *src, when given, is copied to *dst beside the count, so that one read brings
+// both.
 frw_status launch_compact_entries(const unsigned long long *acc_n, const double *acc_s, const double *acc_s2,
                                   int64_t rows, RowEntry *out, unsigned long long *d_count, const uint32_t *src,
                                   uint32_t *dst, cudaStream_t stream);

@@ -9,7 +9,8 @@
 //   3. a level-synchronous split of Morton ranges: each frontier range is cut
 //      at its next base-4 digit by binary search on the sorted keys (no data
 //      movement); child node ids come from a block scan and an atomic per
-//      block, the level sizes staying on the device; single-quadrant ranges
+//      block (so above kSmallBuild rects they follow the blocks' order, which no
+//      result depends on), the level sizes staying on the device; single-quadrant ranges
 //      are re-split one level down without emitting a node (path
 //      compression); ranges whose keys are all equal are split by index;
 //   4. a bottom-up refit of the child boxes, batch by batch in reverse
@@ -598,8 +599,10 @@ frw_status build_tree(const float4 *d_rects_in, int32_t n, const double bounds[4
         if (!ck(cudaMallocAsync(&v0, (size_t)n * 4, st), "malloc vals")) break;
         if (!ck(cudaMallocAsync(&v1, (size_t)n * 4, st), "malloc vals")) break;
         if (!ck(cudaMallocAsync(&hist, (size_t)256 * (nblk + 1) * 4, st), "malloc hist")) break;
-        if (!ck(cudaMallocAsync(&cnt, (size_t)cap_nodes * 8, st), "malloc cnt")) break;
-        if (!ck(cudaMallocAsync(&tot, 16, st), "malloc tot")) break;  // scan total, or the small build's result
+        if (n <= kSmallBuild) {  // the one-block build's counts and result
+            if (!ck(cudaMallocAsync(&cnt, (size_t)cap_nodes * 8, st), "malloc cnt")) break;
+            if (!ck(cudaMallocAsync(&tot, 16, st), "malloc result")) break;
+        }
         if (!ck(cudaMallocAsync(&frb, (size_t)cap_nodes * 8 * 4, st), "malloc frontier")) break;
 
         double W = bounds[2] - bounds[0], H = bounds[3] - bounds[1];
