@@ -170,7 +170,10 @@ frw_status prepare_walk(const frw3_layout *L, int64_t target, uint64_t first, ui
 
 // Device scratch of walks from T targets: the rows of T x n boxes and a header
 // of words (counter, row count, grid status, pad, stats[4 T]), cleared in one
-// memset; the nonzero rows as entries behind the header; `extra` bytes.
+// memset; the nonzero rows as entries behind the header; `extra` bytes.  There is
+// room for kEntryRoom entries: a matrix of many targets has far more rows, most
+// of them zero, and one with more nonzero rows brings them in ranges.
+constexpr int64_t kEntryRoom = 1 << 18;
 struct WalkScratch3 {
     Scratch3 mem{nullptr};
     cudaStream_t st = nullptr;
@@ -191,8 +194,9 @@ struct WalkScratch3 {
     frw_status read(const uint32_t *status, const char *what, std::vector<unsigned long long> *stats,
                     std::vector<RowEntry> *rows) const {
         const double *sw = (const double *)(hits + nrow);
-        frw_status rc = launch_compact_entries(hits, sw, sw + nrow, (int64_t)nrow, (RowEntry *)(hdr + words), hdr + 1,
-                                               status, (uint32_t *)(hdr + 2), st);
+        RowEntry *entries = (RowEntry *)(hdr + words);
+        frw_status rc = launch_compact_entries(hits, sw, sw + nrow, (int64_t)nrow, entries, room, hdr + 1, status,
+                                               (uint32_t *)(hdr + 2), st);
         if (rc) return rc;
         std::vector<unsigned long long> h(words);
         if ((rc = read_rows(hdr, words * 8, 8, room, st, what, h.data(), rows))) return rc;
@@ -201,6 +205,17 @@ struct WalkScratch3 {
             return FRW_E_KERNEL;
         }
         stats->assign(h.begin() + 4, h.end());
+        if (h[1] <= (unsigned long long)room) return FRW_OK;
+        std::vector<RowEntry> range;
+        for (int64_t r = 0; r < (int64_t)nrow; r += room) {
+            FRW_CK(cudaMemsetAsync(hdr + 1, 0, 8, st));
+            if ((rc = launch_compact_entries(hits + r, sw + r, sw + nrow + r, std::min<int64_t>(room, (int64_t)nrow - r),
+                                             entries, room, hdr + 1, nullptr, nullptr, st)))
+                return rc;
+            if ((rc = read_rows(hdr, words * 8, 8, room, st, what, h.data(), &range))) return rc;
+            for (RowEntry &e : range) e.row += r;
+            rows->insert(rows->end(), range.begin(), range.end());
+        }
         return FRW_OK;
     }
 };
@@ -209,7 +224,7 @@ frw_status walk_scratch3(int64_t T, int64_t n, uint64_t walks, size_t extra, cud
     W->st = W->mem.st = st;
     W->nrow = (size_t)(T * n);
     W->words = 4 + 4 * (size_t)T;
-    W->room = (int64_t)std::min<uint64_t>(W->nrow, std::max<uint64_t>(walks, 1));
+    W->room = (int64_t)std::min<uint64_t>({W->nrow, std::max<uint64_t>(walks, 1), (uint64_t)kEntryRoom});
     const size_t clear = (3 * W->nrow + W->words) * 8, rows = (size_t)W->room * sizeof(RowEntry);
     FRW_CK(cudaMallocAsync(&W->mem.p, clear + rows + extra, st));
     FRW_CK(cudaMemsetAsync(W->mem.p, 0, clear, st));

@@ -379,14 +379,18 @@ frw_status run_walks(const frw_layout *lay, int64_t target, uint64_t first_walk,
         return check_status(d_status, st);
     }
     FRW_CK(cudaEventRecord(e1, st));
-    rc = launch_compact_entries(d_acc_n, d_acc_s, d_acc_s2, rows, reinterpret_cast<RowEntry *>(h + 1), &h->cnt, nullptr,
-                                nullptr, st);
+    rc = launch_compact_entries(d_acc_n, d_acc_s, d_acc_s2, rows, reinterpret_cast<RowEntry *>(h + 1), room, &h->cnt,
+                                nullptr, nullptr, st);
     if (rc) return rc;
     Hdr hh;
     rc = read_rows(h, sizeof(Hdr), offsetof(Hdr, cnt), room, st, "walk results", &hh, &out->rows);
     if (rc) return rc;
     rc = status_error(hh.status);
     if (rc) return rc;
+    if (hh.cnt > (unsigned long long)room) {  // (room holds every row that a walk can end on)
+        set_error("walk results: more rows than walks");
+        return FRW_E_KERNEL;
+    }
     memcpy(out->gauss, &hh.gauss, sizeof(out->gauss));
     out->escaped = hh.stats[0];
     out->aborted = hh.stats[1];
@@ -559,10 +563,8 @@ frw_status read_rows(const void *dev, size_t hdr_bytes, size_t count_at, int64_t
     memcpy(hdr, buf.data(), hdr_bytes);
     unsigned long long cnt;
     memcpy(&cnt, buf.data() + count_at, 8);
-    if (cnt > (unsigned long long)room) {
-        set_error(std::string(what) + ": more rows than room for them");
-        return FRW_E_KERNEL;
-    }
+    rows->clear();
+    if (cnt > (unsigned long long)room) return FRW_OK;
     rows->resize(cnt);
     const size_t got = std::min<size_t>(head, cnt);
     if (got) memcpy(rows->data(), buf.data() + hdr_bytes, got * sizeof(RowEntry));

@@ -308,16 +308,17 @@ struct RowEntry {
     unsigned long long n;
     double s, s2;
 };
-// The same as entries of 32 bytes (room for every nonzero row); a status word
+// The same as entries of 32 bytes, those past `room` counted only; a status word
 // *src, when given, is copied to *dst beside the count, so that one read brings
 // both.
 frw_status launch_compact_entries(const unsigned long long *acc_n, const double *acc_s, const double *acc_s2,
-                                  int64_t rows, RowEntry *out, unsigned long long *d_count, const uint32_t *src,
-                                  uint32_t *dst, cudaStream_t stream);
+                                  int64_t rows, RowEntry *out, int64_t room, unsigned long long *d_count,
+                                  const uint32_t *src, uint32_t *dst, cudaStream_t stream);
 // A result header of hdr_bytes at dev with its `room` row entries right behind
 // it, after everything enqueued on `st`: one copy for the header and the
 // entries of a small result, a second one for the rest of a large one.  The
-// count (u64) lies at hdr + count_at.  Entries come sorted by row.
+// count (u64) lies at hdr + count_at; *rows stays empty when it is above room.
+// Entries come sorted by row.
 frw_status read_rows(const void *dev, size_t hdr_bytes, size_t count_at, int64_t room, cudaStream_t st,
                      const char *what, void *hdr, std::vector<RowEntry> *rows);
 

@@ -591,7 +591,7 @@ __global__ void k_compact(const unsigned long long *__restrict__ acc_n, const do
 
 __global__ void k_compact_entries(const unsigned long long *__restrict__ acc_n, const double *__restrict__ acc_s,
                                   const double *__restrict__ acc_s2, int64_t rows, RowEntry *__restrict__ out,
-                                  unsigned long long *count, const uint32_t *src, uint32_t *dst) {
+                                  int64_t room, unsigned long long *count, const uint32_t *src, uint32_t *dst) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0 && src) *dst = *src;
     const unsigned long long n = i < rows ? acc_n[i] : 0;
@@ -601,7 +601,8 @@ __global__ void k_compact_entries(const unsigned long long *__restrict__ acc_n, 
     unsigned long long base = 0;
     if (lane == leader) base = atomicAdd(count, (unsigned long long)__popc(m));
     base = __shfl_sync(kFull, base, leader);
-    if (n) out[base + __popc(m & ((1u << lane) - 1u))] = RowEntry{i, n, acc_s[i], acc_s2[i]};
+    const unsigned long long at = base + __popc(m & ((1u << lane) - 1u));
+    if (n && at < (unsigned long long)room) out[at] = RowEntry{i, n, acc_s[i], acc_s2[i]};
 }
 
 }  // namespace
@@ -664,10 +665,10 @@ frw_status launch_walk(const WalkParams &Pin, int threads, int blocks, cudaStrea
 }
 
 frw_status launch_compact_entries(const unsigned long long *acc_n, const double *acc_s, const double *acc_s2,
-                                  int64_t rows, RowEntry *out, unsigned long long *d_count, const uint32_t *src,
-                                  uint32_t *dst, cudaStream_t stream) {
-    k_compact_entries<<<(unsigned)((rows + 255) / 256), 256, 0, stream>>>(acc_n, acc_s, acc_s2, rows, out, d_count,
-                                                                          src, dst);
+                                  int64_t rows, RowEntry *out, int64_t room, unsigned long long *d_count,
+                                  const uint32_t *src, uint32_t *dst, cudaStream_t stream) {
+    k_compact_entries<<<(unsigned)((rows + 255) / 256), 256, 0, stream>>>(acc_n, acc_s, acc_s2, rows, out, room,
+                                                                          d_count, src, dst);
     FRW_CK(cudaGetLastError());
     return FRW_OK;
 }
