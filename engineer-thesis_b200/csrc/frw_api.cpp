@@ -479,7 +479,10 @@ frw_status copy_out(std::initializer_list<HostOut> arrays, int device, cudaStrea
     // measured on 24 MB of per-walk records.  Past kLarge bytes, kCopiers threads
     // (the caller one of them) take chunks in turn, each through a pinned buffer
     // (1e6 traced walks 4.5 -> 2.6 ms; 12 MB of queries 1.02 -> 1.17 ms, so not
-    // below 16).  Page-locked, managed and device memory, which the driver
+    // below 16; from 4 MB on, 7 MB of queries 0.87 -> 1.00; not below 64, 22 MB of
+    // walks 1.49 -> 1.87).  On a host of 16 cores 38 MB of queries take 4.8 ms with
+    // one copier, 3.4 with two, 2.8 with four and 2.7 with eight; 3.3 and 3.2 in
+    // chunks of 256 KiB and 4 MiB.  Page-locked, managed and device memory, which the driver
     // writes to directly, is left to it: 3e6 queries into page-locked arrays 5.6 ms
     // in chunks, 3.2 in one copy each.
     constexpr size_t kLarge = 16 << 20, kChunk = 1 << 20;
