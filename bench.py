@@ -514,7 +514,8 @@ def walk3d_run(frw, device, stream, steps, cpu_seconds, cores, sm_mhz=None):
            "queries_1e7": {"ms": qms, "queries_per_s": 1e7 / (qms * 1e-3)},
            "roofline": roof3,
            "e2e": {"value": W3D["walks"] / e2e_s, "unit": "walks/s", "h2d_bytes_per_step": W3D["boxes"] * 24,
-                   "d2h_bytes_per_step": (5 + 3 * W3D["boxes"]) * 8}}
+                   # the header's 8 words and the row entries (the first read brings 126)
+                   "d2h_bytes_per_step": 64 + 32 * max(126, len(r.conductor))}}
     if cpu_seconds > 0 and cores > 0:
         ctx = mp.get_context("spawn")
         with ctx.Pool(cores) as pool:
@@ -777,7 +778,8 @@ def main():
                       "traversal's); the reference CPU tree as shipped misses collisions"},
             "e2e": {"value": W["walks"] / (e2e_ms * 1e-3), "unit": "walks/s",
                     "h2d_bytes_per_step": W["rects"] * 16 + 32,
-                    "d2h_bytes_per_step": nrows * 32 + 64},
+                    # the header and the row entries (the first read brings 125)
+                    "d2h_bytes_per_step": 96 + 32 * max(125, nrows)},
             "gpu_launches": (2 if world == 1 else 3) * args.steps,
             "roofline": roof,
             "clocks": clocks,
