@@ -45,7 +45,10 @@ constexpr int kHopsPerRound = 4;
 // block spill (1e7 capacitance walks on 10^4 rects 2.06 -> 1.98 ms, 28 batched
 // layouts 2.18 -> 1.94 against 5; Green-function starts 2e7 walks on 10^6 rects
 // 5.09 -> 5.03, 3e6 on 10^4 0.86 -> 0.81, 10^5 0.21 -> 0.20; 3 blocks and 6 are
-// slower).
+// slower).  With the tree's code too: a call of 1e6 walks on 10^4 rects without
+// cell lists 2.55 -> 2.43 ms (Green-function starts) and 2.12 -> 1.99
+// (capacitance) against 5 blocks, on 3e5 3.01 -> 2.68 and 2.09 -> 1.98, with the
+// other steps since.
 constexpr int kWalkMinBlocks = 4;
 constexpr int kWarpsPerBlock = kWalkThreads / 32;
 constexpr int kTabSlots = 32;  // per warp
